@@ -171,131 +171,175 @@ __global__ void k_map_targets(const int64_t *__restrict__ tg, int64_t nt, const 
     out[t] = inv[tg[t]];
 }
 // gravity_direct (src/gravity/gravdirect.c:61-257) with force_evaluate_direct's pair arithmetic
-// (src/gravity/forcetree_walk.c:557-708): the n particles are targets and sources; every thread sums
-// all sources in their order with the reference's operations (FP64, no contraction), so the result is
+// (src/gravity/forcetree_walk.c:557-708): the n particles are targets and sources; every target's terms
+// are the reference's operations (FP64, no contraction) and are added in source order, so the result is
 // bit-identical.  Flag bit 1: a softening type >= nsofttypes.
-__global__ void __launch_bounds__(kTile) k_gravity_direct(const double *__restrict__ pos, const double *__restrict__ mass,
-                                                          const uint8_t *__restrict__ st, int64_t n,
-                                                          const WalkConst *__restrict__ wcp, double *__restrict__ acc,
-                                                          double *__restrict__ pot, int *__restrict__ flag)
+//
+// Only the additions have to follow each other; the terms (a square root, divisions, the table) do not.
+// A warp takes T targets and 32 sources at a time: every lane computes the terms of its source for the T
+// targets into shared memory, then 4 T lanes add them, one sum component each, in source order.
+template <bool EWALD>
+__device__ __forceinline__ void direct_terms(const double4 s, double h_j, double4 me, double h_i, const WalkConst &w, double *__restrict__ out)
 {
-  __shared__ double4 src[kTile];
-  __shared__ double hsrc[kTile];
-  const WalkConst &w = *wcp;
-  const int64_t i    = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  double pos_x = 0, pos_y = 0, pos_z = 0, h_i = 0;
-  if(i < n)
+  constexpr int P = 33;  // component pitch of `out`
+#pragma unroll
+  for(int c = 0; c < (EWALD ? 8 : 4); c++)
+    out[c * P] = 0.0;
+  double hmax = (h_j > h_i) ? h_j : h_i;
+  double dx = s.x - me.x, dy = s.y - me.y, dz = s.z - me.z;
+  if(w.periodic)
     {
-      pos_x = pos[3 * i + 0];
-      pos_y = pos[3 * i + 1];
-      pos_z = pos[3 * i + 2];
-      if(st[i] >= w.nsoft)
-        atomicOr(flag, 1);
-      h_i = w.soft[st[i] < w.nsoft ? st[i] : 0];
+      dx = (dx > w.half_box) ? (dx - w.box) : ((dx < -w.half_box) ? (dx + w.box) : dx);
+      dy = (dy > w.half_box) ? (dy - w.box) : ((dy < -w.half_box) ? (dy + w.box) : dy);
+      dz = (dz > w.half_box) ? (dz - w.box) : ((dz < -w.half_box) ? (dz + w.box) : dz);
     }
-  double acc_x = 0, acc_y = 0, acc_z = 0, pt = 0;
-  for(int64_t jb = 0; jb < n && n > 1; jb += kTile)
+  double r2 = dx * dx + dy * dy + dz * dz;
+  double m  = s.w;
+  double r  = sqrt(r2);
+  double factor_force = 0, factor_pot = 0;
+  if(w.pm)
     {
-      __syncthreads();
-      const int64_t j = jb + threadIdx.x;
+      double tabentry = w.asmthfac * r;
+      int tabindex    = (int)tabentry;
+      if(tabindex >= kNtab)
+        return;
+      double tabweight = tabentry - tabindex;
+      factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
+      factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];
+    }
+  double fac, wp;
+  if(r >= hmax)
+    {
+      double rinv  = 1.0 / r;
+      double rinv3 = rinv * rinv * rinv;
+      if(w.pm)
+        {
+          fac = rinv3 + rinv * factor_force * w.asmthinv2;
+          wp  = rinv * factor_pot;
+        }
+      else
+        {
+          fac = rinv3;
+          wp  = -rinv;
+        }
+    }
+  else
+    {
+      double h_inv  = 1.0 / hmax;
+      double h3_inv = h_inv * h_inv * h_inv;
+      double u      = r * h_inv;
+      if(u < 0.5)
+        {
+          double u2 = u * u;
+          fac       = h3_inv * (SF1 + u2 * (SF2 * u + SF3));
+          wp        = h_inv * (SF4 + u2 * (SF5 + u2 * (SF6 * u + SF7)));
+        }
+      else
+        {
+          double u2 = u * u;
+          double u3 = u2 * u;
+          fac       = h3_inv * (SF8 + SF9 * u + SF10 * u2 + SF11 * u3 + SF12 / u3);
+          wp        = h_inv * (SF13 + SF14 / u + u2 * (SF1 + u * (SF15 + u * (SF16 + SF17 * u))));
+        }
+      if(w.pm && r > 0)
+        {
+          double rinv = 1.0 / r;
+          fac += rinv * factor_force * w.asmthinv2;
+          wp += rinv * (factor_pot + 1.0);
+        }
+    }
+  fac *= m;
+  out[0 * P] = dx * fac;
+  out[1 * P] = dy * fac;
+  out[2 * P] = dz * fac;
+  out[3 * P] = m * wp;
+  if(EWALD)
+    {
+      double fcorr[3], pcorr;
+      ewald_corr(dx, dy, dz, w, fcorr, pcorr);
+      out[4 * P] = m * fcorr[0];
+      out[5 * P] = m * fcorr[1];
+      out[6 * P] = m * fcorr[2];
+      out[7 * P] = m * pcorr;
+    }
+}
+
+constexpr int kDirWarps        = 4;
+constexpr int64_t kDirOneTarget = 8192;
+template <int T, bool EWALD>
+__global__ void __launch_bounds__(32 * kDirWarps) k_gravity_direct(const double *__restrict__ pos, const double *__restrict__ mass,
+                                                                   const uint8_t *__restrict__ st, int64_t n,
+                                                                   const WalkConst *__restrict__ wcp, double *__restrict__ acc,
+                                                                   double *__restrict__ pot, int *__restrict__ flag)
+{
+  constexpr int C = EWALD ? 8 : 4;
+  static_assert(4 * T <= 32, "one lane per target and component");
+  __shared__ WalkConst w;
+  __shared__ double term[kDirWarps][T][C][33];
+  for(int t = threadIdx.x; t < (int)(sizeof(WalkConst) / 4); t += blockDim.x)
+    ((int *)&w)[t] = ((const int *)wcp)[t];
+  __syncthreads();
+  const int warp   = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t i0 = ((int64_t)blockIdx.x * kDirWarps + warp) * T;
+  if(i0 >= n)
+    return;
+  double4 me[T];
+  double h_i[T];
+#pragma unroll
+  for(int t = 0; t < T; t++)
+    {
+      const int64_t i = i0 + t < n ? i0 + t : n - 1;  // a target past the end repeats the last one
+      const int ty    = st[i];
+      if(ty >= w.nsoft)
+        atomicOr(flag, 1);
+      me[t]  = make_double4(pos[3 * i + 0], pos[3 * i + 1], pos[3 * i + 2], 0.0);
+      h_i[t] = w.soft[ty < w.nsoft ? ty : 0];
+    }
+  const int st_ = lane >> 2, sc = lane & 3;  // this lane's target and component in the additions
+  double sum    = 0;
+  for(int64_t jb = 0; jb < n && n > 1; jb += 32)
+    {
+      const int64_t j = jb + lane;
       if(j < n)
         {
-          src[threadIdx.x]  = make_double4(pos[3 * j + 0], pos[3 * j + 1], pos[3 * j + 2], mass[j]);
-          hsrc[threadIdx.x] = w.soft[st[j] < w.nsoft ? st[j] : 0];
+          const double4 s  = make_double4(pos[3 * j + 0], pos[3 * j + 1], pos[3 * j + 2], mass[j]);
+          const int ty     = st[j];
+          const double h_j = w.soft[ty < w.nsoft ? ty : 0];
+#pragma unroll
+          for(int t = 0; t < T; t++)
+            direct_terms<EWALD>(s, h_j, me[t], h_i[t], w, &term[warp][t][0][lane]);
         }
-      __syncthreads();
-      const int cnt = (int)((n - jb) < kTile ? (n - jb) : kTile);
-      if(i < n)
-        for(int q = 0; q < cnt; q++)
-          {
-            const double4 s  = src[q];
-            const double h_j = hsrc[q];
-            double hmax      = (h_j > h_i) ? h_j : h_i;
-            double dx = s.x - pos_x, dy = s.y - pos_y, dz = s.z - pos_z;
-            if(w.periodic)
+      __syncwarp();
+      const int cnt = n - jb < 32 ? (int)(n - jb) : 32;
+      if(st_ < T)
+        {
+          const double *q = &term[warp][st_][sc][0];
+          if(cnt == 32)
+            {
+#pragma unroll
+              for(int k = 0; k < 32; k++)
+                {
+                  sum += q[k];
+                  if(EWALD)
+                    sum += q[4 * 33 + k];
+                }
+            }
+          else
+            for(int k = 0; k < cnt; k++)
               {
-                dx = (dx > w.half_box) ? (dx - w.box) : ((dx < -w.half_box) ? (dx + w.box) : dx);
-                dy = (dy > w.half_box) ? (dy - w.box) : ((dy < -w.half_box) ? (dy + w.box) : dy);
-                dz = (dz > w.half_box) ? (dz - w.box) : ((dz < -w.half_box) ? (dz + w.box) : dz);
+                sum += q[k];
+                if(EWALD)
+                  sum += q[4 * 33 + k];
               }
-            double r2 = dx * dx + dy * dy + dz * dz;
-            double m  = s.w;
-            double r  = sqrt(r2);
-            double factor_force = 0, factor_pot = 0;
-            if(w.pm)
-              {
-                double tabentry = w.asmthfac * r;
-                int tabindex    = (int)tabentry;
-                if(tabindex >= kNtab)
-                  continue;
-                double tabweight = tabentry - tabindex;
-                factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
-                factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];
-              }
-            double fac, wp;
-            if(r >= hmax)
-              {
-                double rinv  = 1.0 / r;
-                double rinv3 = rinv * rinv * rinv;
-                if(w.pm)
-                  {
-                    fac = rinv3 + rinv * factor_force * w.asmthinv2;
-                    wp  = rinv * factor_pot;
-                  }
-                else
-                  {
-                    fac = rinv3;
-                    wp  = -rinv;
-                  }
-              }
-            else
-              {
-                double h_inv  = 1.0 / hmax;
-                double h3_inv = h_inv * h_inv * h_inv;
-                double u      = r * h_inv;
-                if(u < 0.5)
-                  {
-                    double u2 = u * u;
-                    fac       = h3_inv * (SF1 + u2 * (SF2 * u + SF3));
-                    wp        = h_inv * (SF4 + u2 * (SF5 + u2 * (SF6 * u + SF7)));
-                  }
-                else
-                  {
-                    double u2 = u * u;
-                    double u3 = u2 * u;
-                    fac       = h3_inv * (SF8 + SF9 * u + SF10 * u2 + SF11 * u3 + SF12 / u3);
-                    wp        = h_inv * (SF13 + SF14 / u + u2 * (SF1 + u * (SF15 + u * (SF16 + SF17 * u))));
-                  }
-                if(w.pm && r > 0)
-                  {
-                    double rinv = 1.0 / r;
-                    fac += rinv * factor_force * w.asmthinv2;
-                    wp += rinv * (factor_pot + 1.0);
-                  }
-              }
-            pt += m * wp;
-            fac *= m;
-            acc_x += dx * fac;
-            acc_y += dy * fac;
-            acc_z += dz * fac;
-            if(w.ewald)
-              {
-                double fcorr[3], pcorr;
-                ewald_corr(dx, dy, dz, w, fcorr, pcorr);
-                acc_x += m * fcorr[0];
-                acc_y += m * fcorr[1];
-                acc_z += m * fcorr[2];
-                pt += m * pcorr;
-              }
-          }
+        }
+      __syncwarp();
     }
-  if(i < n)
+  if(st_ < T && i0 + st_ < n)
     {
-      acc[3 * i + 0] = acc_x;
-      acc[3 * i + 1] = acc_y;
-      acc[3 * i + 2] = acc_z;
-      if(pot)
-        pot[i] = pt;
+      if(sc < 3)
+        acc[3 * (i0 + st_) + sc] = sum;
+      else if(pot)
+        pot[i0 + st_] = sum;
     }
 }
 
@@ -309,8 +353,14 @@ __global__ void k_fill_i32(int32_t *__restrict__ a, int64_t n, int32_t v)
 cudaError_t gravity_direct_stage(gpugrav_ctx *c, int64_t n, const double *d_pos, const double *d_mass, const uint8_t *d_st,
                                  double *d_acc, double *d_pot, int32_t *d_nint, int *d_flag)
 {
-  k_gravity_direct<<<(unsigned)((n + kTile - 1) / kTile), kTile, 0, c->stream>>>(d_pos, d_mass, d_st, n, c->wconst.as<WalkConst>(),
-                                                                                   d_acc, d_pot, d_flag);
+  // one target per warp while the chip has room for more warps than targets, else 4
+  const bool ewald = c->prm.periodic && !(c->prm.asmth > 0);
+  const int T      = n <= kDirOneTarget ? 1 : 4;
+  auto kern        = T == 1 ? (ewald ? k_gravity_direct<1, true> : k_gravity_direct<1, false>)
+                            : (ewald ? k_gravity_direct<4, true> : k_gravity_direct<4, false>);
+  const int64_t per = (int64_t)kDirWarps * T;
+  kern<<<(unsigned)((n + per - 1) / per), 32 * kDirWarps, 0, c->stream>>>(d_pos, d_mass, d_st, n, c->wconst.as<WalkConst>(), d_acc, d_pot,
+                                                                        d_flag);
   if(d_nint)
     k_fill_i32<<<(unsigned)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368), 256, 0, c->stream>>>(d_nint, n, (int32_t)n);
   return cudaGetLastError();
