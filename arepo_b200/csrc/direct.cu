@@ -3,8 +3,10 @@
 // (src/gravity/gravtree_forcetest.c:483-601) without the Ewald terms.  For a
 // periodic TreePM run it returns the short-range force with the exact erfc
 // factor (u = r / (2 Asmth)); for an isolated run the Newtonian force.  Both
-// with the cubic-spline softening of the walk.  Sources are split in chunks;
-// partial sums are reduced in a fixed order (deterministic).
+// with the cubic-spline softening of the walk.  Source tiles are dealt out to
+// chunks; partial sums are reduced in a fixed order (deterministic).
+#include <cub/cub.cuh>
+
 #include "internal.h"
 
 namespace gg
@@ -29,121 +31,195 @@ namespace
 #define SF16 9.6
 #define SF17 (-2.133333333333)
 
-constexpr int kTile   = 128;  // targets per block (one per thread)
-constexpr int kChunks = 64;   // source chunks
-
-__global__ void __launch_bounds__(kTile) k_direct(const double4 *__restrict__ pm, const uint8_t *__restrict__ st, int64_t n,
-                                                  const int64_t *__restrict__ targets_sorted, int64_t nt,
-                                                  const WalkConst *__restrict__ wcp, int cut, double4 *__restrict__ partial)
+// Source tiles: 32 consecutive sources in key order and their bounding box (centre, half extents).
+constexpr int kTileSrc = 32;
+constexpr int kTgt     = 4;  // targets per warp: a source is loaded once for them
+struct TileBox
 {
-  __shared__ double4 src[kTile];
-  __shared__ double hsrc[kTile];
-  const WalkConst &w = *wcp;
-  const int64_t t    = (int64_t)blockIdx.x * kTile + threadIdx.x;
-  const int chunk    = blockIdx.y;
-  const int64_t per  = (n + kChunks - 1) / kChunks;
-  const int64_t j0 = chunk * per, j1 = (j0 + per < n) ? j0 + per : n;
-  double4 me = make_double4(0, 0, 0, 0);
-  double h_i = 0;
-  if(t < nt)
+  double cx, cy, cz, hx, hy, hz;
+};
+
+__global__ void k_tile_box(const double4 *__restrict__ pm, int64_t n, int64_t ntile, TileBox *__restrict__ box)
+{
+  const int lane = threadIdx.x & 31;
+  for(int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; t < ntile; t += ((int64_t)gridDim.x * blockDim.x) >> 5)
     {
-      int64_t i = targets_sorted[t];
-      me        = pm[i];
-      h_i       = w.soft[st[i]];
-    }
-  const double asmth = (w.pm) ? (0.5 / sqrt(w.asmthinv2)) : 0.0;
-  double ax = 0, ay = 0, az = 0, pt = 0;
-  for(int64_t jb = j0; jb < j1; jb += kTile)
-    {
-      __syncthreads();
-      int64_t j = jb + threadIdx.x;
-      if(j < j1)
-        {
-          src[threadIdx.x]  = pm[j];
-          hsrc[threadIdx.x] = w.soft[st[j]];
-        }
-      __syncthreads();
-      int cnt = (int)((j1 - jb) < kTile ? (j1 - jb) : kTile);
-      if(t < nt)
-        for(int q = 0; q < cnt; q++)
+      const int64_t j = t * kTileSrc + lane;
+      const double4 p = pm[j < n ? j : n - 1];
+      double lo[3] = {p.x, p.y, p.z}, hi[3] = {p.x, p.y, p.z};
+#pragma unroll
+      for(int k = 0; k < 3; k++)
+        for(int o = 16; o > 0; o >>= 1)
           {
-            double4 s   = src[q];
-            double dx   = s.x - me.x, dy = s.y - me.y, dz = s.z - me.z;
-            if(w.periodic)
-              {
-                dx = (dx > w.half_box) ? dx - w.box : ((dx < -w.half_box) ? dx + w.box : dx);
-                dy = (dy > w.half_box) ? dy - w.box : ((dy < -w.half_box) ? dy + w.box : dy);
-                dz = (dz > w.half_box) ? dz - w.box : ((dz < -w.half_box) ? dz + w.box : dz);
-              }
-            double r2 = dx * dx + dy * dy + dz * dz;
-            if(cut && w.pm && !(r2 < w.rcut2))
-              continue;  // beyond Rcut: the part of the force left to the PM mesh
-            double r  = sqrt(r2);
-            double m  = s.w;
-            double h_j  = hsrc[q];
-            double hmax = (h_j > h_i) ? h_j : h_i;
-            double fac_newton = 0, wp_newton = 0, fac, wp;
-            if(r > 0)
-              {
-                fac_newton = m / (r2 * r);
-                wp_newton  = -m / r;
-              }
-            if(r >= hmax)
-              {
-                fac = fac_newton;
-                wp  = wp_newton;
-              }
-            else
-              {
-                double h_inv = 1.0 / hmax, h3_inv = h_inv * h_inv * h_inv, u = r * h_inv;
-                if(u < 0.5)
-                  {
-                    double u2 = u * u;
-                    fac       = m * h3_inv * (SF1 + u2 * (SF2 * u + SF3));
-                    wp        = m * h_inv * (SF4 + u2 * (SF5 + u2 * (SF6 * u + SF7)));
-                  }
-                else
-                  {
-                    double u2 = u * u, u3 = u2 * u;
-                    fac = m * h3_inv * (SF8 + SF9 * u + SF10 * u2 + SF11 * u3 + SF12 / u3);
-                    wp  = m * h_inv * (SF13 + SF14 / u + u2 * (SF1 + u * (SF15 + u * (SF16 + SF17 * u))));
-                  }
-              }
-            if(w.pm)
-              {
-                double u            = 0.5 / asmth * r;
-                double factor_force = (erfc(u) + 2.0 * u / sqrt(M_PI) * exp(-u * u) - 1.0);
-                double factor_pot   = erfc(u);
-                fac += fac_newton * factor_force;
-                wp += wp_newton * (factor_pot - 1.0);
-              }
-            ax += dx * fac;
-            ay += dy * fac;
-            az += dz * fac;
-            pt += wp;
-            if(w.ewald)
-              {
-                // pure periodic tree: every image through the Ewald correction
-                double fcorr[3], pcorr;
-                ewald_corr(dx, dy, dz, w, fcorr, pcorr);
-                ax += m * fcorr[0];
-                ay += m * fcorr[1];
-                az += m * fcorr[2];
-                pt += m * pcorr;
-              }
+            lo[k] = fmin(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+            hi[k] = fmax(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
           }
+      if(lane == 0)
+        box[t] = TileBox{0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]), 0.5 * (lo[2] + hi[2]),
+                         0.5 * (hi[0] - lo[0]), 0.5 * (hi[1] - lo[1]), 0.5 * (hi[2] - lo[2])};
     }
-  if(t < nt)
-    partial[(int64_t)chunk * nt + t] = make_double4(ax, ay, az, pt);
 }
 
-__global__ void k_direct_reduce(const double4 *__restrict__ partial, int64_t nt, double *__restrict__ acc, double *__restrict__ pot)
+__device__ __forceinline__ double nearest_image(double d, const WalkConst &w)
+{
+  return !w.periodic ? d : (d > w.half_box) ? d - w.box : ((d < -w.half_box) ? d + w.box : d);
+}
+
+// One pair: gravity_forcetest_evaluate's force and potential (src/gravity/gravtree_forcetest.c:483-601).
+// u = r / (2 Asmth): beyond kUZero both factors of the split are below 2^-54 of the Newtonian pair, which
+// the reference's sums round to no contribution at all (softened pairs excepted); one exponential and
+// erfcx serve both factors.
+constexpr double kUZero = 6.5;
+template <bool PM, bool EWALD>
+__device__ __forceinline__ void direct_pair(double dx, double dy, double dz, double r2, double m, double hmax, double uscale,
+                                            const WalkConst &w, double4 &a)
+{
+  const double rinv = r2 > 0 ? rsqrt(r2) : 0.0;
+  const double r    = r2 * rinv;
+  const double wpn  = -m * rinv;
+  const double fn   = -wpn * rinv * rinv;
+  double g = 1.0, gp = 1.0;  // force and potential factors of the Newtonian pair
+  if(PM)
+    {
+      const double u = uscale * r, e = exp(-u * u);
+      gp             = erfcx(u) * e;
+      g              = fma(u * 1.1283791670955126, e, gp);  // 2 / sqrt(pi)
+    }
+  double fac = fn * g, wp = wpn * gp;
+  if(r < hmax)
+    {
+      const double h_inv = 1.0 / hmax, h3_inv = h_inv * h_inv * h_inv, u = r * h_inv, u2 = u * u;
+      if(u < 0.5)
+        {
+          fac = m * h3_inv * (SF1 + u2 * (SF2 * u + SF3));
+          wp  = m * h_inv * (SF4 + u2 * (SF5 + u2 * (SF6 * u + SF7)));
+        }
+      else
+        {
+          const double u3 = u2 * u;
+          fac = m * h3_inv * (SF8 + SF9 * u + SF10 * u2 + SF11 * u3 + SF12 / u3);
+          wp  = m * h_inv * (SF13 + SF14 / u + u2 * (SF1 + u * (SF15 + u * (SF16 + SF17 * u))));
+        }
+      if(PM)
+        {
+          fac = fma(fn, g - 1.0, fac);
+          wp  = fma(wpn, gp - 1.0, wp);
+        }
+    }
+  a.x = fma(dx, fac, a.x);
+  a.y = fma(dy, fac, a.y);
+  a.z = fma(dz, fac, a.z);
+  a.w += wp;
+  if(EWALD)
+    {
+      // pure periodic tree: every image through the Ewald correction
+      double fcorr[3], pcorr;
+      ewald_corr(dx, dy, dz, w, fcorr, pcorr);
+      a.x += m * fcorr[0];
+      a.y += m * fcorr[1];
+      a.z += m * fcorr[2];
+      a.w += m * pcorr;
+    }
+}
+
+// A warp sums kTgt targets (consecutive in key order) over the batches of 32 tiles blockIdx.y,
+// blockIdx.y + gridDim.y, ...: each lane compares one tile's box with the targets, then the warp visits the
+// tiles that can hold a pair closer than the split's reach (PM: rskip; else every tile), one source per
+// lane.  Lane sums are added over the warp at the end.
+constexpr int kDirectWarps = 4;
+template <bool PM, bool EWALD>
+__global__ void __launch_bounds__(32 * kDirectWarps) k_direct(const double4 *__restrict__ pm, const uint8_t *__restrict__ st, int64_t n,
+                                                              const TileBox *__restrict__ box, int64_t ntile,
+                                                              const int32_t *__restrict__ targets, int64_t nt,
+                                                              const WalkConst *__restrict__ wcp, int cut, double rskip2,
+                                                              double4 *__restrict__ partial)
+{
+  __shared__ WalkConst w;
+  for(int t = threadIdx.x; t < (int)(sizeof(WalkConst) / 4); t += blockDim.x)
+    ((int *)&w)[t] = ((const int *)wcp)[t];
+  __syncthreads();
+  const int lane   = threadIdx.x & 31;
+  const int64_t t0 = ((int64_t)blockIdx.x * kDirectWarps + (threadIdx.x >> 5)) * kTgt;
+  if(t0 >= nt)
+    return;
+  const double uscale = PM ? sqrt(w.asmthinv2) : 0.0;  // 1 / (2 Asmth)
+  double4 me[kTgt], a[kTgt];
+  double h_i[kTgt];
+#pragma unroll
+  for(int k = 0; k < kTgt; k++)
+    {
+      const int i = targets[t0 + k < nt ? t0 + k : t0];
+      me[k]       = pm[i];
+      h_i[k]      = w.soft[st[i]];
+      a[k]        = make_double4(0, 0, 0, 0);
+    }
+  for(int64_t b = (int64_t)blockIdx.y * 32; b < ntile; b += (int64_t)gridDim.y * 32)
+    {
+      unsigned near = 0;
+      if(b + lane < ntile)
+        {
+          near = (1u << kTgt) - 1u;
+          if(PM)
+            {
+              const TileBox q = box[b + lane];
+              near            = 0;
+#pragma unroll
+              for(int k = 0; k < kTgt; k++)
+                {
+                  // least distance of the target to any image of the box
+                  const double x = fmax(fabs(nearest_image(q.cx - me[k].x, w)) - q.hx, 0.0),
+                               y = fmax(fabs(nearest_image(q.cy - me[k].y, w)) - q.hy, 0.0),
+                               z = fmax(fabs(nearest_image(q.cz - me[k].z, w)) - q.hz, 0.0);
+                  near |= (x * x + y * y + z * z < rskip2 ? 1u : 0u) << k;
+                }
+            }
+        }
+      for(unsigned todo = __ballot_sync(0xffffffffu, near != 0); todo; todo &= todo - 1)
+        {
+          const int q        = __ffs(todo) - 1;
+          const unsigned who = __shfl_sync(0xffffffffu, near, q);
+          const int64_t j    = (b + q) * kTileSrc + lane;
+          const bool valid   = j < n;
+          const double4 s    = pm[valid ? j : n - 1];
+          const double h_j   = w.soft[st[valid ? j : n - 1]];
+#pragma unroll
+          for(int k = 0; k < kTgt; k++)
+            if(who >> k & 1u)
+              {
+                const double dx = nearest_image(s.x - me[k].x, w), dy = nearest_image(s.y - me[k].y, w),
+                             dz   = nearest_image(s.z - me[k].z, w);
+                const double r2   = fma(dx, dx, fma(dy, dy, dz * dz));
+                const double hmax = h_j > h_i[k] ? h_j : h_i[k];
+                // cut: beyond Rcut lies the part of the force left to the PM mesh
+                if(valid && (!PM || (cut ? r2 < w.rcut2 : r2 < rskip2)))
+                  direct_pair<PM, EWALD>(dx, dy, dz, r2, s.w, hmax, uscale, w, a[k]);
+              }
+        }
+    }
+#pragma unroll
+  for(int k = 0; k < kTgt; k++)
+    {
+      for(int o = 16; o > 0; o >>= 1)
+        {
+          a[k].x += __shfl_xor_sync(0xffffffffu, a[k].x, o);
+          a[k].y += __shfl_xor_sync(0xffffffffu, a[k].y, o);
+          a[k].z += __shfl_xor_sync(0xffffffffu, a[k].z, o);
+          a[k].w += __shfl_xor_sync(0xffffffffu, a[k].w, o);
+        }
+      if(lane == 0 && t0 + k < nt)
+        partial[(int64_t)blockIdx.y * nt + t0 + k] = a[k];
+    }
+}
+
+// chunk sums of the t-th target in key order, to its place in the caller's list
+__global__ void k_direct_reduce(const double4 *__restrict__ partial, int chunks, int64_t nt, const int32_t *__restrict__ place,
+                                double *__restrict__ acc, double *__restrict__ pot)
 {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if(t >= nt)
     return;
   double ax = 0, ay = 0, az = 0, pt = 0;
-  for(int c = 0; c < kChunks; c++)
+  for(int c = 0; c < chunks; c++)
     {
       double4 p = partial[(int64_t)c * nt + t];
       ax += p.x;
@@ -151,10 +227,11 @@ __global__ void k_direct_reduce(const double4 *__restrict__ partial, int64_t nt,
       az += p.z;
       pt += p.w;
     }
-  acc[3 * t + 0] = ax;
-  acc[3 * t + 1] = ay;
-  acc[3 * t + 2] = az;
-  pot[t]         = pt;
+  const int64_t o = place[t];
+  acc[3 * o + 0]  = ax;
+  acc[3 * o + 1]  = ay;
+  acc[3 * o + 2]  = az;
+  pot[o]          = pt;
 }
 
 // caller index -> sorted index
@@ -164,11 +241,15 @@ __global__ void k_invert(const uint32_t *__restrict__ perm, int64_t n, int32_t *
     inv[perm[i]] = (int32_t)i;
 }
 
-__global__ void k_map_targets(const int64_t *__restrict__ tg, int64_t nt, const int32_t *__restrict__ inv, int64_t *__restrict__ out)
+__global__ void k_map_targets(const int64_t *__restrict__ tg, int64_t nt, const int32_t *__restrict__ inv, int32_t *__restrict__ out,
+                              int32_t *__restrict__ place)
 {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if(t < nt)
-    out[t] = inv[tg[t]];
+    {
+      out[t]   = inv[tg[t]];
+      place[t] = (int32_t)t;
+    }
 }
 // gravity_direct (src/gravity/gravdirect.c:61-257) with force_evaluate_direct's pair arithmetic
 // (src/gravity/forcetree_walk.c:557-708): the n particles are targets and sources; every target's terms
@@ -369,26 +450,45 @@ cudaError_t gravity_direct_stage(gpugrav_ctx *c, int64_t n, const double *d_pos,
 cudaError_t direct_stage(gpugrav_ctx *c, const WalkConst &wc, int64_t nt, const int64_t *d_targets, int cut, double *d_acc,
                          double *d_pot)
 {
-  (void)wc;
   if(nt == 0)
     return cudaSuccess;
-  cudaError_t e;
-  DevBuf inv, ts, part;
-  if((e = inv.ensure(c->n * sizeof(int32_t))) != cudaSuccess || (e = ts.ensure(nt * sizeof(int64_t))) != cudaSuccess ||
-     (e = part.ensure((size_t)kChunks * nt * sizeof(double4))) != cudaSuccess)
-    return e;
-  k_invert<<<(unsigned)((c->n + 255) / 256 < 2368 ? (c->n + 255) / 256 : 2368), 256, 0, c->stream>>>(c->perm.as<uint32_t>(), c->n,
-                                                                                                       inv.as<int32_t>());
-  k_map_targets<<<(unsigned)((nt + 255) / 256), 256, 0, c->stream>>>(d_targets, nt, inv.as<int32_t>(), ts.as<int64_t>());
-  dim3 grid((unsigned)((nt + kTile - 1) / kTile), kChunks);
-  k_direct<<<grid, kTile, 0, c->stream>>>(c->s_pm.as<double4>(), c->s_st.as<uint8_t>(), c->n, ts.as<int64_t>(), nt,
-                                         c->wconst.as<WalkConst>(), cut, part.as<double4>());
-  k_direct_reduce<<<(unsigned)((nt + 255) / 256), 256, 0, c->stream>>>(part.as<double4>(), nt, d_acc, d_pot);
-  e = cudaGetLastError();
-  cudaStreamSynchronize(c->stream);
-  inv.release();
-  ts.release();
-  part.release();
-  return e;
+  cudaStream_t st     = c->stream;
+  const int64_t n     = c->n;
+  const int64_t ntile = (n + kTileSrc - 1) / kTileSrc, nwarp = (nt + kTgt - 1) / kTgt;
+  // enough warps for several waves whatever the number of targets (at least 8 chunks, at most one
+  // batch of 32 tiles each)
+  int64_t chunks         = 148 * 128 / nwarp;
+  const int64_t nbatch   = (ntile + 31) / 32;
+  chunks                 = chunks < 8 ? 8 : chunks;
+  chunks                 = chunks > nbatch ? nbatch : chunks;
+  // scratch: boxes | chunk sums | inverse order | sorted positions and places (before and after the sort) | sort space
+  size_t tb = 0;
+  GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, (int32_t *)nullptr, (int32_t *)nullptr, (int32_t *)nullptr, (int32_t *)nullptr,
+                                         (int)nt, 0, 31, st));
+  auto up             = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t bytes  = up(ntile * sizeof(TileBox)) + up((size_t)chunks * nt * sizeof(double4)) + up(n * 4) + 4 * up(nt * 4) + up(tb);
+  GG_TRY(c->dir_buf.ensure(bytes));
+  char *q   = c->dir_buf.as<char>();
+  auto take = [&](size_t b) { char *r = q; q += up(b); return r; };
+  TileBox *box  = (TileBox *)take(ntile * sizeof(TileBox));
+  double4 *part = (double4 *)take((size_t)chunks * nt * sizeof(double4));
+  int32_t *inv = (int32_t *)take(n * 4), *ts = (int32_t *)take(nt * 4), *ts2 = (int32_t *)take(nt * 4), *pl = (int32_t *)take(nt * 4),
+          *pl2 = (int32_t *)take(nt * 4);
+  k_invert<<<(unsigned)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368), 256, 0, st>>>(c->perm.as<uint32_t>(), n, inv);
+  k_map_targets<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(d_targets, nt, inv, ts, pl);
+  GG_TRY(cub::DeviceRadixSort::SortPairs(q, tb, ts, ts2, pl, pl2, (int)nt, 0, 31, st));
+  // the reach of a pair: Rcut, or where the exact factor vanishes in double precision and no pair is softened
+  double hmax = 0;
+  for(int i = 0; i < wc.nsoft; i++)
+    hmax = wc.soft[i] > hmax ? wc.soft[i] : hmax;
+  const double r0 = wc.pm ? kUZero / sqrt(wc.asmthinv2) : 0.0, reach = cut ? wc.rcut : (r0 > hmax ? r0 : hmax);
+  if(wc.pm)
+    k_tile_box<<<(unsigned)((ntile + 7) / 8 < 2368 ? (ntile + 7) / 8 : 2368), 256, 0, st>>>(c->s_pm.as<double4>(), n, ntile, box);
+  auto kern = wc.pm ? k_direct<true, false> : wc.ewald ? k_direct<false, true> : k_direct<false, false>;
+  kern<<<dim3((unsigned)((nwarp + kDirectWarps - 1) / kDirectWarps), (unsigned)chunks), 32 * kDirectWarps, 0, st>>>(
+      c->s_pm.as<double4>(), c->s_st.as<uint8_t>(), n, box, ntile, ts2, nt, c->wconst.as<WalkConst>(), cut,
+      reach * reach * (1.0 + 1e-9), part);
+  k_direct_reduce<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(part, (int)chunks, nt, pl2, d_acc, d_pot);
+  return cudaGetLastError();
 }
 }  // namespace gg

@@ -149,6 +149,8 @@ int grid_for(int64_t n, int threads)
   return (int)(b < 1 ? 1 : b);
 }
 
+constexpr size_t kDirectKeep = (size_t)256 << 20;  // working space of gpugrav_direct kept between calls
+
 struct DeviceGuard
 {
   int prev = -1;
@@ -354,7 +356,7 @@ int32_t gpugrav_destroy(gpugrav_ctx *c)
                         &c->g_groups, &c->g_ngroups, &c->g_gpd, &c->g_gseg, &c->g_gflag, &c->g_gid, &c->t_cd, &c->t_pd, &c->m_sys, &c->m_doms,
                         &c->pm_pos, &c->pm_mass, &c->pm_acc, &c->pm_pot, &c->ewd, &c->ewd32, &c->n_mpt, &c->w_mpt,
                         &c->g_mpt, &c->iperm, &c->t_in, &c->t_pos, &c->t_pos_alt, &c->t_idx, &c->t_idx_alt,
-                        &c->cost_in, &c->cost_u, &c->cost_p, &c->slice_rng};
+                        &c->cost_in, &c->cost_u, &c->cost_p, &c->slice_rng, &c->dir_buf, &c->dir_io};
   gg::pm_release(c);
   for(auto *b : bufs)
     b->release();
@@ -1231,10 +1233,11 @@ int32_t gpugrav_direct(gpugrav_ctx *c, int64_t ntargets, const int64_t *targets,
   for(int64_t i = 0; i < ntargets; i++)
     if(targets[i] < 0 || targets[i] >= c->n)
       return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_direct: target index out of range");
-  gg::DevBuf dt, da, dp;
-  if(dt.ensure(ntargets * 8 + 8) != cudaSuccess || da.ensure(ntargets * 24 + 8) != cudaSuccess ||
-     dp.ensure(ntargets * 8 + 8) != cudaSuccess)
+  // targets (ntargets) | accelerations (3 ntargets) | potentials (ntargets), 8 bytes each
+  if(c->dir_io.ensure(ntargets * 40 + 64) != cudaSuccess)
     return fail(c, GPUGRAV_ERR_OOM, "gpugrav_direct: allocation");
+  int64_t *dt = c->dir_io.as<int64_t>();
+  double *da  = c->dir_io.as<double>() + ntargets, *dp = da + 3 * ntargets;
   WalkConst wc;
   make_walk_const(c->prm, &wc);
   if(wc.ewald)
@@ -1245,16 +1248,14 @@ int32_t gpugrav_direct(gpugrav_ctx *c, int64_t ntargets, const int64_t *targets,
       wc.ewd = c->ewd.as<double>();
     }
   CK(cudaMemcpyAsync(c->wconst.p, &wc, sizeof(wc), cudaMemcpyHostToDevice, st), "walk constants");
-  CK(cudaMemcpyAsync(dt.p, targets, ntargets * 8, cudaMemcpyHostToDevice, st), "targets");
-  CK(gg::direct_stage(c, wc, ntargets, dt.as<int64_t>(), mode == GPUGRAV_DIRECT_CUT, da.as<double>(), dp.as<double>()),
-     "direct summation");
-  CK(cudaMemcpyAsync(acc, da.p, ntargets * 24, cudaMemcpyDeviceToHost, st), "download");
+  CK(cudaMemcpyAsync(dt, targets, ntargets * 8, cudaMemcpyHostToDevice, st), "targets");
+  CK(gg::direct_stage(c, wc, ntargets, dt, mode == GPUGRAV_DIRECT_CUT, da, dp), "direct summation");
+  CK(cudaMemcpyAsync(acc, da, ntargets * 24, cudaMemcpyDeviceToHost, st), "download");
   if(pot)
-    CK(cudaMemcpyAsync(pot, dp.p, ntargets * 8, cudaMemcpyDeviceToHost, st), "download");
+    CK(cudaMemcpyAsync(pot, dp, ntargets * 8, cudaMemcpyDeviceToHost, st), "download");
   CK(cudaStreamSynchronize(st), "direct summation");
-  dt.release();
-  da.release();
-  dp.release();
+  if(c->dir_buf.cap > kDirectKeep)  // an exceptionally large call's working space is not kept
+    c->dir_buf.release();
   return GPUGRAV_OK;
 }
 

@@ -248,6 +248,7 @@ struct gpugrav_ctx
   gg::DevBuf acc_s, pot_s, nint_s, oldacc_s, oldacc_in;  // per target (sorted), inputs
   gg::DevBuf out_acc, out_pot, out_nint;      // caller order staging for host copies
   gg::DevBuf scratch;                         // reductions
+  gg::DevBuf dir_buf, dir_io;                 // direct summation: working space; targets and results
   gg::PinnedBuf pinned;
 
   cudaEvent_t ev[20] = {};
