@@ -95,9 +95,23 @@ __global__ void k_extent_partial(const double *__restrict__ pos, int64_t n, int 
     atomicOr(flags, 2);
 }
 
+// one warp per bound (6 warps), the rest by one thread
 __global__ void k_extent_final(const double *partial, int nblocks, BuildConst *bc)
 {
-  if(threadIdx.x != 0 || blockIdx.x != 0)
+  __shared__ double ext[6];
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v = k < 3 ? INFINITY : -INFINITY;
+  for(int b = lane; b < nblocks; b += 32)
+    v = k < 3 ? fmin(v, partial[b * 6 + k]) : fmax(v, partial[b * 6 + k]);
+  for(int o = 16; o > 0; o >>= 1)
+    {
+      const double u = __shfl_xor_sync(0xffffffffu, v, o);
+      v              = k < 3 ? fmin(v, u) : fmax(v, u);
+    }
+  if(lane == 0)
+    ext[k] = v;
+  __syncthreads();
+  if(threadIdx.x != 0)
     return;
   double xmin[3], xmax[3];
   for(int j = 0; j < 3; j++)
@@ -105,15 +119,11 @@ __global__ void k_extent_final(const double *partial, int nblocks, BuildConst *b
       // preset to the simulation box (src/domain/domain_box.c:113-118)
       xmin[j] = 0;
       xmax[j] = bc->box;
+      if(xmin[j] > ext[j])
+        xmin[j] = ext[j];
+      if(xmax[j] < ext[3 + j])
+        xmax[j] = ext[3 + j];
     }
-  for(int b = 0; b < nblocks; b++)
-    for(int j = 0; j < 3; j++)
-      {
-        if(xmin[j] > partial[b * 6 + j])
-          xmin[j] = partial[b * 6 + j];
-        if(xmax[j] < partial[b * 6 + 3 + j])
-          xmax[j] = partial[b * 6 + 3 + j];
-      }
   double len = 0;
   for(int j = 0; j < 3; j++)
     if(__dsub_rn(xmax[j], xmin[j]) > len)
@@ -229,7 +239,7 @@ cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent, int *status_flags)
     {
       k_extent_partial<<<kExtBlocks, kExtThreads, 0, c->stream>>>(c->pos_in.as<double>(), n, c->prm.periodic, c->prm.box_size,
                                                                   c->scratch.as<double>(), flags);
-      k_extent_final<<<1, 32, 0, c->stream>>>(c->scratch.as<double>(), kExtBlocks, bc);
+      k_extent_final<<<1, 192, 0, c->stream>>>(c->scratch.as<double>(), kExtBlocks, bc);
     }
   k_keys<<<grid_for(n, 256), 256, 0, c->stream>>>(c->pos_in.as<double>(), n, bc, c->key.as<u128>(), c->idx.as<uint32_t>(), flags);
   if((e = cudaGetLastError()) != cudaSuccess)

@@ -174,7 +174,8 @@ __device__ __forceinline__ int64_t node_of(const TreeArgs &a, int64_t s, int d)
 // ------------------------------------------------------------------------------
 // Top-level tree for one rank (domain_determineTopTree, src/domain/domain_toplevel.c:111-269,
 // domain_do_local_refine :280-368, domain_walktoptree :381-393), work load = count / N.
-// One thread; particle counts of key ranges by binary search in the sorted keys.
+// One block: the candidates are ranked in parallel and a warp searches the sorted keys for each new
+// cell's first particle (a serial search took 0.1 to 0.3 ms); the choice itself is one thread's loop.
 // ------------------------------------------------------------------------------
 struct TopTmp
 {
@@ -184,15 +185,19 @@ struct TopTmp
   double work;
 };
 
+// first position in [lo, hi) whose key is not below k; the whole warp probes 32 positions at a time
 __device__ int64_t lower_bound_key(const u128 *keys, int64_t lo, int64_t hi, u128 k)
 {
-  while(lo < hi)
+  const int lane = threadIdx.x & 31;
+  while(hi > lo)
     {
-      int64_t m = lo + (hi - lo) / 2;
-      if(keys[m] < k)
-        lo = m + 1;
-      else
-        hi = m;
+      const int64_t len = hi - lo;
+      if(len <= 32)
+        return lo + __popc(__ballot_sync(0xffffffffu, lane < len && keys[lo + (lane < len ? lane : 0)] < k));
+      const int c = __popc(__ballot_sync(0xffffffffu, keys[lo + (lane + 1) * len / 33] < k));
+      const int64_t l = lo;
+      lo              = c > 0 ? l + c * len / 33 + 1 : l;
+      hi              = c < 32 ? l + (c + 1) * len / 33 : hi;
     }
   return lo;
 }
@@ -206,137 +211,141 @@ __device__ bool top_less(const TopTmp *T, int a, int b)
   return a < b;
 }
 
-__global__ void k_toptree(const u128 *__restrict__ keys, int64_t n, double tnf, int mdom, TopTmp *T, int *queue, int *list,
-                          gpugrav_topnode *out, int max_top, int *result)
+constexpr int kTopThreads = 256;
+__global__ void __launch_bounds__(kTopThreads) k_toptree(const u128 *__restrict__ keys, int64_t n, double tnf, int mdom, TopTmp *T, int *queue,
+                                                         int *list, int *sorted, gpugrav_topnode *out, int max_top, int *result)
 {
-  if(threadIdx.x != 0 || blockIdx.x != 0)
-    return;
   const int ntask = 1;
   int a = 1 + (ntask / 7 + 1) * 8, b = (int)(tnf * mdom * ntask);
   int limit_ntop = 2 * (a > b ? a : b);
   if(limit_ntop + 8 > max_top)
     {
-      *result = -1;
+      if(threadIdx.x == 0)
+        *result = -1;
       return;
     }
   double limit = 1.0 / (tnf * mdom * ntask);
-  int nq = 0, ntop = 1, nleaves = 1;
-  T[0].daughter = -1;
-  T[0].size     = (u128)1 << (3 * kBits);
-  T[0].start    = 0;
-  T[0].pindex   = 0;
-  T[0].count    = n;
-  T[0].work     = 1.0;
-  queue[nq++]   = 0;
-  int count;
-  do
+  __shared__ int s_count, s_nq;
+  int nq = 1, ntop = 1, nleaves = 1;
+  if(threadIdx.x == 0)
     {
-      for(int i = 1; i < nq; i++)
-        for(int j = i; j > 0 && top_less(T, queue[j], queue[j - 1]); j--)
-          {
-            int t        = queue[j];
-            queue[j]     = queue[j - 1];
-            queue[j - 1] = t;
-          }
-      count                 = 0;
-      double first_workload = 0;
-      for(int q = 0; q < nq; q++)
-        if(T[queue[q]].size >= 8)
-          {
-            first_workload = T[queue[q]].work;
-            break;
-          }
-      for(int q = 0; q < nq; q++)
+      T[0].daughter = -1;
+      T[0].size     = (u128)1 << (3 * kBits);
+      T[0].start    = 0;
+      T[0].pindex   = 0;
+      T[0].count    = n;
+      T[0].work     = 1.0;
+      queue[0]      = 0;
+    }
+  __syncthreads();
+  while(true)
+    {
+      // the queue by decreasing work, then index
+      for(int q = threadIdx.x; q < nq; q += kTopThreads)
         {
-          int np = queue[q];
-          if(T[np].work < 0.125 * first_workload)
-            break;
-          if(ntop + 8 * (count + 1) >= limit_ntop)
-            break;
-          if(T[np].work > limit || (nleaves < mdom * ntask && count == 0))
+          const int me = queue[q];
+          int rank     = 0;
+          for(int p = 0; p < nq; p++)
+            rank += top_less(T, queue[p], me) ? 1 : 0;
+          sorted[rank] = me;
+        }
+      __syncthreads();
+      for(int q = threadIdx.x; q < nq; q += kTopThreads)
+        queue[q] = sorted[q];
+      if(threadIdx.x == 0)
+        {
+          int count             = 0;
+          double first_workload = 0;
+          for(int q = 0; q < nq; q++)
+            if(T[sorted[q]].size >= 8)
+              {
+                first_workload = T[sorted[q]].work;
+                break;
+              }
+          for(int q = 0; q < nq; q++)
             {
-              if(T[np].size < 8)
+              int np = sorted[q];
+              if(T[np].work < 0.125 * first_workload)
+                break;
+              if(ntop + 8 * (count + 1) >= limit_ntop)
+                break;
+              if(T[np].work > limit || (nleaves < mdom * ntask && count == 0))
                 {
-                  *result = -2;  // the reference stops here: PEANOGRID not fine enough
-                  return;
+                  if(T[np].size < 8)
+                    {
+                      count = -1;  // the reference stops here: PEANOGRID not fine enough
+                      break;
+                    }
+                  list[count++] = np;
                 }
-              list[count++] = np;
+            }
+          s_count = count;
+        }
+      __syncthreads();
+      const int count = s_count;
+      if(count < 0)
+        {
+          if(threadIdx.x == 0)
+            *result = -2;
+          return;
+        }
+      if(count == 0)
+        break;
+      // eight daughters each: first particle of every daughter (a warp per daughter), then the counts
+      for(int it = threadIdx.x >> 5; it < 8 * count; it += kTopThreads / 32)
+        {
+          const int i = list[it >> 3], j = it & 7, sub = ntop + it;
+          const u128 size  = T[i].size >> 3;
+          const u128 start = T[i].start + (u128)j * size;
+          const int64_t f  = lower_bound_key(keys, T[i].pindex, T[i].pindex + T[i].count, start);
+          if((threadIdx.x & 31) == 0)
+            {
+              T[sub].daughter = -1;
+              T[sub].size     = size;
+              T[sub].start    = start;
+              T[sub].pindex   = f;
             }
         }
-      if(count > 0)
+      __syncthreads();
+      for(int it = threadIdx.x; it < 8 * count; it += kTopThreads)
         {
-          for(int k = 0; k < count; k++)
-            {
-              int i         = list[k];
-              T[i].daughter = ntop;
-              ntop += 8;
-              nleaves += 7;
-              int64_t lo = T[i].pindex, hi = T[i].pindex + T[i].count;
-              int64_t first[9];
-              for(int j = 0; j < 8; j++)
-                {
-                  int sub         = T[i].daughter + j;
-                  T[sub].daughter = -1;
-                  T[sub].size     = T[i].size >> 3;
-                  T[sub].start    = T[i].start + (u128)j * T[sub].size;
-                  first[j]        = lower_bound_key(keys, lo, hi, T[sub].start);
-                }
-              first[8] = hi;
-              for(int j = 0; j < 8; j++)
-                {
-                  int sub       = T[i].daughter + j;
-                  T[sub].pindex = first[j];
-                  T[sub].count  = first[j + 1] - first[j];
-                  T[sub].work   = (double)T[sub].count / (double)n;
-                }
-            }
+          const int i = list[it >> 3], sub = ntop + it;
+          const int64_t next = (it & 7) < 7 ? T[sub + 1].pindex : T[i].pindex + T[i].count;
+          T[sub].count       = next - T[sub].pindex;
+          T[sub].work        = (double)T[sub].count / (double)n;
+          if((it & 7) == 0)
+            T[i].daughter = sub;
+        }
+      __syncthreads();
+      if(threadIdx.x == 0)
+        {
           int w = 0;
           for(int q = 0; q < nq; q++)
             if(T[queue[q]].daughter < 0)
               queue[w++] = queue[q];
-          nq = w;
-          for(int k = 0; k < count; k++)
-            for(int j = 0; j < 8; j++)
-              queue[nq++] = T[list[k]].daughter + j;
+          for(int it = 0; it < 8 * count; it++)
+            queue[w++] = ntop + it;
+          s_nq = w;
         }
+      ntop += 8 * count;
+      nleaves += 7 * count;
+      __syncthreads();
+      nq = s_nq;
     }
-  while(count > 0);
+  __syncthreads();
 
-  // leaf numbering in Peano-Hilbert order (domain_walktoptree): iterative DFS
-  int stack[3 * kBits + 8], sp = 0, leaves = 0;
-  int child[3 * kBits + 8];
-  stack[sp] = 0;
-  child[sp] = 0;
-  if(T[0].daughter < 0)
-    T[0].leaf = leaves++;
-  else
-    {
-      sp = 1;
-      while(sp > 0)
-        {
-          int nd = stack[sp - 1];
-          if(child[sp - 1] == 8)
-            {
-              sp--;
-              continue;
-            }
-          int c = T[nd].daughter + child[sp - 1]++;
-          if(T[c].daughter < 0)
-            T[c].leaf = leaves++;
-          else
-            {
-              stack[sp] = c;
-              child[sp] = 0;
-              sp++;
-            }
-        }
-    }
-  if(T[0].daughter >= 0)
-    {
-      // the DFS above started with stack[0] = root
-    }
+  // leaf numbering in Peano-Hilbert order (domain_walktoptree): the leaves partition the key space, so
+  // a leaf's number is the count of leaves that start before it
+  for(int i = threadIdx.x; i < ntop; i += kTopThreads)
+    if(T[i].daughter < 0)
+      {
+        int leaf = 0;
+        for(int l = 0; l < ntop; l++)
+          leaf += (T[l].daughter < 0 && T[l].start < T[i].start) ? 1 : 0;
+        T[i].leaf = leaf;
+      }
 
-  for(int i = 0; i < ntop; i++)
+  for(int i = threadIdx.x; i < ntop; i += kTopThreads)
     {
       out[i].start_key_hi = (uint64_t)(T[i].start >> 64);
       out[i].start_key_lo = (uint64_t)T[i].start;
@@ -367,114 +376,122 @@ __global__ void k_toptree(const u128 *__restrict__ keys, int64_t n, double tnf, 
           out[i].morton_to_peano[morton] = (uint8_t)(c_ph_tree.e[state * 8 + oct] & 7);
         }
     }
-  *result = ntop;
+  if(threadIdx.x == 0)
+    *result = ntop;
 }
 
 // ------------------------------------------------------------------------------
 // Skeleton: force_create_empty_nodes (src/gravity/forcetree.c:1131-1180), iteratively,
-// creating nodes in the same order (i, j, k loops, depth first).  One thread.
-// Relative node 0 is the root (len DomainLen, centre DomainCenter).
+// creating nodes in the same order (i, j, k loops, depth first).  Relative node 0 is the root (len
+// DomainLen, centre DomainCenter).  One block: the depth-first creation is one thread's, on shared copies
+// of the top nodes, of the cells and of the leaf table where they fit (the chain of dependent reads took
+// 35 us from global memory); validation and output are everyone's.
 // ------------------------------------------------------------------------------
-__global__ void k_skeleton(const gpugrav_topnode *__restrict__ top, int ntop, const BuildConst *__restrict__ bc,
-                           int32_t *__restrict__ suns, double4 *__restrict__ cl, uint8_t *__restrict__ depth,
-                           int32_t *__restrict__ leafnode, int32_t *__restrict__ nodetop, SkelInfo *info)
+constexpr int kSkelThreads = 128, kSkelShared = 256;
+__global__ void __launch_bounds__(kSkelThreads) k_skeleton(const gpugrav_topnode *__restrict__ top_g, int ntop, const BuildConst *__restrict__ bc,
+                                                           int32_t *__restrict__ suns, double4 *__restrict__ cl_g, uint8_t *__restrict__ depth,
+                                                           int32_t *__restrict__ leafnode, int32_t *__restrict__ nodetop, SkelInfo *info)
 {
-  if(threadIdx.x != 0 || blockIdx.x != 0)
-    return;
-  info->status = 0;
-  int nleaves  = 0;
-  for(int t = 0; t < ntop; t++)
+  __shared__ gpugrav_topnode top_sh[kSkelShared];
+  __shared__ double4 cl_sh[kSkelShared];
+  __shared__ int s_leaves, s_bad;
+  const bool fits            = ntop <= kSkelShared;
+  const gpugrav_topnode *top = fits ? top_sh : top_g;
+  double4 *cl                = fits ? cl_sh : cl_g;
+  if(threadIdx.x == 0)
+    s_leaves = s_bad = 0;
+  __syncthreads();
+  for(int t = threadIdx.x; t < ntop; t += kSkelThreads)
     {
-      if(top[t].daughter >= 0)
-        {
-          if(top[t].daughter <= t || top[t].daughter + 8 > ntop)
-            {
-              info->status = -2;
-              return;
-            }
-        }
-      else
-        {
-          nleaves++;
-        }
+      const gpugrav_topnode tn = top_g[t];
+      if(fits)
+        top_sh[t] = tn;
+      if(tn.daughter < 0)
+        atomicAdd(&s_leaves, 1);
+      else if(tn.daughter <= t || tn.daughter + 8 > ntop)
+        s_bad = 1;
     }
-  for(int t = 0; t < ntop; t++)
+  __syncthreads();
+  const int nleaves = s_leaves;
+  for(int t = threadIdx.x; t < ntop; t += kSkelThreads)
     if(top[t].daughter < 0 && (top[t].leaf < 0 || top[t].leaf >= nleaves))
-      {
-        info->status = -2;
-        return;
-      }
-  for(int l = 0; l < nleaves; l++)
+      s_bad = 1;
+  for(int l = threadIdx.x; l < nleaves; l += kSkelThreads)
     leafnode[l] = -1;
-
-  const gpugrav_domain &dom = bc->dom;
-  for(int j = 0; j < 8; j++)
-    suns[j] = -1;
-  cl[0]    = make_double4(dom.center[0], dom.center[1], dom.center[2], dom.len);
-  depth[0] = 0;
-  nodetop[0] = 0;
-  int numnodes = 1;
-  if(top[0].daughter < 0)
-    leafnode[top[0].leaf] = 0;
-
-  struct Frame
-  {
-    int no, topnode, bits, ijk;
-    uint64_t x, y, z;
-  };
-  Frame st[3 * kBits + 8];
-  int sp      = 0;
-  st[sp++]    = Frame{0, 0, 1, 0, 0, 0, 0};
-  int maxd    = 0;
-  while(sp > 0)
+  for(int64_t q = threadIdx.x; q < 8 * (int64_t)ntop; q += kSkelThreads)
+    suns[q] = -1;
+  __syncthreads();
+  if(s_bad)
     {
-      Frame &f = st[sp - 1];
-      if(top[f.topnode].daughter < 0 || f.ijk == 8)
-        {
-          sp--;
-          continue;
-        }
-      int i = (f.ijk >> 2) & 1, j = (f.ijk >> 1) & 1, k = f.ijk & 1;
-      f.ijk++;
-      if(numnodes >= ntop)
-        {
-          info->status = -2;
-          return;
-        }
-      int sub   = ph_last_digit_dev(c_ph_tree.e, (f.x << 1) + i, (f.y << 1) + j, (f.z << 1) + k, f.bits);
-      int count = i + 2 * j + 4 * k;
-      int nf    = numnodes++;
-      suns[8 * f.no + count] = (int32_t)(nf + bc->n);  // slots hold global indices: nodes start at n
-      double4 p      = cl[f.no];
-      double lenhalf = __dmul_rn(0.25, p.w);
-      cl[nf] = make_double4(__dadd_rn(p.x, __dmul_rn((double)(2 * i - 1), lenhalf)),
-                            __dadd_rn(p.y, __dmul_rn((double)(2 * j - 1), lenhalf)),
-                            __dadd_rn(p.z, __dmul_rn((double)(2 * k - 1), lenhalf)), __dmul_rn(0.5, p.w));
-      for(int q = 0; q < 8; q++)
-        suns[8 * nf + q] = -1;
-      depth[nf] = (uint8_t)(depth[f.no] + 1);
-      if(depth[nf] > maxd)
-        maxd = depth[nf];
-      int d = top[f.topnode].daughter + sub;
-      nodetop[nf] = d;
-      if(top[d].daughter == -1)
-        leafnode[top[d].leaf] = nf;
-      if(sp >= 3 * kBits + 8)
-        {
-          info->status = -2;
-          return;
-        }
-      st[sp++] = Frame{nf, d, f.bits + 1, 0, 2 * f.x + i, 2 * f.y + j, 2 * f.z + k};
-    }
-  for(int l = 0; l < nleaves; l++)
-    if(leafnode[l] < 0)
-      {
+      if(threadIdx.x == 0)
         info->status = -2;
-        return;
-      }
-  info->ntop_nodes    = numnodes;
-  info->nleaves       = nleaves;
-  info->max_top_depth = maxd;
+      return;
+    }
+  if(threadIdx.x == 0)
+    {
+      const gpugrav_domain dom = bc->dom;
+      const int64_t n          = bc->n;
+      cl[0]                    = make_double4(dom.center[0], dom.center[1], dom.center[2], dom.len);
+      depth[0]                 = 0;
+      nodetop[0]               = 0;
+      int numnodes = 1, maxd = 0, bad = 0;
+      if(top[0].daughter < 0)
+        leafnode[top[0].leaf] = 0;
+      struct Frame
+      {
+        int no, topnode, state, ijk;  // state: of the Peano-Hilbert curve in the node's cell
+      };
+      Frame st[3 * kBits + 8];
+      int sp   = 0;
+      st[sp++] = Frame{0, 0, 0, 0};
+      while(sp > 0)
+        {
+          Frame &f = st[sp - 1];
+          if(top[f.topnode].daughter < 0 || f.ijk == 8)
+            {
+              sp--;
+              continue;
+            }
+          int i = (f.ijk >> 2) & 1, j = (f.ijk >> 1) & 1, k = f.ijk & 1;
+          const unsigned e = c_ph_tree.e[f.state * 8 + f.ijk];  // octant (x << 2) | (y << 1) | z
+          f.ijk++;
+          if(numnodes >= ntop || sp >= 3 * kBits + 8)
+            {
+              bad = 1;
+              break;
+            }
+          int count = i + 2 * j + 4 * k;
+          int nf    = numnodes++;
+          suns[8 * f.no + count] = (int32_t)(nf + n);  // slots hold global indices: nodes start at n
+          double4 p      = cl[f.no];
+          double lenhalf = __dmul_rn(0.25, p.w);
+          cl[nf] = make_double4(__dadd_rn(p.x, __dmul_rn((double)(2 * i - 1), lenhalf)),
+                                __dadd_rn(p.y, __dmul_rn((double)(2 * j - 1), lenhalf)),
+                                __dadd_rn(p.z, __dmul_rn((double)(2 * k - 1), lenhalf)), __dmul_rn(0.5, p.w));
+          depth[nf] = (uint8_t)sp;  // the parent's depth is sp - 1
+          maxd      = sp > maxd ? sp : maxd;
+          int d       = top[f.topnode].daughter + (int)(e & 7);
+          nodetop[nf] = d;
+          if(top[d].daughter == -1)
+            leafnode[top[d].leaf] = nf;
+          st[sp++] = Frame{nf, d, (int)(e >> 3), 0};
+        }
+      s_bad               = bad;
+      info->ntop_nodes    = numnodes;
+      info->nleaves       = nleaves;
+      info->max_top_depth = maxd;
+      s_leaves            = numnodes;
+    }
+  __syncthreads();
+  for(int l = threadIdx.x; l < nleaves; l += kSkelThreads)
+    if(leafnode[l] < 0)
+      s_bad = 1;
+  if(fits)
+    for(int t = threadIdx.x; t < s_leaves; t += kSkelThreads)
+      cl_g[t] = cl_sh[t];
+  __syncthreads();
+  if(threadIdx.x == 0)
+    info->status = s_bad ? -2 : 0;
 }
 
 // top leaf of every sorted particle: walk TopNodes with MortonToPeanoSubnode
@@ -1061,15 +1078,15 @@ cudaError_t toptree_stage(gpugrav_ctx *c, int *status)
   GG_TRY(ensure_ph(c->device));
   const int max_top = kMaxTop;
   GG_TRY(c->top.ensure(max_top * sizeof(gpugrav_topnode)));
-  GG_TRY(c->scratch.ensure(max_top * (sizeof(TopTmp) + 2 * sizeof(int)) + 256));
+  GG_TRY(c->scratch.ensure(max_top * (sizeof(TopTmp) + 3 * sizeof(int)) + 256));
   GG_TRY(c->counters.ensure(64 * sizeof(int)));
   char *s     = (char *)c->scratch.p;
   TopTmp *T   = (TopTmp *)s;
   int *queue  = (int *)(s + max_top * sizeof(TopTmp));
   int *list   = queue + max_top;
   int *result = c->counters.as<int>() + 8;
-  k_toptree<<<1, 32, 0, c->stream>>>(c->key_alt.as<u128>(), c->n, c->prm.top_node_factor, c->prm.multiple_domains, T, queue,
-                                      list, c->top.as<gpugrav_topnode>(), max_top, result);
+  k_toptree<<<1, kTopThreads, 0, c->stream>>>(c->key_alt.as<u128>(), c->n, c->prm.top_node_factor, c->prm.multiple_domains, T, queue,
+                                              list, list + max_top, c->top.as<gpugrav_topnode>(), max_top, result);
   GG_TRY(cudaGetLastError());
   int r = 0;
   GG_TRY(cudaMemcpyAsync(&r, result, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1181,7 +1198,7 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
     }
   else
     {
-      k_skeleton<<<1, 32, 0, st>>>(c->top.as<gpugrav_topnode>(), ntop, c->bconst.as<BuildConst>(), c->n_suns.as<int32_t>(),
+      k_skeleton<<<1, kSkelThreads, 0, st>>>(c->top.as<gpugrav_topnode>(), ntop, c->bconst.as<BuildConst>(), c->n_suns.as<int32_t>(),
                                     c->n_cl.as<double4>(), c->n_depth.as<uint8_t>(), leafnode, nodetop, sinfo);
       launches++;
       SkelInfo si;
@@ -1289,7 +1306,7 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
         k_roots<<<grid_for(ntop, 128), 128, 0, st>>>(ntop, mdoms, c->n_suns.as<int32_t>(), c->n_cl.as<double4>(),
                                                       c->n_depth.as<uint8_t>());
       else
-        k_skeleton<<<1, 32, 0, st>>>(c->top.as<gpugrav_topnode>(), ntop, c->bconst.as<BuildConst>(), c->n_suns.as<int32_t>(),
+        k_skeleton<<<1, kSkelThreads, 0, st>>>(c->top.as<gpugrav_topnode>(), ntop, c->bconst.as<BuildConst>(), c->n_suns.as<int32_t>(),
                                       c->n_cl.as<double4>(), c->n_depth.as<uint8_t>(), leafnode, nodetop, sinfo);
       launches++;
     }
