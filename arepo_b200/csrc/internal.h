@@ -242,7 +242,8 @@ struct gpugrav_ctx
   gg::DevBuf m_sys, m_doms;
   // FP32 walk launch plan (walk32_prepare)
   void *w32_kernel   = nullptr;
-  int32_t w32_blocks = 0;
+  int32_t w32_blocks = 0, w32_threads = 0;
+  size_t w32_smem    = 0;
   bool want_pot       = true;  // potential requested by the current walk call
   int walk32_tpl      = 0;     // targets per lane of the group walk: 0 auto, 1 or 2 (GPUGRAV_WALK32_TPL)
   gg::DevBuf acc_s, pot_s, nint_s, oldacc_s, oldacc_in;  // per target (sorted), inputs

@@ -23,36 +23,38 @@
 // (depth, depth-first position)), particles grouped by parent node.
 #include <cub/cub.cuh>
 
+#include <type_traits>
+
 #include "internal.h"
 
 namespace gg
 {
 namespace
 {
-#ifndef GG_W32_WARPS
-#define GG_W32_WARPS 4
-#endif
 #ifndef GG_W32_EVAL_AT
 #define GG_W32_EVAL_AT 192
 #endif
 #ifndef GG_W32_UNROLL
 #define GG_W32_UNROLL 8
 #endif
-constexpr int kWarps   = GG_W32_WARPS;    // warps per block
-constexpr int kEvalAt  = GG_W32_EVAL_AT;  // evaluate once this many entries are queued
-#ifndef GG_W32_MINBLOCKS
-#define GG_W32_MINBLOCKS 7  // blocks per SM the register budget is sized for (72 registers a thread, 31 KB of shared memory a block)
-#endif
-// two targets per lane: fewer entries in flight, 80 registers (6 blocks per SM, 35 KB of shared memory a block)
 #ifndef GG_W32_UNROLL2
 #define GG_W32_UNROLL2 4
 #endif
-#ifndef GG_W32_MINBLOCKS2
-#define GG_W32_MINBLOCKS2 6
-#endif
+constexpr int kEvalAt  = GG_W32_EVAL_AT;  // evaluate once this many entries are queued
 // list entries in flight per lane in the evaluation loop
 template <int TPL>
 constexpr int kUnroll = TPL == 2 ? GG_W32_UNROLL2 : GG_W32_UNROLL;
+// Launch shape.  The FP32 TreePM walk keeps kCopies copies of the short-range table in shared memory
+// (see TabF), 16 KB that one block per SM can afford and six small ones cannot: one block of 24 warps
+// with two targets per lane (80 registers a thread), 28 warps with one (72 registers).  The others
+// need no table copies: blocks of 4 warps, 6 or 7 (FP64 form: 3) per SM.
+template <typename R, bool PERIODIC, int TPL>
+struct Shape
+{
+  static constexpr bool big   = sizeof(R) == 4 && PERIODIC;
+  static constexpr int warps  = big ? (TPL == 2 ? 24 : 28) : 4;
+  static constexpr int blocks = big ? 1 : (sizeof(R) == 4 ? (TPL == 2 ? 6 : 7) : 3);
+};
 // capacity (Cap below): accepted nodes (<= 32) join a list holding fewer than kEvalAt entries;
 // particles are added at most 32 per round and the list is evaluated first whenever a round could
 // overflow it.  Entries inside some target's softening length go to a separate, smaller near list,
@@ -134,7 +136,6 @@ struct W32Const
   float theta2, erracc;
   int periodic, bh;
   float soft[GPUGRAV_MAX_SOFTTYPES + 1];
-  float4 tab[kNtab + 1];  // (f[i], f[i+1] - f[i], p[i], p[i+1] - p[i]): force table times 1/Asmth^2, potential table
   const float4 *ewd;       // Ewald correction (fx, fy, fz, pot) per table entry (pure periodic tree)
   float ewd_fac;           // 2 EN / L
   int mns;                 // MULTIPLE_NODE_SOFTENING: nodes used per softening type
@@ -143,11 +144,32 @@ struct W32Const
   int minangle;            // ACTIVATE_MINIMUM_OPENING_ANGLE
   // FP64 form only (the FP32 kernels do not copy these into shared memory)
   double rcut2_d, asmthfac_d;  // Rcut^2 and the table index factor in double
-  double4 tab64[kNtab + 1];    // the table above in double
+  double4 tab64[kNtab + 1];    // the table below in double
+  // (f[i], f[i+1] - f[i], p[i], p[i+1] - p[i]): force table times 1/Asmth^2, potential table (FP32 form)
+  float4 tab[kNtab + 1];
 };
 // bytes of the constants a kernel of arithmetic type R keeps in shared memory
 template <typename R>
-constexpr int kW32Bytes = sizeof(R) == 4 ? (int)offsetof(W32Const, rcut2_d) : (int)sizeof(W32Const);
+constexpr int kW32Bytes = sizeof(R) == 4 ? (int)offsetof(W32Const, rcut2_d) : (int)offsetof(W32Const, tab);
+
+// The FP32 short-range table in shared memory: every pair of the evaluation reads one 16-byte row at an
+// index of its own, and a 16-byte load is served a quarter-warp at a time, each lane from one of the 8
+// groups of 4 banks.  With one copy of the table the lanes of a quarter collide (measured: about 9
+// wavefronts per warp and pair, which bounded the whole walk); with one copy per bank group lane q reads
+// copy q mod 8 and a load takes its 4 wavefronts.
+constexpr int kCopies = 8;
+struct TabF
+{
+  float4 row[(kNtab + 1) * kCopies];
+};
+struct TabNone
+{
+};
+// what short_range reads: the lane's copy of the table (FP32), or nothing
+struct TabRef
+{
+  const float4 *row;
+};
 
 // ------------------------------------------------------------------------------
 // layout
@@ -225,11 +247,21 @@ __global__ void k_g_fill(int64_t nn, int64_t n, const int32_t *__restrict__ sort
 // ------------------------------------------------------------------------------
 // walk
 // ------------------------------------------------------------------------------
+// nearest image (only the few separations beyond half a box take the branch)
+template <bool WRAP>
 __device__ __forceinline__ double wrapd(double d, const W32Const &w)
 {
-  if(!w.periodic)
-    return d;
-  return (d > w.half_box) ? d - w.box : ((d < -w.half_box) ? d + w.box : d);
+  if(WRAP && fabs(d) > w.half_box)
+    d -= copysign(w.box, d);
+  return d;
+}
+
+// 32 bytes in one load (32-byte aligned)
+__device__ __forceinline__ double4 load32(const double4 *p)
+{
+  double4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
 }
 
 __device__ __forceinline__ double wmin(double v)
@@ -288,18 +320,18 @@ __device__ __forceinline__ double rcut2_of(const W32Const &w, double) { return w
 // is clamped to the last interval, which only entries beyond Rcut reach (they are masked); without
 // CLAMP the entry is inside Rcut, so floor(te) <= NTAB (the table has NTAB + 1 rows).
 template <bool CLAMP = true>
-__device__ __forceinline__ void short_range(float r, const W32Const &w, float &ff, float &fpt)
+__device__ __forceinline__ void short_range(float r, const W32Const &w, TabRef tab, float &ff, float &fpt)
 {
   const float tr  = __fmaf_rd(r, w.asmthfac, 12582912.0f);
   const float tb0 = CLAMP ? fminf(tr, 12582912.0f + (float)(kNtab - 1)) : tr;
   const float tw  = fmaf(r, w.asmthfac, 12582912.0f - tb0);
-  const float4 t  = w.tab[__float_as_int(tb0) - 0x4B400000];
+  const float4 t  = tab.row[(__float_as_int(tb0) - 0x4B400000) * kCopies];
   ff              = fmaf(tw, t.y, t.x);
   fpt             = fmaf(tw, t.w, t.z);
 }
 // the same in double: floor(te) by conversion
 template <bool CLAMP = true>
-__device__ __forceinline__ void short_range(double r, const W32Const &w, double &ff, double &fpt)
+__device__ __forceinline__ void short_range(double r, const W32Const &w, TabRef, double &ff, double &fpt)
 {
   const double te = r * w.asmthfac_d;
   int i           = (int)te;
@@ -377,7 +409,7 @@ __device__ __forceinline__ Sep<R> separation(const V4<R> e, const Tgt<R> &T)
 // entry is known to lie outside the softening length of every target of the group.  The Ewald
 // correction (EWALD: pure periodic tree, nearest image) is taken here for every pair.
 template <typename R, bool PERIODIC, bool POT, bool EWALD = false, bool CHECK = true, bool MASK = true>
-__device__ __forceinline__ bool far(const V4<R> e, const R hj, Tgt<R> &T, const W32Const &w)
+__device__ __forceinline__ bool far(const V4<R> e, const R hj, Tgt<R> &T, const W32Const &w, TabRef tab)
 {
   constexpr bool PAIRWISE = MASK || CHECK;  // Rcut mask and count per pair
   // outside every target's softening length (no CHECK) r > 0 unless the softening is zero
@@ -388,7 +420,7 @@ __device__ __forceinline__ bool far(const V4<R> e, const R hj, Tgt<R> &T, const 
     {
       if(PAIRWISE)
         in = s.r2 < rcut2_of(w, R(0));
-      short_range<PAIRWISE>(s.r, w, ff, fpt);
+      short_range<PAIRWISE>(s.r, w, tab, ff, fpt);
     }
   // force m (1/r^3 + f_s / (r Asmth^2)) = (m/r) (1/r^2 + f_s'), potential (m/r) p_s (Newtonian: -m/r);
   // 1/r^2 stays finite at the clamped r = 0, so masking m/r masks both
@@ -419,7 +451,7 @@ __device__ __forceinline__ bool far(const V4<R> e, const R hj, Tgt<R> &T, const 
 // (nothing otherwise): the reference's spline (src/gravity/forcetree_walk.c:421-455), plus the
 // TreePM short-range correction of the Newtonian part away from r = 0.
 template <typename R, bool PERIODIC, bool POT>
-__device__ __forceinline__ void near(const V4<R> e, const R hj, Tgt<R> &T, const W32Const &w)
+__device__ __forceinline__ void near(const V4<R> e, const R hj, Tgt<R> &T, const W32Const &w, TabRef tab)
 {
   const Sep<R> s = separation<R>(e, T);
   const R hmax   = maxR(T.h, hj);
@@ -450,7 +482,7 @@ __device__ __forceinline__ void near(const V4<R> e, const R hj, Tgt<R> &T, const
       if(s.r > R(0))
         {
           R ff, fpt;
-          short_range(s.r, w, ff, fpt);
+          short_range(s.r, w, tab, ff, fpt);
           fac = fmaR(s.rinv, ff, fac);
           if(POT)
             wp = fmaR(s.rinv, fpt + R(1), wp);
@@ -495,7 +527,7 @@ namespace
 // is revisited for those pairs.  MASK: per-pair Rcut mask and count (see far()).
 template <typename R, bool PERIODIC, bool POT, int TPL, bool EWALD, bool CHECK, bool MASK>
 __device__ __forceinline__ void evaluate_region(const V4<R> *__restrict__ LP, const R *__restrict__ LH, int nl, Tgt<R> (&T)[TPL],
-                                                const W32Const &w)
+                                                const W32Const &w, TabRef tab)
 {
   int j = 0;
   constexpr int U = kUnroll<TPL>;
@@ -514,7 +546,7 @@ __device__ __forceinline__ void evaluate_region(const V4<R> *__restrict__ LP, co
       for(int u = 0; u < U; u++)
 #pragma unroll
         for(int k = 0; k < TPL; k++)
-          soft |= far<R, PERIODIC, POT, EWALD, CHECK, MASK>(e[u], hj[u], T[k], w);
+          soft |= far<R, PERIODIC, POT, EWALD, CHECK, MASK>(e[u], hj[u], T[k], w, tab);
       if(CHECK && soft)
         {
 #pragma unroll 1
@@ -524,7 +556,7 @@ __device__ __forceinline__ void evaluate_region(const V4<R> *__restrict__ LP, co
               const R hu     = LH[j + u];
 #pragma unroll
               for(int k = 0; k < TPL; k++)
-                near<R, PERIODIC, POT>(eu, hu, T[k], w);
+                near<R, PERIODIC, POT>(eu, hu, T[k], w, tab);
             }
         }
     }
@@ -534,9 +566,137 @@ __device__ __forceinline__ void evaluate_region(const V4<R> *__restrict__ LP, co
       const R hj    = CHECK ? LH[j] : R(0);
 #pragma unroll
       for(int k = 0; k < TPL; k++)
-        if(far<R, PERIODIC, POT, EWALD, CHECK, MASK>(e, hj, T[k], w) && CHECK)
-          near<R, PERIODIC, POT>(e, hj, T[k], w);
+        if(far<R, PERIODIC, POT, EWALD, CHECK, MASK>(e, hj, T[k], w, tab) && CHECK)
+          near<R, PERIODIC, POT>(e, hj, T[k], w, tab);
     }
+}
+
+// ---- packed evaluation: the lane's two targets as the halves of 64-bit register pairs ----
+// Blackwell's f32x2 instructions do the same IEEE operation on both halves, so a pair's sums are bitwise
+// those of far().  They keep the FP32 pipe's rate (two cycles each) but take one issue slot for two
+// operations, which leaves slots to the warps that traverse.  Per entry and two targets, 24 warps per SM,
+// measured apart from the walk: scalar 48.3 instructions and 14.2 SM cycles, packed 32.1 and 13.1 (without
+// a short-range table 30.3 and 9.0 against 17.3 and 7.6); the FP32 operations alone take 9.5 (6.5).
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b)
+{
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void upk(f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c)
+{
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 fma2_rd(f2 a, f2 b, f2 c)
+{
+  f2 r;
+  asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b)
+{
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b)
+{
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+struct Sum2
+{
+  f2 ax, ay, az, pot;
+};
+
+// far() without CHECK for the lane's two targets at once (outside every target's softening length); N: the
+// targets' negated positions
+template <bool PERIODIC, bool POT, bool MASK>
+__device__ __forceinline__ void far2(const float4 e, const f2 (&N)[3], Tgt<float> (&T)[2], Sum2 &S, const W32Const &w, TabRef tab, f2 afac,
+                                     f2 big)
+{
+  const f2 dx = add2(pk(e.x, e.x), N[0]), dy = add2(pk(e.y, e.y), N[1]), dz = add2(pk(e.z, e.z), N[2]);
+  const f2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+  float r2a, r2b;
+  upk(r2, r2a, r2b);
+  const float ra = rsqrt_normal(r2a), rb = rsqrt_normal(r2b);
+  const f2 rinv = pk(ra, rb);
+  float ma = e.w, mb = e.w;
+  if(PERIODIC)
+    {
+      const f2 r = mul2(r2, rinv);
+      f2 tb      = fma2_rd(r, afac, big);
+      float ta, tc;
+      upk(tb, ta, tc);
+      if(MASK)
+        {
+          const bool ina = r2a < w.rcut2, inb = r2b < w.rcut2;
+          ma = ina ? e.w : 0.0f;
+          mb = inb ? e.w : 0.0f;
+          T[0].ni += ina ? 1 : 0;
+          T[1].ni += inb ? 1 : 0;
+          ta = fminf(ta, 12582912.0f + (float)(kNtab - 1));
+          tc = fminf(tc, 12582912.0f + (float)(kNtab - 1));
+          tb = pk(ta, tc);
+        }
+      const float4 qa = tab.row[(__float_as_int(ta) - 0x4B400000) * kCopies], qb = tab.row[(__float_as_int(tc) - 0x4B400000) * kCopies];
+      float wa, wb;
+      upk(fma2(r, afac, fma2(tb, pk(-1.0f, -1.0f), big)), wa, wb);
+      const f2 ff = pk(fmaf(wa, qa.y, qa.x), fmaf(wb, qb.y, qb.x));
+      const f2 mr = mul2(pk(ma, mb), rinv);
+      const f2 fm = mul2(mr, fma2(rinv, rinv, ff));
+      S.ax        = fma2(dx, fm, S.ax);
+      S.ay        = fma2(dy, fm, S.ay);
+      S.az        = fma2(dz, fm, S.az);
+      if(POT)
+        S.pot = fma2(mr, pk(fmaf(wa, qa.w, qa.z), fmaf(wb, qb.w, qb.z)), S.pot);
+    }
+  else
+    {
+      const f2 mr = mul2(pk(ma, mb), rinv);
+      const f2 fm = mul2(mr, mul2(rinv, rinv));
+      S.ax        = fma2(dx, fm, S.ax);
+      S.ay        = fma2(dy, fm, S.ay);
+      S.az        = fma2(dz, fm, S.az);
+      if(POT)
+        S.pot = fma2(mr, pk(-1.0f, -1.0f), S.pot);
+    }
+}
+
+// evaluate_region without CHECK for two FP32 targets per lane
+template <bool PERIODIC, bool POT, bool MASK>
+__device__ __forceinline__ void evaluate_region2(const float4 *__restrict__ LP, int nl, Tgt<float> (&T)[2], const W32Const &w, TabRef tab)
+{
+  constexpr int U = kUnroll<2>;
+  Sum2 S;
+  S.ax  = pk(T[0].ax, T[1].ax);
+  S.ay  = pk(T[0].ay, T[1].ay);
+  S.az  = pk(T[0].az, T[1].az);
+  S.pot = pk(T[0].pot, T[1].pot);
+  const f2 afac = pk(w.asmthfac, w.asmthfac), big = pk(12582912.0f, 12582912.0f);
+  const f2 N[3] = {pk(-T[0].x, -T[1].x), pk(-T[0].y, -T[1].y), pk(-T[0].z, -T[1].z)};
+  int j         = 0;
+  for(; j + U <= nl; j += U)
+    {
+      float4 e[U];
+#pragma unroll
+      for(int u = 0; u < U; u++)
+        e[u] = LP[j + u];
+#pragma unroll
+      for(int u = 0; u < U; u++)
+        far2<PERIODIC, POT, MASK>(e[u], N, T, S, w, tab, afac, big);
+    }
+  for(; j < nl; j++)
+    far2<PERIODIC, POT, MASK>(LP[j], N, T, S, w, tab, afac, big);
+  upk(S.ax, T[0].ax, T[1].ax);
+  upk(S.ay, T[0].ay, T[1].ay);
+  upk(S.az, T[0].az, T[1].az);
+  upk(S.pot, T[0].pot, T[1].pot);
 }
 
 // The warp's interaction list in shared memory.  Main buffer: entries outside the softening length of
@@ -555,13 +715,23 @@ struct List
 // Evaluates and empties the list, then folds the batch partials into the lane's FP64 sums (shared
 // memory, dsum[(4k + c) * 32] for target k and component c = x, y, z, potential).
 template <typename R, bool PERIODIC, bool POT, int TPL, bool EWALD = false>
-__device__ __forceinline__ void evaluate(List<R> &L, Tgt<R> (&T)[TPL], double *dsum, const W32Const &w)
+__device__ __forceinline__ void evaluate(List<R> &L, Tgt<R> (&T)[TPL], double *dsum, const W32Const &w, TabRef tab)
 {
   WALK_STAT(4, L.na);
   WALK_STAT(5, L.nb);
-  evaluate_region<R, PERIODIC, POT, TPL, EWALD, false, false>(L.P, nullptr, L.na, T, w);
-  evaluate_region<R, PERIODIC, POT, TPL, EWALD, false, true>(L.P + Cap<R>::list - L.nb, nullptr, L.nb, T, w);
-  evaluate_region<R, PERIODIC, POT, TPL, EWALD, true, true>(L.NP, L.NH, L.nn, T, w);
+  if constexpr(TPL == 2 && sizeof(R) == 4)
+    {
+      evaluate_region2<PERIODIC, POT, false>(L.P, L.na, T, w, tab);
+      if(PERIODIC)
+        evaluate_region2<PERIODIC, POT, true>(L.P + Cap<R>::list - L.nb, L.nb, T, w, tab);
+    }
+  else
+    {
+      evaluate_region<R, PERIODIC, POT, TPL, EWALD, false, false>(L.P, nullptr, L.na, T, w, tab);
+      if(PERIODIC)  // without Rcut no entry is a border entry
+        evaluate_region<R, PERIODIC, POT, TPL, EWALD, false, true>(L.P + Cap<R>::list - L.nb, nullptr, L.nb, T, w, tab);
+    }
+  evaluate_region<R, PERIODIC, POT, TPL, EWALD, true, true>(L.NP, L.NH, L.nn, T, w, tab);
 #pragma unroll
   for(int k = 0; k < TPL; k++)
     {
@@ -592,34 +762,38 @@ template <typename R, bool PERIODIC>
 __device__ __forceinline__ void push(List<R> &L, bool keep, const V4<R> e, R h, float d2, float hn, float bx, float by, float bz,
                                      const W32Const &w, unsigned lt_mask)
 {
-  int cls = 2;
-  if(!(d2 < hn * hn))
+  const bool nr     = d2 < hn * hn;
+  const unsigned kn = __ballot_sync(0xffffffffu, keep && nr);
+  keep              = keep && !nr;
+  unsigned ka, kb;
+  int at;
+  if(PERIODIC)
     {
-      cls = 0;
-      if(PERIODIC)
-        {
-          const float fx = fabsf((float)e.x) + bx, fy = fabsf((float)e.y) + by, fz = fabsf((float)e.z) + bz;
-          cls = (fmaf(fx, fx, fmaf(fy, fy, fz * fz)) < w.rcut2_all) ? 0 : 1;
-        }
+      const float fx = fabsf((float)e.x) + bx, fy = fabsf((float)e.y) + by, fz = fabsf((float)e.z) + bz;
+      const bool all = fmaf(fx, fx, fmaf(fy, fy, fz * fz)) < w.rcut2_all;
+      ka             = __ballot_sync(0xffffffffu, keep && all);
+      kb             = __ballot_sync(0xffffffffu, keep && !all);
+      at             = all ? L.na + __popc(ka & lt_mask) : Cap<R>::list - 1 - (L.nb + __popc(kb & lt_mask));
+      L.nb += __popc(kb);
     }
-  const unsigned ka = __ballot_sync(0xffffffffu, keep && cls == 0), kb = __ballot_sync(0xffffffffu, keep && cls == 1),
-                 kn = __ballot_sync(0xffffffffu, keep && cls == 2);
-  if(keep)
+  else
     {
-      if(cls == 0)
-        L.P[L.na + __popc(ka & lt_mask)] = e;
-      else if(cls == 1)
-        L.P[Cap<R>::list - 1 - (L.nb + __popc(kb & lt_mask))] = e;
-      else
+      ka = __ballot_sync(0xffffffffu, keep);
+      at = L.na + __popc(ka & lt_mask);
+    }
+  if(keep)
+    L.P[at] = e;
+  L.na += __popc(ka);
+  if(kn)
+    {
+      if(kn >> (threadIdx.x & 31) & 1u)
         {
           const int q = L.nn + __popc(kn & lt_mask);
           L.NP[q]     = e;
           L.NH[q]     = h;
         }
+      L.nn += __popc(kn);
     }
-  L.na += __popc(ka);
-  L.nb += __popc(kb);
-  L.nn += __popc(kn);
 }
 
 // A warp's group: centre (FP64), half extents, smallest and (with margin) largest target softening,
@@ -630,8 +804,31 @@ struct GroupSh
   float ex, ey, ez, h_min, h_grp, aold_min, vote_r2;
 };
 
+// A warp's shared memory: its list, and cold per-lane and per-warp state kept out of registers -- the
+// FP64 sums of the lanes' targets, ErrTolForceAcc x |OldAcc| of the targets (read by the per-target
+// vote), the group, the warp's interaction total.
+template <typename R, int TPL>
+struct WarpSh
+{
+  V4<R> p[Cap<R>::list];
+  V4<R> np[Cap<R>::near_cap];
+  R nh[Cap<R>::near_cap];
+  double dsum[4 * TPL][32];
+  float aold[32 * TPL];
+  unsigned long long total;
+  GroupSh group;
+};
+// A block's shared memory (dynamic: the FP32 TreePM walk's block needs 212 KB)
+template <typename R, bool PERIODIC, int TPL>
+struct BlockSh
+{
+  WarpSh<R, TPL> warp[Shape<R, PERIODIC, TPL>::warps];
+  std::conditional_t<Shape<R, PERIODIC, TPL>::big, TabF, TabNone> tab;
+  __align__(16) unsigned char w_raw[kW32Bytes<R>];
+};
+
 template <bool PERIODIC, bool POT, int TPL, bool EWALD = false, typename R = float>
-__global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W32_MINBLOCKS2 : GG_W32_MINBLOCKS) : 3) k_walk32(const double4 *__restrict__ g_sm, const float4 *__restrict__ g_rel,
+__global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, PERIODIC, TPL>::blocks) k_walk32(const double4 *__restrict__ g_sm, const float4 *__restrict__ g_rel,
                                                         const int4 *__restrict__ g_kids, const double4 *__restrict__ g_pm,
                                                         const uint8_t *__restrict__ g_pst, const double4 *__restrict__ tpm,
                                                         const uint8_t *__restrict__ tst, const float *__restrict__ oldacc,
@@ -644,45 +841,46 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W
                                                         int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total,
                                                         int *__restrict__ err)
 {
-  __shared__ __align__(16) unsigned char w_raw[kW32Bytes<R>];
-  const W32Const &w = *reinterpret_cast<const W32Const *>(w_raw);
-  __shared__ V4<R> il_p[kWarps][Cap<R>::list];
-  __shared__ V4<R> il_np[kWarps][Cap<R>::near_cap];
-  __shared__ R il_nh[kWarps][Cap<R>::near_cap];
-  // cold per-lane and per-warp state kept out of registers: the FP64 sums of the lanes' targets,
-  // ErrTolForceAcc x |OldAcc| of the targets (read by the per-target vote), the warp's interaction total
-  __shared__ double dsum_sh[kWarps][4 * TPL][32];
-  __shared__ float aold_sh[kWarps][32 * TPL];
-  __shared__ unsigned long long total_sh[kWarps];
-  __shared__ GroupSh group_sh[kWarps];
+  constexpr int kWarps = Shape<R, PERIODIC, TPL>::warps;
+  constexpr bool WRAP  = PERIODIC || EWALD;  // nearest images in a periodic box
+  extern __shared__ __align__(16) unsigned char sh_raw[];
+  BlockSh<R, PERIODIC, TPL> &sh = *reinterpret_cast<BlockSh<R, PERIODIC, TPL> *>(sh_raw);
+  const W32Const &w             = *reinterpret_cast<const W32Const *>(sh.w_raw);
   static_assert(kW32Bytes<R> % 4 == 0, "constants copied in 4-byte words");
   for(int t = threadIdx.x; t < kW32Bytes<R> / 4; t += blockDim.x)
-    ((int *)w_raw)[t] = ((const int *)wcp)[t];
-  __syncthreads();
-
+    ((int *)sh.w_raw)[t] = ((const int *)wcp)[t];
   const int warp         = threadIdx.x >> 5;
   const int lane         = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  int *stack             = stack_base + ((int64_t)blockIdx.x * kWarps + warp) * kStackCap;
+  TabRef tab{nullptr};
+  if constexpr(Shape<R, PERIODIC, TPL>::big)
+    {
+      for(int t = threadIdx.x; t < (kNtab + 1) * kCopies; t += blockDim.x)
+        sh.tab.row[t] = wcp->tab[t / kCopies];
+      tab.row = sh.tab.row + lane % kCopies;
+    }
+  __syncthreads();
+
+  int *stack = stack_base + ((int64_t)blockIdx.x * kWarps + warp) * kStackCap;
+  WarpSh<R, TPL> &ws = sh.warp[warp];
   List<R> L;
-  L.P  = il_p[warp];
-  L.NP = il_np[warp];
-  L.NH = il_nh[warp];
-  double *dsum = &dsum_sh[warp][0][lane];
+  L.P  = ws.p;
+  L.NP = ws.np;
+  L.NH = ws.nh;
+  double *dsum = &ws.dsum[0][lane];
   if(lane == 0)
-    total_sh[warp] = 0;
+    ws.total = 0;
   // groups of this target slice; the count lives on the device (no host round trip, graph replays)
   const int64_t ng       = *ngroups_dev;
   // (or the cost-balanced range computed on the device, slice_rng[0..1])
   const int g_begin = slice_rng ? (int)slice_rng[0] : (int)(ng * slice / nslices);
   const int g_end   = slice_rng ? (int)slice_rng[1] : (int)(ng * (slice + 1) / nslices);
+  // a warp's first group is its number, counted over the blocks first so that a small walk spreads
+  // over the SMs; the next ones come from the counter
+  int grp = g_begin + warp * (int)gridDim.x + (int)blockIdx.x;
 
   while(true)
     {
-      int grp = 0;
-      if(lane == 0)
-        grp = atomicAdd(work, 1);
-      grp = g_begin + __shfl_sync(0xffffffffu, grp, 0);
       if(grp >= g_end)
         break;
       // group of up to 32*TPL consecutive targets; lane holds targets t0 + lane + 32k.  A group lies
@@ -705,7 +903,7 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W
           const int64_t tt = tlist ? (int64_t)tlist[t0 + (s < cnt ? s : 0)] : t0 + (s < cnt ? s : 0);
           p[k]             = tpm[tt];
           const float a_l  = w.erracc * oldacc[tt];
-          aold_sh[warp][s] = a_l;
+          ws.aold[s] = a_l;
           mnx = fmin(mnx, p[k].x), mxx = fmax(mxx, p[k].x);
           mny = fmin(mny, p[k].y), mxy = fmax(mxy, p[k].y);
           mnz = fmin(mnz, p[k].z), mxz = fmax(mxz, p[k].z);
@@ -729,11 +927,11 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W
         const float side = 2.0f * fmaxf(g.ex, fmaxf(g.ey, g.ez));
         g.vote_r2        = side * side * (1.0f / (kVote * kVote));
         if(lane == 0)
-          group_sh[warp] = g;
+          ws.group = g;
       }
       __syncwarp();
       // the group's constants are read from shared memory where they are used (out of registers)
-      const GroupSh &gs = group_sh[warp];
+      const GroupSh &gs = ws.group;
       const double &gx = gs.gx, &gy = gs.gy, &gz = gs.gz;
       const float &ex = gs.ex, &ey = gs.ey, &ez = gs.ez, &h_min = gs.h_min, &h_grp = gs.h_grp, &aold_min = gs.aold_min,
                   &vote_r2 = gs.vote_r2;
@@ -779,7 +977,7 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W
             {
               WALK_STAT(0, queued);
               WALK_STAT(10, 1);
-              evaluate<R, PERIODIC, POT, TPL, EWALD>(L, T, dsum, w);
+              evaluate<R, PERIODIC, POT, TPL, EWALD>(L, T, dsum, w, tab);
               __syncwarp();
             }
           if(t_next < t_end)
@@ -817,8 +1015,8 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W
               if(q < ptot)
                 {
                   const int pi     = ofp + (q - oexc);
-                  const double4 pp = g_pm[pi];
-                  pe   = mk4<R>(wrapd(pp.x - gx, w), wrapd(pp.y - gy, w), wrapd(pp.z - gz, w), pp.w);
+                  const double4 pp = load32(g_pm + pi);
+                  pe   = mk4<R>(wrapd<WRAP>(pp.x - gx, w), wrapd<WRAP>(pp.y - gy, w), wrapd<WRAP>(pp.z - gz, w), pp.w);
                   ph   = w.soft[g_pst[pi]];
                   keep = pp.w != 0.0;
                   const float dmx = fmaxf(fabsf((float)pe.x) - ex, 0.0f), dmy = fmaxf(fabsf((float)pe.y) - ey, 0.0f),
@@ -855,12 +1053,12 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W
           if(node >= 0)
             {
               // the three records of the node are fetched together (one memory round trip)
-              const double4 sm = g_sm[node];
+              const double4 sm = load32(g_sm + node);
               const float4 rel = g_rel[node];
               const int4 kd    = g_kids[node];
               if(sm.w != 0.0)
                 {
-                  const double dsx = wrapd(sm.x - gx, w), dsy = wrapd(sm.y - gy, w), dsz = wrapd(sm.z - gz, w);
+                  const double dsx = wrapd<WRAP>(sm.x - gx, w), dsy = wrapd<WRAP>(sm.y - gy, w), dsz = wrapd<WRAP>(sm.z - gz, w);
                   const float sx = (float)dsx, sy = (float)dsy, sz = (float)dsz;
                   const float cx = sx + rel.x, cy = sy + rel.y, cz = sz + rel.z;
                   const float L  = rel.w;
@@ -927,32 +1125,36 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W
             {
               WALK_STAT(7, 1);
               WALK_STAT(8, __popc(vm));
-              bool need    = false;
-              const float L = vrel.w, L2 = L * L;
+              // one voting node after the other, every lane testing its own targets
+              bool need = false;
+              for(unsigned v = vm; v; v &= v - 1)
+                {
+                  const int b     = __ffs(v) - 1;
+                  const float enx = (float)__shfl_sync(0xffffffffu, entry.x, b), eny = (float)__shfl_sync(0xffffffffu, entry.y, b),
+                              enz = (float)__shfl_sync(0xffffffffu, entry.z, b), em = (float)__shfl_sync(0xffffffffu, entry.w, b),
+                              rx = __shfl_sync(0xffffffffu, vrel.x, b), ry = __shfl_sync(0xffffffffu, vrel.y, b),
+                              rz = __shfl_sync(0xffffffffu, vrel.z, b), L = __shfl_sync(0xffffffffu, vrel.w, b),
+                              hn = __shfl_sync(0xffffffffu, hj, b);
+                  const float L2 = L * L;
+                  bool o         = false;
 #pragma unroll
-              for(int k = 0; k < TPL; k++)
-                for(int i = 0; i < 32; i++)
-                  {
-                    const float tx = (float)__shfl_sync(0xffffffffu, T[k].x, i), ty = (float)__shfl_sync(0xffffffffu, T[k].y, i),
-                                tz = (float)__shfl_sync(0xffffffffu, T[k].z, i), th = (float)__shfl_sync(0xffffffffu, T[k].h, i),
-                                ta = aold_sh[warp][i + 32 * k];
-                    if(vote && !need && i + 32 * k < cnt)
+                  for(int k = 0; k < TPL; k++)
+                    if(lane + 32 * k < cnt)
                       {
-                        const float enx = (float)entry.x, eny = (float)entry.y, enz = (float)entry.z;
+                        const float tx = (float)T[k].x, ty = (float)T[k].y, tz = (float)T[k].z, ta = ws.aold[lane + 32 * k];
                         const float dx = enx - tx, dy = eny - ty, dz = enz - tz;
                         const float r2 = dx * dx + dy * dy + dz * dz;
-                        bool o;
                         if(bh)
-                          o = L2 > r2 * w.theta2;
+                          o |= L2 > r2 * w.theta2;
                         else
-                          o = (L2 > r2 * 1.44f) || ((float)entry.w * L2 > r2 * r2 * ta && (!w.minangle || L2 > r2 * 0.16f)) ||
-                              (fabsf(enx + vrel.x - tx) < 0.6f * L && fabsf(eny + vrel.y - ty) < 0.6f * L &&
-                               fabsf(enz + vrel.z - tz) < 0.6f * L);
-                        if(!o && !w.mns && hj > th && r2 < hj * hj)
-                          o = true;
-                        need = o;
+                          o |= (L2 > r2 * 1.44f) || (em * L2 > r2 * r2 * ta && (!w.minangle || L2 > r2 * 0.16f)) ||
+                               (fabsf(enx + rx - tx) < 0.6f * L && fabsf(eny + ry - ty) < 0.6f * L && fabsf(enz + rz - tz) < 0.6f * L);
+                        o |= !w.mns && hn > (float)T[k].h && r2 < hn * hn;
                       }
-                  }
+                  o = __any_sync(0xffffffffu, o);
+                  if(lane == b)
+                    need = o;
+                }
               if(vote && !need)
                 {
                   action = vote_keep ? 1 : 0;
@@ -1012,12 +1214,16 @@ __global__ void __launch_bounds__(32 * kWarps, sizeof(R) == 4 ? (TPL == 2 ? GG_W
         gtot += lane + 32 * k < cnt ? (unsigned long long)T[k].ni : 0ull;
       for(int o = 16; o > 0; o >>= 1)
         gtot += __shfl_xor_sync(0xffffffffu, gtot, o);
+      int nextg = 0;
       if(lane == 0)
-        total_sh[warp] += gtot;
-      __syncwarp();
+        {
+          ws.total += gtot;
+          nextg = atomicAdd(work, 1);
+        }
+      grp = g_begin + kWarps * (int)gridDim.x + __shfl_sync(0xffffffffu, nextg, 0);
     }
-  if(lane == 0 && total_sh[warp])
-    atomicAdd(total, total_sh[warp]);
+  if(lane == 0 && ws.total)
+    atomicAdd(total, ws.total);
 }
 
 // ---- walk groups -------------------------------------------------------------------------
@@ -1370,6 +1576,20 @@ cudaError_t layout32_stage(gpugrav_ctx *c)
 
 typedef decltype(&k_walk32<true, true, 1>) Walk32Kernel;
 
+// launch plan of one kernel form: block size and dynamic shared memory
+struct Walk32Plan
+{
+  Walk32Kernel kern;
+  int warps;
+  size_t smem;
+};
+template <bool PERIODIC, int TPL, bool EWALD = false, typename R = float>
+Walk32Plan plan_of(bool pot)
+{
+  return {pot ? k_walk32<PERIODIC, true, TPL, EWALD, R> : k_walk32<PERIODIC, false, TPL, EWALD, R>, Shape<R, PERIODIC, TPL>::warps,
+          sizeof(BlockSh<R, PERIODIC, TPL>)};
+}
+
 // Everything that must happen before the walk launch and may not be captured in a graph
 // (layout, constants upload from host memory, stack allocation, launch shape).
 cudaError_t walk32_prepare(gpugrav_ctx *c, const WalkConst &wc)
@@ -1399,21 +1619,21 @@ cudaError_t walk32_prepare(gpugrav_ctx *c, const WalkConst &wc)
   const bool fp64     = c->prm.precision == GPUGRAV_PREC_FP64_GROUP;
   if(fp64 && wc.ewald)
     return cudaErrorNotSupported;
-  Walk32Kernel kern = fp64 ? (tpl == 2 ? (periodic ? (pot ? k_walk32<true, true, 2, false, double> : k_walk32<true, false, 2, false, double>)
-                                                    : (pot ? k_walk32<false, true, 2, false, double> : k_walk32<false, false, 2, false, double>))
-                                      : (periodic ? (pot ? k_walk32<true, true, 1, false, double> : k_walk32<true, false, 1, false, double>)
-                                                  : (pot ? k_walk32<false, true, 1, false, double> : k_walk32<false, false, 1, false, double>)))
-                    : wc.ewald ? (pot ? k_walk32<false, true, 1, true> : k_walk32<false, false, 1, true>)
-                      : tpl == 2 ? (periodic ? (pot ? k_walk32<true, true, 2> : k_walk32<true, false, 2>)
-                                             : (pot ? k_walk32<false, true, 2> : k_walk32<false, false, 2>))
-                                 : (periodic ? (pot ? k_walk32<true, true, 1> : k_walk32<true, false, 1>)
-                                             : (pot ? k_walk32<false, true, 1> : k_walk32<false, false, 1>));
-  GG_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarps, 0));
+  const Walk32Plan plan =
+      fp64 ? (tpl == 2 ? (periodic ? plan_of<true, 2, false, double>(pot) : plan_of<false, 2, false, double>(pot))
+                       : (periodic ? plan_of<true, 1, false, double>(pot) : plan_of<false, 1, false, double>(pot)))
+      : wc.ewald ? plan_of<false, 1, true>(pot)
+      : tpl == 2 ? (periodic ? plan_of<true, 2>(pot) : plan_of<false, 2>(pot))
+                 : (periodic ? plan_of<true, 1>(pot) : plan_of<false, 1>(pot));
+  GG_TRY(cudaFuncSetAttribute(plan.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+  GG_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, plan.kern, 32 * plan.warps, plan.smem));
   if(per_sm < 1)
     per_sm = 1;
-  c->w32_kernel = (void *)kern;
-  c->w32_blocks = sms * per_sm;
-  GG_TRY(c->g_stack.ensure((size_t)c->w32_blocks * kWarps * kStackCap * sizeof(int)));
+  c->w32_kernel  = (void *)plan.kern;
+  c->w32_threads = 32 * plan.warps;
+  c->w32_smem    = plan.smem;
+  c->w32_blocks  = sms * per_sm;
+  GG_TRY(c->g_stack.ensure((size_t)c->w32_blocks * plan.warps * kStackCap * sizeof(int)));
   return cudaSuccess;
 }
 
@@ -1426,7 +1646,7 @@ cudaError_t walk32_launch(gpugrav_ctx *c)
   int *err        = c->counters.as<int>() + 14;
   GG_TRY(cudaMemsetAsync(work, 0, sizeof(int), st));
   Walk32Kernel kern = (Walk32Kernel)c->w32_kernel;
-  kern<<<c->w32_blocks, 32 * kWarps, 0, st>>>(c->g_sm.as<double4>(), c->g_rel.as<float4>(), c->g_kids.as<int4>(),
+  kern<<<c->w32_blocks, c->w32_threads, c->w32_smem, st>>>(c->g_sm.as<double4>(), c->g_rel.as<float4>(), c->g_kids.as<int4>(),
                                               c->g_pm.as<double4>(), c->g_pst.as<uint8_t>(), c->s_pm.as<double4>(),
                                               c->s_st.as<uint8_t>(), c->oldacc_s.as<float>(), c->g_ngroups.as<int>(),
                                               c->g_groups.as<int4>(), c->w_tlist, c->slice, c->nslices,
