@@ -141,7 +141,7 @@ __global__ void k_extent_final(const double *partial, int nblocks, BuildConst *b
 
 // ---- keys ----
 __global__ void k_keys(const double *__restrict__ pos, int64_t n, const BuildConst *__restrict__ bc, u128 *__restrict__ key,
-                       uint32_t *__restrict__ idx, int *flags)
+                       uint64_t *__restrict__ lead, uint32_t *__restrict__ idx, int *flags)
 {
   __shared__ uint16_t tab[48 * 8];
   for(int t = threadIdx.x; t < 48 * 8; t += blockDim.x)
@@ -168,8 +168,45 @@ __global__ void k_keys(const double *__restrict__ pos, int64_t n, const BuildCon
         }
       if(bad)
         atomicOr(flags, 1);
-      key[i] = ph_key_dev(tab, ip[0] >> (52 - kBits), ip[1] >> (52 - kBits), ip[2] >> (52 - kBits), kBits);
-      idx[i] = (uint32_t)i;
+      const u128 k = ph_key_dev(tab, ip[0] >> (52 - kBits), ip[1] >> (52 - kBits), ip[2] >> (52 - kBits), kBits);
+      key[i]       = k;
+      lead[i]      = (uint64_t)(k >> (3 * kBits - 64));
+      idx[i]       = (uint32_t)i;
+    }
+}
+
+// ---- the key order from the leading 64 key bits ----
+// Sorting 126-bit keys takes 16 radix passes over 20 bytes a particle; their leading 64 bits (21 levels
+// of the curve, a cell of 5e-7 of the domain) take 8 over 12 bytes and leave few particles in runs of
+// equal leading bits, which are ordered here by their full keys.  A run longer than kMaxRun (coincident
+// or nearly coincident points) sets flag 8: the caller then sorts the full keys.
+constexpr int kMaxRun = 32;
+__global__ void k_sort_ties(int64_t n, const uint64_t *__restrict__ lead, const u128 *__restrict__ key, uint32_t *__restrict__ perm,
+                            int *__restrict__ flags)
+{
+  for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i + 1 < n; i += (int64_t)gridDim.x * blockDim.x)
+    {
+      const uint64_t p = lead[i];
+      if(lead[i + 1] != p || (i > 0 && lead[i - 1] == p))
+        continue;  // not the first of a run
+      int64_t e = i + 2;
+      while(e < n && e - i <= kMaxRun && lead[e] == p)
+        e++;
+      if(e - i > kMaxRun)
+        {
+          atomicOr(flags, 8);
+          continue;
+        }
+      // insertion by the full key; the radix sort left equal keys in the caller's order
+      for(int64_t a = i + 1; a < e; a++)
+        {
+          const uint32_t o = perm[a];
+          const u128 k     = key[o];
+          int64_t b        = a;
+          for(; b > i && key[perm[b - 1]] > k; b--)
+            perm[b] = perm[b - 1];
+          perm[b] = o;
+        }
     }
 }
 
@@ -214,7 +251,7 @@ int grid_for(int64_t n, int threads)
 }
 }  // namespace
 
-cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent, int *status_flags)
+cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent)
 {
   cudaError_t e;
   if(!g_ph_ready)
@@ -241,30 +278,36 @@ cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent, int *status_flags)
                                                                   c->scratch.as<double>(), flags);
       k_extent_final<<<1, 192, 0, c->stream>>>(c->scratch.as<double>(), kExtBlocks, bc);
     }
-  k_keys<<<grid_for(n, 256), 256, 0, c->stream>>>(c->pos_in.as<double>(), n, bc, c->key.as<u128>(), c->idx.as<uint32_t>(), flags);
-  if((e = cudaGetLastError()) != cudaSuccess)
-    return e;
-  if((e = cudaMemcpyAsync(status_flags, flags, sizeof(int), cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess)
-    return e;
-  return cudaStreamSynchronize(c->stream);
+  k_keys<<<grid_for(n, 256), 256, 0, c->stream>>>(c->pos_in.as<double>(), n, bc, c->key.as<u128>(), c->key_alt.as<uint64_t>(),
+                                                 c->idx.as<uint32_t>(), flags);
+  return cudaGetLastError();
 }
 
-cudaError_t sort_stage(gpugrav_ctx *c)
+// Order of the n keys in c->key (perm) from their leading bits, which the caller put into the first half of
+// c->key_alt; flag 8 of *flags: sort_full_stage is needed.
+cudaError_t sort_lead_stage(gpugrav_ctx *c, int64_t n, int *flags)
 {
-  const int64_t n = c->n;
-  cudaError_t e;
-  size_t tmp_bytes = 0;
-  e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
-                                      c->perm.as<uint32_t>(), (int)n, 0, 3 * kBits, c->stream);
-  if(e != cudaSuccess)
-    return e;
-  if((e = c->sort_tmp.ensure(tmp_bytes)) != cudaSuccess)
-    return e;
-  // stable LSD radix sort over the 126 key bits: equal keys keep the caller order,
-  // as the merge sort of peano_hilbert_order does
-  e = cub::DeviceRadixSort::SortPairs(c->sort_tmp.p, tmp_bytes, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
-                                      c->perm.as<uint32_t>(), (int)n, 0, 3 * kBits, c->stream);
-  return e;
+  uint64_t *lead = c->key_alt.as<uint64_t>();
+  size_t tb      = 0;
+  GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, lead, lead + n, c->idx.as<uint32_t>(), c->perm.as<uint32_t>(), (int)n, 0, 64,
+                                         c->stream));
+  GG_TRY(c->sort_tmp.ensure(tb));
+  GG_TRY(cub::DeviceRadixSort::SortPairs(c->sort_tmp.p, tb, lead, lead + n, c->idx.as<uint32_t>(), c->perm.as<uint32_t>(), (int)n, 0, 64,
+                                         c->stream));
+  k_sort_ties<<<grid_for(n, 256), 256, 0, c->stream>>>(n, lead + n, c->key.as<u128>(), c->perm.as<uint32_t>(), flags);
+  return cudaGetLastError();
+}
+
+// stable LSD radix sort over key bits [0, bits): equal keys keep the caller order, as the merge sort of
+// peano_hilbert_order does
+cudaError_t sort_full_stage(gpugrav_ctx *c, int64_t n, int bits)
+{
+  size_t tb = 0;
+  GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
+                                         c->perm.as<uint32_t>(), (int)n, 0, bits, c->stream));
+  GG_TRY(c->sort_tmp.ensure(tb));
+  return cub::DeviceRadixSort::SortPairs(c->sort_tmp.p, tb, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
+                                         c->perm.as<uint32_t>(), (int)n, 0, bits, c->stream);
 }
 
 cudaError_t gather_stage(gpugrav_ctx *c)

@@ -461,21 +461,28 @@ int32_t gpugrav_load(gpugrav_ctx *c, int64_t n, const double *pos, const double 
   CK(cudaMemcpyAsync(c->bconst.p, &bc, sizeof(bc), cudaMemcpyHostToDevice, st), "upload constants");
 
   int flags = 0;
-  CK(gg::domain_stage(c, dom == nullptr, &flags), "domain stage");
-  if(flags & 2)
-    return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_load: non-finite particle position");
-  if(flags & 1)
-    return fail(c, GPUGRAV_ERR_OUT_OF_BOX, "gpugrav_load: particle outside the domain box");
+  CK(gg::domain_stage(c, dom == nullptr), "domain stage");
   cudaEventRecord(c->ev[2], st);
-  CK(gg::sort_stage(c), "key sort");
+  CK(gg::sort_lead_stage(c, n, c->counters.as<int>()), "key sort");
   cudaEventRecord(c->ev[3], st);
   CK(gg::gather_stage(c), "gather");
   CK(cudaMemcpyAsync(&bc, c->bconst.p, sizeof(bc), cudaMemcpyDeviceToHost, st), "download domain");
   CK(cudaMemcpyAsync(&flags, c->counters.p, sizeof(int), cudaMemcpyDeviceToHost, st), "download flags");
   CK(cudaStreamSynchronize(st), "domain stage");
+  if(flags & 2)
+    return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_load: non-finite particle position");
+  if(flags & 1)
+    return fail(c, GPUGRAV_ERR_OUT_OF_BOX, "gpugrav_load: particle outside the domain box");
   c->dom = bc.dom;
   if(flags & 4)
     return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_load: softening type >= nsofttypes");
+  if(flags & 8)
+    {
+      CK(gg::sort_full_stage(c, n, 3 * kBits), "key sort");
+      cudaEventRecord(c->ev[3], st);
+      CK(gg::gather_stage(c), "gather");
+      CK(cudaStreamSynchronize(st), "key sort");
+    }
   c->timings.upload_ms = elapsed(c->ev[0], c->ev[1]);
   c->timings.domain_ms = elapsed(c->ev[1], c->ev[2]);
   c->timings.sort_ms   = elapsed(c->ev[2], c->ev[3]);
@@ -1058,13 +1065,15 @@ int32_t gpugrav_get_keys(gpugrav_ctx *c, uint64_t *hi, uint64_t *lo)
   if(!c->loaded)
     return fail(c, GPUGRAV_ERR_STATE, "no particles loaded");
   DeviceGuard g(c->device);
-  std::vector<u128> tmp(c->n);
-  CK(cudaMemcpyAsync(tmp.data(), c->key_alt.p, c->n * sizeof(u128), cudaMemcpyDeviceToHost, c->stream), "download keys");
+  std::vector<u128> tmp(c->n);  // caller order
+  std::vector<uint32_t> order(c->n);
+  CK(cudaMemcpyAsync(tmp.data(), c->key.p, c->n * sizeof(u128), cudaMemcpyDeviceToHost, c->stream), "download keys");
+  CK(cudaMemcpyAsync(order.data(), c->perm.p, c->n * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream), "download order");
   CK(cudaStreamSynchronize(c->stream), "download keys");
   for(int64_t i = 0; i < c->n; i++)
     {
-      hi[i] = (uint64_t)(tmp[i] >> 64);
-      lo[i] = (uint64_t)tmp[i];
+      hi[i] = (uint64_t)(tmp[order[i]] >> 64);
+      lo[i] = (uint64_t)tmp[order[i]];
     }
   return GPUGRAV_OK;
 }

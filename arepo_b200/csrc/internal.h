@@ -51,6 +51,9 @@ struct BuildConst
   double soft[GPUGRAV_MAX_SOFTTYPES + 1];
 };
 
+constexpr int kSortFlag     = 24;  // gpugrav_ctx::counters: sort_lead_stage's flag in the serving loop
+constexpr int kNeedFullSort = 1;   // build_stage status: the particles are not in full key order yet
+
 // Walk constants
 constexpr int kEwaldN = 64;  // EN of the Ewald correction tables (src/gravity/forcetree.h:90)
 
@@ -193,7 +196,7 @@ struct gpugrav_ctx
   // ---- device buffers ----
   gg::DevBuf bconst, wconst;
   gg::DevBuf pos_in, mass_in, st_in;          // caller order
-  gg::DevBuf key, key_alt, idx, perm;         // keys / sort
+  gg::DevBuf key, key_alt, idx, perm;         // full keys (caller order); leading key bits before and after the sort; order
   gg::DevBuf sort_tmp;
   gg::DevBuf s_pm, s_ix, s_iy, s_iz, s_st;    // sorted SoA: (x,y,z,m) double4, 52-bit coordinates, softening type
   gg::DevBuf s_cd, s_tl, s_tlnode;            // pair depth, top-leaf depth / node
@@ -267,8 +270,9 @@ __device__ __forceinline__ int common_depth(uint64_t ax, uint64_t ay, uint64_t a
 namespace gg
 {
 // launchers implemented in the .cu files; each returns cudaGetLastError() of its launches
-cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent, int *out_of_box);
-cudaError_t sort_stage(gpugrav_ctx *c);
+cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent);
+cudaError_t sort_lead_stage(gpugrav_ctx *c, int64_t n, int *flags);
+cudaError_t sort_full_stage(gpugrav_ctx *c, int64_t n, int bits);
 cudaError_t gather_stage(gpugrav_ctx *c);
 cudaError_t toptree_stage(gpugrav_ctx *c, int *status);
 cudaError_t skeleton_stage(gpugrav_ctx *c, int *status);

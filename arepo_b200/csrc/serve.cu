@@ -200,10 +200,11 @@ __global__ void k_srv_pack(int64_t n, int64_t off, const double4 *__restrict__ p
 
 __device__ __forceinline__ uint64_t to52(double x, double corner, double inv) { return mant52((x - corner) * inv + 1.0); }
 
-// key = slot of the system in the top bits, then the system's 126-bit Peano-Hilbert key
+// key = slot of the system in the top 14 bits, then the system's Peano-Hilbert key; lead: the first 64 bits
+// of the key without the slot's unused bits
 __global__ void k_srv_keys(int64_t ntot, const int32_t *__restrict__ csys, const int64_t *__restrict__ c2p,
                            const double4 *__restrict__ pos, const gpugrav_domain *__restrict__ doms, u128 *__restrict__ key,
-                           uint32_t *__restrict__ idx)
+                           uint64_t *__restrict__ lead, int unused_bits, uint32_t *__restrict__ idx)
 {
   __shared__ uint16_t tab[48 * 8];
   for(int t = threadIdx.x; t < 48 * 8; t += blockDim.x)
@@ -217,8 +218,10 @@ __global__ void k_srv_keys(int64_t ntot, const int32_t *__restrict__ csys, const
       uint64_t ix = to52(x.x, d.corner[0], d.inverse_len), iy = to52(x.y, d.corner[1], d.inverse_len),
                iz = to52(x.z, d.corner[2], d.inverse_len);
       u128 k = ph_key_dev(tab, ix >> 10, iy >> 10, iz >> 10, kBits);
-      key[i] = ((u128)(uint32_t)s << 114) | (k >> 12);
-      idx[i] = (uint32_t)i;
+      k       = ((u128)(uint32_t)s << 114) | (k >> 12);
+      key[i]  = k;
+      lead[i] = (uint64_t)((k << unused_bits) >> 64);
+      idx[i]  = (uint32_t)i;
     }
 }
 
@@ -417,10 +420,12 @@ cudaError_t serve_reserve(gpugrav_serve *s)
   GG_TRY(c->acc_s.ensure(n * 24));
   GG_TRY(c->pot_s.ensure(n * 8));
   GG_TRY(c->nint_s.ensure(n * 4));
-  size_t tb = 0;
+  size_t tb = 0, t2 = 0;
   GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
                                          c->perm.as<uint32_t>(), (int)n, 0, 128, s->st));
-  GG_TRY(c->sort_tmp.ensure(tb));
+  GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, t2, c->key_alt.as<uint64_t>(), c->key_alt.as<uint64_t>() + n, c->idx.as<uint32_t>(),
+                                         c->perm.as<uint32_t>(), (int)n, 0, 64, s->st));
+  GG_TRY(c->sort_tmp.ensure(tb > t2 ? tb : t2));
   GG_TRY(gg::build_reserve(c, n, n, nsys));
   GG_TRY(gg::layout32_reserve(c, n, n));
   GG_TRY(s->up.ensure((size_t)n * (7 * sizeof(double) + 1)));
@@ -793,23 +798,24 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
   k_srv_extent<<<dim3(nsys, 32), 256, 0, st>>>(nsys, dsys, s->c2p.as<int64_t>(), s->pos.as<double4>(),
                                                s->ext.as<unsigned long long>());
   k_srv_domains<<<grid_for(nsys, 128), 128, 0, st>>>(nsys, s->ext.as<unsigned long long>(), c->m_doms.as<gpugrav_domain>());
+  int slot_bits = 0;
+  while(slot_bits < 14 && (1 << slot_bits) < nsys)
+    slot_bits++;
   k_srv_keys<<<grid_for(ntot, 256), 256, 0, st>>>(ntot, s->csys.as<int32_t>(), s->c2p.as<int64_t>(), s->pos.as<double4>(),
-                                                  c->m_doms.as<gpugrav_domain>(), c->key.as<u128>(), c->idx.as<uint32_t>());
-  size_t tb = 0;
-  SCK(cub::DeviceRadixSort::SortPairs(nullptr, tb, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
-                                      c->perm.as<uint32_t>(), (int)ntot, 0, 128, st),
-      "sort");
-  if(c->sort_tmp.ensure(tb) != cudaSuccess)
-    return sfail(s, GPUGRAV_ERR_OOM, "sort");
-  SCK(cub::DeviceRadixSort::SortPairs(c->sort_tmp.p, tb, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
-                                      c->perm.as<uint32_t>(), (int)ntot, 0, 128, st),
-      "sort");
-  k_srv_gather<<<grid_for(ntot, 256), 256, 0, st>>>(ntot, c->perm.as<uint32_t>(), s->csys.as<int32_t>(), s->c2p.as<int64_t>(),
-                                                    s->pos.as<double4>(), s->stype.as<uint8_t>(), s->oldacc.as<float>(),
-                                                    c->m_doms.as<gpugrav_domain>(), c->s_pm.as<double4>(),
-                                                    c->s_ix.as<uint64_t>(), c->s_iy.as<uint64_t>(), c->s_iz.as<uint64_t>(),
-                                                    c->s_st.as<uint8_t>(), c->m_sys.as<int32_t>(), s->s2p.as<int64_t>(),
-                                                    c->oldacc_s.as<float>());
+                                                  c->m_doms.as<gpugrav_domain>(), c->key.as<u128>(), c->key_alt.as<uint64_t>(),
+                                                  14 - slot_bits, c->idx.as<uint32_t>());
+  int *sort_flag = c->counters.as<int>() + kSortFlag;
+  SCK(cudaMemsetAsync(sort_flag, 0, sizeof(int), st), "sort");
+  SCK(gg::sort_lead_stage(c, ntot, sort_flag), "sort");
+  auto gather = [&]() {
+    k_srv_gather<<<grid_for(ntot, 256), 256, 0, st>>>(ntot, c->perm.as<uint32_t>(), s->csys.as<int32_t>(), s->c2p.as<int64_t>(),
+                                                      s->pos.as<double4>(), s->stype.as<uint8_t>(), s->oldacc.as<float>(),
+                                                      c->m_doms.as<gpugrav_domain>(), c->s_pm.as<double4>(),
+                                                      c->s_ix.as<uint64_t>(), c->s_iy.as<uint64_t>(), c->s_iz.as<uint64_t>(),
+                                                      c->s_st.as<uint8_t>(), c->m_sys.as<int32_t>(), s->s2p.as<int64_t>(),
+                                                      c->oldacc_s.as<float>());
+  };
+  gather();
   SCK(cudaGetLastError(), "tick kernels");
 
   // ---- batched build over all systems ----
@@ -821,6 +827,13 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
   c->mark("s1 pre+extent+keys+sort+gather");
   cudaEventRecord(c->ev[16], st);
   SCK(gg::build_stage(c, &bstat), "build");
+  if(bstat == kNeedFullSort)
+    {
+      SCK(cudaMemsetAsync(sort_flag, 0, sizeof(int), st), "sort");
+      SCK(gg::sort_full_stage(c, ntot, 128), "sort");
+      gather();
+      SCK(gg::build_stage(c, &bstat), "build");
+    }
   cudaEventRecord(c->ev[17], st);
   if(bstat != GPUGRAV_OK)
     return sfail(s, bstat, "build failed");

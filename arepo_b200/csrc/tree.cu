@@ -186,15 +186,15 @@ struct TopTmp
 };
 
 // first position in [lo, hi) whose key is not below k; the whole warp probes 32 positions at a time
-__device__ int64_t lower_bound_key(const u128 *keys, int64_t lo, int64_t hi, u128 k)
+__device__ int64_t lower_bound_key(const u128 *keys, const uint32_t *perm, int64_t lo, int64_t hi, u128 k)
 {
   const int lane = threadIdx.x & 31;
   while(hi > lo)
     {
       const int64_t len = hi - lo;
       if(len <= 32)
-        return lo + __popc(__ballot_sync(0xffffffffu, lane < len && keys[lo + (lane < len ? lane : 0)] < k));
-      const int c = __popc(__ballot_sync(0xffffffffu, keys[lo + (lane + 1) * len / 33] < k));
+        return lo + __popc(__ballot_sync(0xffffffffu, lane < len && keys[perm[lo + (lane < len ? lane : 0)]] < k));
+      const int c = __popc(__ballot_sync(0xffffffffu, keys[perm[lo + (lane + 1) * len / 33]] < k));
       const int64_t l = lo;
       lo              = c > 0 ? l + c * len / 33 + 1 : l;
       hi              = c < 32 ? l + (c + 1) * len / 33 : hi;
@@ -212,7 +212,7 @@ __device__ bool top_less(const TopTmp *T, int a, int b)
 }
 
 constexpr int kTopThreads = 256;
-__global__ void __launch_bounds__(kTopThreads) k_toptree(const u128 *__restrict__ keys, int64_t n, double tnf, int mdom, TopTmp *T, int *queue,
+__global__ void __launch_bounds__(kTopThreads) k_toptree(const u128 *__restrict__ keys, const uint32_t *__restrict__ perm, int64_t n, double tnf, int mdom, TopTmp *T, int *queue,
                                                          int *list, int *sorted, gpugrav_topnode *out, int max_top, int *result)
 {
   const int ntask = 1;
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kTopThreads) k_toptree(const u128 *__restrict_
           const int i = list[it >> 3], j = it & 7, sub = ntop + it;
           const u128 size  = T[i].size >> 3;
           const u128 start = T[i].start + (u128)j * size;
-          const int64_t f  = lower_bound_key(keys, T[i].pindex, T[i].pindex + T[i].count, start);
+          const int64_t f  = lower_bound_key(keys, perm, T[i].pindex, T[i].pindex + T[i].count, start);
           if((threadIdx.x & 31) == 0)
             {
               T[sub].daughter = -1;
@@ -1085,7 +1085,7 @@ cudaError_t toptree_stage(gpugrav_ctx *c, int *status)
   int *queue  = (int *)(s + max_top * sizeof(TopTmp));
   int *list   = queue + max_top;
   int *result = c->counters.as<int>() + 8;
-  k_toptree<<<1, kTopThreads, 0, c->stream>>>(c->key_alt.as<u128>(), c->n, c->prm.top_node_factor, c->prm.multiple_domains, T, queue,
+  k_toptree<<<1, kTopThreads, 0, c->stream>>>(c->key.as<u128>(), c->perm.as<uint32_t>(), c->n, c->prm.top_node_factor, c->prm.multiple_domains, T, queue,
                                               list, list + max_top, c->top.as<gpugrav_topnode>(), max_top, result);
   GG_TRY(cudaGetLastError());
   int r = 0;
@@ -1242,9 +1242,14 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
   GG_TRY(cudaMemsetAsync(counters, 0, 16 * sizeof(int), st));
   k_count<<<grid_for(n + 1, 256), 256, 0, st>>>(a, c->cnt.as<int32_t>(), c->hack_list.as<int32_t>(), counters);
   launches++;
-  int hc[2];
-  GG_TRY(cudaMemcpyAsync(hc, counters, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  int hc[kSortFlag + 1];
+  GG_TRY(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
   GG_TRY(cudaStreamSynchronize(st));
+  if(c->multi && hc[kSortFlag])
+    {
+      *status = kNeedFullSort;  // the serving loop sorts the full keys and builds again
+      return cudaSuccess;
+    }
   const int nh  = hc[1];
   c->hack_cells = nh;
   HackCell *cells = nullptr;
