@@ -350,8 +350,7 @@ int32_t gpugrav_destroy(gpugrav_ctx *c)
                         &c->sort_tmp, &c->s_pm, &c->s_ix, &c->s_iy, &c->s_iz, &c->s_st, &c->s_cd, &c->s_tl, &c->s_tlnode,
                         &c->cnt, &c->base, &c->hcnt, &c->hack_list, &c->hack_scratch, &c->counters, &c->top, &c->skel,
                         &c->n_suns, &c->n_depth, &c->n_cl, &c->n_sm, &c->n_maxsoft, &c->n_size, &c->n_father, &c->n_sibling,
-                        &c->n_next, &c->n_dfs, &c->n_first, &c->p_next, &c->p_father, &c->p_dfs, &c->depth_hist,
-                        &c->depth_order, &c->w_sm, &c->w_cl, &c->w_link, &c->g_key, &c->g_key_alt, &c->g_val, &c->g_val_alt, &c->g_bfs, &c->g_np, &c->g_poff, &c->g_sm, &c->g_rel, &c->g_kids, &c->g_pm, &c->g_pst, &c->g_stack, &c->acc_s, &c->pot_s,
+                        &c->n_next, &c->n_dfs, &c->n_count, &c->n_arrived, &c->n_off, &c->p_next, &c->p_father, &c->p_off, &c->w_sm, &c->w_cl, &c->w_link, &c->g_scan, &c->g_sm, &c->g_rel, &c->g_kids, &c->g_pm, &c->g_pst, &c->g_stack, &c->acc_s, &c->pot_s,
                         &c->nint_s, &c->oldacc_s, &c->oldacc_in, &c->out_acc, &c->out_pot, &c->out_nint, &c->scratch,
                         &c->g_groups, &c->g_ngroups, &c->g_gpd, &c->g_gseg, &c->g_gflag, &c->g_gid, &c->t_cd, &c->t_pd, &c->m_sys, &c->m_doms,
                         &c->pm_pos, &c->pm_mass, &c->pm_acc, &c->pm_pot, &c->ewd, &c->ewd32, &c->n_mpt, &c->w_mpt,
@@ -690,6 +689,10 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
       CK(gg::ewald_ensure(c), "Ewald tables");
       wc.ewd = c->ewd.as<double>();
     }
+  if(wc.mns && !c->built_mns)
+    return fail(c, GPUGRAV_ERR_STATE, "gpugrav_walk: the tree was built without MULTIPLE_NODE_SOFTENING");
+  if(c->prm.precision == GPUGRAV_PREC_FP64)
+    CK(gg::thread_ensure(c), "walk layout");
   if(wc.mns)
     wc.w_mpt = c->w_mpt.as<double>();
   c->want_pot = (pot != nullptr);
@@ -1121,6 +1124,8 @@ int32_t gpugrav_export_tree(gpugrav_ctx *c, double *center, double *len, double 
   DeviceGuard g(c->device);
   const int64_t nn = c->num_nodes, n = c->n;
   cudaStream_t st  = c->stream;
+  if(sibling || nextnode || p_next || p_father)
+    CK(gg::thread_ensure(c), "export");
   std::vector<double4> cl, sm;
   if(center || len)
     {

@@ -202,14 +202,14 @@ struct gpugrav_ctx
   gg::DevBuf s_cd, s_tl, s_tlnode;            // pair depth, top-leaf depth / node
   gg::DevBuf cnt, base, hcnt, hack_list, hack_scratch, counters;
   gg::DevBuf top, skel;                       // top nodes, skeleton description
-  gg::DevBuf n_suns, n_depth, n_cl, n_sm, n_maxsoft, n_size, n_father, n_sibling, n_next, n_dfs, n_first;
+  gg::DevBuf n_suns, n_depth, n_cl, n_sm, n_maxsoft, n_size, n_father, n_count, n_arrived;
   gg::DevBuf n_mpt, w_mpt, g_mpt;             // MULTIPLE_NODE_SOFTENING: per-type node masses (node, walk, FP32 layouts)
-  gg::DevBuf p_next, p_father, p_dfs;
-  gg::DevBuf depth_hist, depth_order;
-  gg::DevBuf w_sm, w_cl, w_link;              // walk layout (DFS order)
-  // FP32 group walk: nodes in breadth-first order (children contiguous), particles grouped by parent
-  gg::DevBuf g_key, g_key_alt, g_val, g_val_alt, g_bfs;   // (depth, dfs) sort -> breadth-first rank
-  gg::DevBuf g_np, g_poff;                    // particle children per node (bfs order), their offsets
+  // threading and depth-first walk layout (FP64 walk, exports): thread_stage
+  gg::DevBuf n_off, n_sibling, n_next, n_dfs, p_next, p_father, p_off;
+  gg::DevBuf w_sm, w_cl, w_link;
+  bool threaded = false, built_mns = false;   // built_mns: per-type node masses belong to the tree
+  // FP32 group walk: nodes with the children of a node contiguous, particles grouped by parent
+  gg::DevBuf g_scan;                          // per node: node children | particle children << 32 of the nodes before it
   gg::DevBuf g_sm, g_rel, g_kids;             // node: (CoM, mass) double4; (centre - CoM, len) float4; int4 links
   gg::DevBuf g_pm, g_pst;                     // particles in parent order: (x, y, z, m) double4; softening type
   gg::DevBuf g_stack;                         // per-warp traversal stacks
@@ -277,6 +277,8 @@ cudaError_t gather_stage(gpugrav_ctx *c);
 cudaError_t toptree_stage(gpugrav_ctx *c, int *status);
 cudaError_t skeleton_stage(gpugrav_ctx *c, int *status);
 cudaError_t build_stage(gpugrav_ctx *c, int *status);
+cudaError_t thread_stage(gpugrav_ctx *c);
+cudaError_t thread_ensure(gpugrav_ctx *c);
 cudaError_t walk64_stage(gpugrav_ctx *c, const WalkConst &wc);
 cudaError_t walk32_stage(gpugrav_ctx *c, const WalkConst &wc);
 cudaError_t walk32_prepare(gpugrav_ctx *c, const WalkConst &wc);

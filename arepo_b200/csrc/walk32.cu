@@ -19,9 +19,9 @@
 //    never carries the absolute position (error ~ eps32 x |x - g|, not eps32 x |x|);
 //  * sums: FP32 within a list batch, batch partials accumulated in FP64.
 //
-// Layout: nodes in breadth-first order with contiguous children (ranked by
-// (depth, depth-first position)), particles grouped by parent node.
+// Layout: the node children of a node contiguous, particles grouped by parent node.
 #include <cub/cub.cuh>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <type_traits>
 
@@ -174,73 +174,64 @@ struct TabRef
 // ------------------------------------------------------------------------------
 // layout
 // ------------------------------------------------------------------------------
-__global__ void k_g_keys(int64_t nn, const uint8_t *__restrict__ depth, const int32_t *__restrict__ ndfs,
-                         uint64_t *__restrict__ key, int32_t *__restrict__ val)
+// Nodes are placed family by family: the node children of a node follow each other in slot order, the
+// families in the order of their parents' numbers (which follow the key order); the particle children
+// likewise.  Positions come from one scan over the children counts, after the roots.
+struct ChildCounts
 {
-  for(int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nn; k += (int64_t)gridDim.x * blockDim.x)
-    {
-      key[k] = ((uint64_t)depth[k] << 32) | (uint32_t)ndfs[k];
-      val[k] = (int32_t)k;
-    }
-}
+  __device__ __forceinline__ uint64_t operator()(uint8_t c) const { return (uint64_t)(c & 15) | ((uint64_t)(c >> 4) << 32); }
+};
 
-__global__ void k_g_rank(int64_t nn, int64_t n, const int32_t *__restrict__ sorted, const int32_t *__restrict__ suns,
-                         int32_t *__restrict__ bfs, int32_t *__restrict__ np)
+// 8 lanes per node, one per slot: every lane moves its child's record to the node's block
+__global__ void k_g_fill(int64_t nn, int64_t n, int nroots, const int32_t *__restrict__ suns, const uint8_t *__restrict__ count,
+                         const uint64_t *__restrict__ scan, const double4 *__restrict__ sm, const double4 *__restrict__ cl,
+                         const uint8_t *__restrict__ maxsoft, const double4 *__restrict__ pm, const uint8_t *__restrict__ st,
+                         double4 *__restrict__ g_sm, float4 *__restrict__ g_rel, int4 *__restrict__ g_kids,
+                         double4 *__restrict__ g_pm, uint8_t *__restrict__ g_pst, int *err, const double *__restrict__ mpt, int nsoft,
+                         float *__restrict__ g_mpt)
 {
-  for(int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nn; b += (int64_t)gridDim.x * blockDim.x)
+  auto put = [&](int64_t b, int64_t k) {
+    const double4 s  = sm[k], c = cl[k];
+    const uint64_t o = scan[k];
+    const int m      = count[k];
+    g_sm[b]          = s;
+    g_rel[b]         = make_float4((float)(c.x - s.x), (float)(c.y - s.y), (float)(c.z - s.z), (float)c.w);
+    g_kids[b]        = make_int4((m & 15) ? nroots + (int)(uint32_t)o : -1, (int)(o >> 32), m, (int)maxsoft[k]);
+    if(g_mpt)
+      for(int q = 0; q < nsoft; q++)
+        g_mpt[b * nsoft + q] = (float)mpt[k * nsoft + q];
+  };
+  const int lane      = threadIdx.x & 31;
+  const unsigned below = (1u << (lane & 7)) - 1u;
+  for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ((8 * nn + 31) & ~(int64_t)31); i += (int64_t)gridDim.x * blockDim.x)
     {
-      int32_t k = sorted[b];
-      bfs[k]    = (int32_t)b;
-      int c     = 0;
-      for(int q = 0; q < 8; q++)
+      const int64_t k    = i >> 3;
+      const int32_t c    = k < nn ? suns[i] : -1;
+      const unsigned nm  = __ballot_sync(0xffffffffu, c >= n) >> (lane & 24) & below;
+      const unsigned pmk = __ballot_sync(0xffffffffu, c >= 0 && c < n) >> (lane & 24) & below;
+      if(c >= n)
+        put((int64_t)nroots + (uint32_t)scan[k] + __popc(nm), c - n);
+      else if(c >= 0)
         {
-          int32_t v = suns[8 * (int64_t)k + q];
-          c += (v >= 0 && v < n) ? 1 : 0;
-        }
-      np[b] = c;
-    }
-}
-
-__global__ void k_g_fill(int64_t nn, int64_t n, const int32_t *__restrict__ sorted, const int32_t *__restrict__ suns,
-                         const int32_t *__restrict__ bfs, const int32_t *__restrict__ poff, const double4 *__restrict__ sm,
-                         const double4 *__restrict__ cl, const uint8_t *__restrict__ maxsoft, const double4 *__restrict__ pm,
-                         const uint8_t *__restrict__ st, double4 *__restrict__ g_sm, float4 *__restrict__ g_rel,
-                         int4 *__restrict__ g_kids, double4 *__restrict__ g_pm, uint8_t *__restrict__ g_pst, int *err,
-                         const double *__restrict__ mpt, int nsoft, float *__restrict__ g_mpt)
-{
-  for(int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nn; b += (int64_t)gridDim.x * blockDim.x)
-    {
-      int32_t k = sorted[b];
-      double4 s = sm[k], c = cl[k];
-      g_sm[b]   = s;
-      g_rel[b]  = make_float4((float)(c.x - s.x), (float)(c.y - s.y), (float)(c.z - s.z), (float)c.w);
-      int32_t fc = -1, nc = 0, npc = 0;
-      int32_t fp = poff[b];
-      for(int q = 0; q < 8; q++)
-        {
-          int32_t v = suns[8 * (int64_t)k + q];
-          if(v < 0)
-            continue;
-          if(v < n)
+          const int64_t b = (int64_t)(scan[k] >> 32) + __popc(pmk);
+          if(b < n)
             {
-              g_pm[fp + npc]  = pm[v];
-              g_pst[fp + npc] = st[v];
-              npc++;
-            }
-          else
-            {
-              int32_t cb = bfs[v - n];
-              if(fc < 0)
-                fc = cb;
-              else if(cb != fc + nc)
-                atomicOr(err, 8);  // children must be contiguous in breadth-first order
-              nc++;
+              g_pm[b]  = pm[c];
+              g_pst[b] = st[c];
             }
         }
-      g_kids[b] = make_int4(fc, fp, nc | (npc << 4), (int)maxsoft[k]);
-      if(g_mpt)
-        for(int q = 0; q < nsoft; q++)
-          g_mpt[b * nsoft + q] = (float)mpt[(int64_t)k * nsoft + q];
+      if((lane & 7) == 0 && k < nn)
+        {
+          if(k < nroots)
+            put(k, k);
+          // every node but the roots and every particle has exactly one place
+          if(k == nn - 1)
+            {
+              const uint64_t t = scan[k] + ChildCounts()(count[k]);
+              if((int64_t)(uint32_t)t != nn - nroots || (int64_t)(t >> 32) != n)
+                atomicOr(err, 8);
+            }
+        }
     }
 }
 
@@ -1312,21 +1303,35 @@ __global__ void k_grp_start(int64_t n, const int32_t *__restrict__ seg, int cap,
     flag[i] = ((i - seg[i]) % cap == 0) ? 1 : 0;
 }
 
-// group table: (first target, count, root node, -1 = criterion of the walk constants)
-__global__ void k_grp_fill(int64_t n, const int32_t *__restrict__ flag, const int32_t *__restrict__ gid, int cap,
-                           const int32_t *__restrict__ sys, int4 *__restrict__ groups, int *__restrict__ ngroups)
+// group table: (first target, count, root node, -1 = criterion of the walk constants); the groups tile the
+// targets, so a count is the distance to the next group's start (k_grp_count)
+__global__ void k_grp_fill(int64_t n, const int32_t *__restrict__ flag, const int32_t *__restrict__ gid, const int32_t *__restrict__ sys,
+                           int4 *__restrict__ groups, int *__restrict__ ngroups)
 {
   for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     {
       if(flag[i])
-        {
-          int cnt = 1;
-          while(cnt < cap && i + cnt < n && !flag[i + cnt])
-            cnt++;
-          groups[gid[i]] = make_int4((int)i, cnt, sys ? sys[i] : 0, -1);
-        }
+        groups[gid[i]] = make_int4((int)i, 0, sys ? sys[i] : 0, -1);
       if(i == n - 1)
         *ngroups = gid[i] + flag[i];
+    }
+}
+__global__ void k_grp_count(int64_t n, const int *__restrict__ ngroups, int4 *groups)
+{
+  const int ng = *ngroups;
+  for(int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x)
+    groups[g].y = (g + 1 < ng ? groups[g + 1].x : (int)n) - groups[g].x;
+}
+// one system without cell cuts: consecutive chunks of cap targets
+__global__ void k_grp_plain(int64_t n, int cap, int4 *__restrict__ groups, int *__restrict__ ngroups)
+{
+  const int ng = (int)((n + cap - 1) / cap);
+  for(int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x)
+    {
+      const int64_t i = (int64_t)g * cap;
+      groups[g]       = make_int4((int)i, (int)(n - i < cap ? n - i : cap), 0, -1);
+      if(g == 0)
+        *ngroups = ng;
     }
 }
 
@@ -1416,13 +1421,7 @@ void make_w32(const WalkConst &wc, W32Const *w)
 // buffers of the FP32 walk layout and group table for n particles and nn nodes
 cudaError_t layout32_buffers(gpugrav_ctx *c, int64_t n, int64_t nn)
 {
-  GG_TRY(c->g_key.ensure(nn * 8));
-  GG_TRY(c->g_key_alt.ensure(nn * 8));
-  GG_TRY(c->g_val.ensure(nn * 4));
-  GG_TRY(c->g_val_alt.ensure(nn * 4));
-  GG_TRY(c->g_bfs.ensure(nn * 4));
-  GG_TRY(c->g_np.ensure((nn + 1) * 4));
-  GG_TRY(c->g_poff.ensure((nn + 1) * 4));
+  GG_TRY(c->g_scan.ensure(nn * 8));
   GG_TRY(c->g_sm.ensure(nn * sizeof(double4)));
   GG_TRY(c->g_rel.ensure(nn * sizeof(float4)));
   GG_TRY(c->g_kids.ensure(nn * sizeof(int4)));
@@ -1442,8 +1441,8 @@ cudaError_t layout32_reserve(gpugrav_ctx *c, int64_t n, int64_t nn)
 {
   GG_TRY(layout32_buffers(c, n, nn));
   size_t tb = 0, t2 = 0;
-  GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, c->g_key.as<uint64_t>(), c->g_key_alt.as<uint64_t>(),
-                                         c->g_val.as<int32_t>(), c->g_val_alt.as<int32_t>(), (int)nn, 0, 40, c->stream));
+  GG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, thrust::make_transform_iterator(c->n_count.as<uint8_t>(), ChildCounts()),
+                                       c->g_scan.as<uint64_t>(), (int)nn, c->stream));
   GG_TRY(cub::DeviceScan::InclusiveScan(nullptr, t2, c->g_gflag.as<int32_t>(), c->g_gseg.as<int32_t>(), MaxOp32(), (int)n,
                                         c->stream));
   tb = t2 > tb ? t2 : tb;
@@ -1463,6 +1462,11 @@ cudaError_t groups_stage(gpugrav_ctx *c)
   if(n == 0)
     return cudaSuccess;
   const bool cells = c->group_slack < 64;  // otherwise: cut at system starts only
+  if(!cells && !c->multi)
+    {
+      k_grp_plain<<<grid_for((n + cap - 1) / cap, 256), 256, 0, st>>>(n, cap, c->g_groups.as<int4>(), c->g_ngroups.as<int>());
+      return cudaGetLastError();
+    }
   if(cells)
     k_grp_pd<<<grid_for(n, 256), 256, 0, st>>>(n, c->s_cd.as<int8_t>(), cap, c->g_gpd.as<int8_t>());
   k_grp_cut<<<grid_for(n, 256), 256, 0, st>>>(n, c->s_cd.as<int8_t>(), cells ? c->g_gpd.as<int8_t>() : nullptr,
@@ -1477,9 +1481,10 @@ cudaError_t groups_stage(gpugrav_ctx *c)
   GG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, c->g_gflag.as<int32_t>(), c->g_gid.as<int32_t>(), (int)n, st));
   GG_TRY(c->sort_tmp.ensure(tb));
   GG_TRY(cub::DeviceScan::ExclusiveSum(c->sort_tmp.p, tb, c->g_gflag.as<int32_t>(), c->g_gid.as<int32_t>(), (int)n, st));
-  k_grp_fill<<<grid_for(n, 256), 256, 0, st>>>(n, c->g_gflag.as<int32_t>(), c->g_gid.as<int32_t>(), cap,
+  k_grp_fill<<<grid_for(n, 256), 256, 0, st>>>(n, c->g_gflag.as<int32_t>(), c->g_gid.as<int32_t>(),
                                                 c->multi ? c->m_sys.as<int32_t>() : nullptr, c->g_groups.as<int4>(),
                                                 c->g_ngroups.as<int>());
+  k_grp_count<<<grid_for((n + cap - 1) / cap, 256), 256, 0, st>>>(n, c->g_ngroups.as<int>(), c->g_groups.as<int4>());
   return cudaGetLastError();
 }
 
@@ -1522,44 +1527,36 @@ cudaError_t groups_active_stage(gpugrav_ctx *c, int64_t nt, int cap)
   GG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, c->g_gflag.as<int32_t>(), c->g_gid.as<int32_t>(), (int)nt, st));
   GG_TRY(c->sort_tmp.ensure(tb));
   GG_TRY(cub::DeviceScan::ExclusiveSum(c->sort_tmp.p, tb, c->g_gflag.as<int32_t>(), c->g_gid.as<int32_t>(), (int)nt, st));
-  k_grp_fill<<<grid_for(nt, 256), 256, 0, st>>>(nt, c->g_gflag.as<int32_t>(), c->g_gid.as<int32_t>(), cap, nullptr,
+  k_grp_fill<<<grid_for(nt, 256), 256, 0, st>>>(nt, c->g_gflag.as<int32_t>(), c->g_gid.as<int32_t>(), nullptr,
                                                  c->g_groups.as<int4>(), c->g_ngroups.as<int>());
+  k_grp_count<<<grid_for((nt + cap - 1) / cap, 256), 256, 0, st>>>(nt, c->g_ngroups.as<int>(), c->g_groups.as<int4>());
   return cudaGetLastError();
 }
 
-// breadth-first node layout + particles grouped by parent (built once per tree)
+// the layout above (built once per tree)
 cudaError_t layout32_stage(gpugrav_ctx *c)
 {
   c->mark(nullptr);
   const int64_t n = c->n, nn = c->num_nodes;
   cudaStream_t st = c->stream;
   GG_TRY(layout32_buffers(c, n, nn));
-  const bool mns = (c->prm.flags & GPUGRAV_FLAG_MULTIPLE_NODE_SOFTENING) != 0;
+  const bool mns = c->built_mns;
   if(mns)
     GG_TRY(c->g_mpt.ensure((size_t)(nn + 16) * c->prm.nsofttypes * sizeof(float)));
-  k_g_keys<<<grid_for(nn, 256), 256, 0, st>>>(nn, c->n_depth.as<uint8_t>(), c->n_dfs.as<int32_t>(), c->g_key.as<uint64_t>(),
-                                               c->g_val.as<int32_t>());
-  size_t tb = 0;
-  GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, c->g_key.as<uint64_t>(), c->g_key_alt.as<uint64_t>(),
-                                         c->g_val.as<int32_t>(), c->g_val_alt.as<int32_t>(), (int)nn, 0, 40, st));
+  auto counts = thrust::make_transform_iterator(c->n_count.as<uint8_t>(), ChildCounts());
+  size_t tb   = 0;
+  GG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts, c->g_scan.as<uint64_t>(), (int)nn, st));
   GG_TRY(c->sort_tmp.ensure(tb));
-  GG_TRY(cub::DeviceRadixSort::SortPairs(c->sort_tmp.p, tb, c->g_key.as<uint64_t>(), c->g_key_alt.as<uint64_t>(),
-                                         c->g_val.as<int32_t>(), c->g_val_alt.as<int32_t>(), (int)nn, 0, 40, st));
-  k_g_rank<<<grid_for(nn, 256), 256, 0, st>>>(nn, n, c->g_val_alt.as<int32_t>(), c->n_suns.as<int32_t>(), c->g_bfs.as<int32_t>(),
-                                               c->g_np.as<int32_t>());
-  tb = 0;
-  GG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, c->g_np.as<int32_t>(), c->g_poff.as<int32_t>(), (int)nn, st));
-  GG_TRY(c->sort_tmp.ensure(tb));
-  GG_TRY(cub::DeviceScan::ExclusiveSum(c->sort_tmp.p, tb, c->g_np.as<int32_t>(), c->g_poff.as<int32_t>(), (int)nn, st));
+  GG_TRY(cub::DeviceScan::ExclusiveSum(c->sort_tmp.p, tb, counts, c->g_scan.as<uint64_t>(), (int)nn, st));
   int *err = c->counters.as<int>() + 13;
   GG_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
-  k_g_fill<<<grid_for(nn, 256), 256, 0, st>>>(nn, n, c->g_val_alt.as<int32_t>(), c->n_suns.as<int32_t>(), c->g_bfs.as<int32_t>(),
-                                               c->g_poff.as<int32_t>(), c->n_sm.as<double4>(), c->n_cl.as<double4>(),
-                                               c->n_maxsoft.as<uint8_t>(), c->s_pm.as<double4>(), c->s_st.as<uint8_t>(),
-                                               c->g_sm.as<double4>(), c->g_rel.as<float4>(), c->g_kids.as<int4>(),
-                                               c->g_pm.as<double4>(), c->g_pst.as<uint8_t>(), err,
-                                               mns ? c->n_mpt.as<double>() : nullptr, c->prm.nsofttypes,
-                                               mns ? c->g_mpt.as<float>() : nullptr);
+  k_g_fill<<<grid_for(8 * nn, 256), 256, 0, st>>>(nn, n, c->multi ? c->ntop : 1, c->n_suns.as<int32_t>(), c->n_count.as<uint8_t>(),
+                                                   c->g_scan.as<uint64_t>(), c->n_sm.as<double4>(), c->n_cl.as<double4>(),
+                                                   c->n_maxsoft.as<uint8_t>(), c->s_pm.as<double4>(), c->s_st.as<uint8_t>(),
+                                                   c->g_sm.as<double4>(), c->g_rel.as<float4>(), c->g_kids.as<int4>(),
+                                                   c->g_pm.as<double4>(), c->g_pst.as<uint8_t>(), err,
+                                                   mns ? c->n_mpt.as<double>() : nullptr, c->prm.nsofttypes,
+                                                   mns ? c->g_mpt.as<float>() : nullptr);
   GG_TRY(cudaGetLastError());
   int e = 0;
   GG_TRY(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
