@@ -234,20 +234,13 @@ __global__ void k_direct_reduce(const double4 *__restrict__ partial, int chunks,
   pot[o]          = pt;
 }
 
-// caller index -> sorted index
-__global__ void k_invert(const uint32_t *__restrict__ perm, int64_t n, int32_t *__restrict__ inv)
-{
-  for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    inv[perm[i]] = (int32_t)i;
-}
-
-__global__ void k_map_targets(const int64_t *__restrict__ tg, int64_t nt, const int32_t *__restrict__ inv, int32_t *__restrict__ out,
+__global__ void k_map_targets(const int64_t *__restrict__ tg, int64_t nt, const uint32_t *__restrict__ iperm, int32_t *__restrict__ out,
                               int32_t *__restrict__ place)
 {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if(t < nt)
     {
-      out[t]   = inv[tg[t]];
+      out[t]   = (int32_t)iperm[tg[t]];
       place[t] = (int32_t)t;
     }
 }
@@ -461,21 +454,19 @@ cudaError_t direct_stage(gpugrav_ctx *c, const WalkConst &wc, int64_t nt, const 
   const int64_t nbatch   = (ntile + 31) / 32;
   chunks                 = chunks < 8 ? 8 : chunks;
   chunks                 = chunks > nbatch ? nbatch : chunks;
-  // scratch: boxes | chunk sums | inverse order | sorted positions and places (before and after the sort) | sort space
+  // scratch: boxes | chunk sums | sorted positions and places (before and after the sort) | sort space
   size_t tb = 0;
   GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, (int32_t *)nullptr, (int32_t *)nullptr, (int32_t *)nullptr, (int32_t *)nullptr,
                                          (int)nt, 0, 31, st));
   auto up             = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t bytes  = up(ntile * sizeof(TileBox)) + up((size_t)chunks * nt * sizeof(double4)) + up(n * 4) + 4 * up(nt * 4) + up(tb);
+  const size_t bytes  = up(ntile * sizeof(TileBox)) + up((size_t)chunks * nt * sizeof(double4)) + 4 * up(nt * 4) + up(tb);
   GG_TRY(c->dir_buf.ensure(bytes));
   char *q   = c->dir_buf.as<char>();
   auto take = [&](size_t b) { char *r = q; q += up(b); return r; };
   TileBox *box  = (TileBox *)take(ntile * sizeof(TileBox));
   double4 *part = (double4 *)take((size_t)chunks * nt * sizeof(double4));
-  int32_t *inv = (int32_t *)take(n * 4), *ts = (int32_t *)take(nt * 4), *ts2 = (int32_t *)take(nt * 4), *pl = (int32_t *)take(nt * 4),
-          *pl2 = (int32_t *)take(nt * 4);
-  k_invert<<<(unsigned)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368), 256, 0, st>>>(c->perm.as<uint32_t>(), n, inv);
-  k_map_targets<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(d_targets, nt, inv, ts, pl);
+  int32_t *ts = (int32_t *)take(nt * 4), *ts2 = (int32_t *)take(nt * 4), *pl = (int32_t *)take(nt * 4), *pl2 = (int32_t *)take(nt * 4);
+  k_map_targets<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(d_targets, nt, c->iperm.as<uint32_t>(), ts, pl);
   GG_TRY(cub::DeviceRadixSort::SortPairs(q, tb, ts, ts2, pl, pl2, (int)nt, 0, 31, st));
   // the reach of a pair: Rcut, or where the exact factor vanishes in double precision and no pair is softened
   double hmax = 0;

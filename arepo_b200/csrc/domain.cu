@@ -213,7 +213,7 @@ __global__ void k_sort_ties(int64_t n, const uint64_t *__restrict__ lead, const 
 // ---- gather into sorted SoA ----
 __global__ void k_gather(const double *__restrict__ pos, const double *__restrict__ mass, const uint8_t *__restrict__ st,
                          const uint32_t *__restrict__ perm, int64_t n, const BuildConst *__restrict__ bc,
-                         double4 *__restrict__ s_pm, uint64_t *__restrict__ s_ix, uint64_t *__restrict__ s_iy,
+                         uint32_t *__restrict__ iperm, double4 *__restrict__ s_pm, uint64_t *__restrict__ s_ix, uint64_t *__restrict__ s_iy,
                          uint64_t *__restrict__ s_iz, uint8_t *__restrict__ s_st, int *flags)
 {
   const int nsoft    = bc->nsoft;
@@ -223,6 +223,7 @@ __global__ void k_gather(const double *__restrict__ pos, const double *__restric
   for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     {
       uint32_t o = perm[i];
+      iperm[o]   = (uint32_t)i;
       double x = pos[3 * (int64_t)o + 0], y = pos[3 * (int64_t)o + 1], z = pos[3 * (int64_t)o + 2];
       if(periodic)
         {
@@ -316,10 +317,10 @@ cudaError_t gather_stage(gpugrav_ctx *c)
   cudaError_t e;
   if((e = c->s_pm.ensure(n * sizeof(double4))) != cudaSuccess || (e = c->s_ix.ensure(n * 8)) != cudaSuccess ||
      (e = c->s_iy.ensure(n * 8)) != cudaSuccess || (e = c->s_iz.ensure(n * 8)) != cudaSuccess ||
-     (e = c->s_st.ensure(n + 16)) != cudaSuccess)
+     (e = c->s_st.ensure(n + 16)) != cudaSuccess || (e = c->iperm.ensure(n * sizeof(uint32_t))) != cudaSuccess)
     return e;
   k_gather<<<grid_for(n, 256), 256, 0, c->stream>>>(c->pos_in.as<double>(), c->mass_in.as<double>(), c->st_in.as<uint8_t>(),
-                                                   c->perm.as<uint32_t>(), n, c->bconst.as<BuildConst>(), c->s_pm.as<double4>(),
+                                                   c->perm.as<uint32_t>(), n, c->bconst.as<BuildConst>(), c->iperm.as<uint32_t>(), c->s_pm.as<double4>(),
                                                    c->s_ix.as<uint64_t>(), c->s_iy.as<uint64_t>(), c->s_iz.as<uint64_t>(),
                                                    c->s_st.as<uint8_t>(), c->counters.as<int>());
   return cudaGetLastError();

@@ -124,20 +124,35 @@ __global__ void k_gather_f32(const float *__restrict__ in, const uint32_t *__res
     out[i] = in ? in[perm[i]] : 0.0f;
 }
 
-__global__ void k_scatter_out(const double *__restrict__ acc_s, const double *__restrict__ pot_s, const int32_t *__restrict__ nint_s,
-                              const uint32_t *__restrict__ perm, int64_t n, double *__restrict__ acc, double *__restrict__ pot,
-                              int32_t *__restrict__ nint)
+// Results to caller order, tile by tile: a thread reads its particle's record (32 bytes, one sector, at a
+// random place) and the tile is written in one piece.  Writing each target's 24 + 8 + 4 bytes to random
+// places instead took 2.5 ms at 2^24 particles.
+constexpr int kOutTile = 256;
+__global__ void __launch_bounds__(kOutTile) k_gather_out(const double4 *__restrict__ res_s, const int32_t *__restrict__ nint_s,
+                                                         const uint32_t *__restrict__ iperm, int64_t n, double *__restrict__ acc,
+                                                         double *__restrict__ pot, int32_t *__restrict__ nint)
 {
-  for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+  __shared__ double a[3 * kOutTile];
+  for(int64_t t0 = (int64_t)blockIdx.x * kOutTile; t0 < n; t0 += (int64_t)gridDim.x * kOutTile)
     {
-      int64_t o      = perm[i];
-      acc[3 * o + 0] = acc_s[3 * i + 0];
-      acc[3 * o + 1] = acc_s[3 * i + 1];
-      acc[3 * o + 2] = acc_s[3 * i + 2];
-      if(pot)
-        pot[o] = pot_s[i];
-      if(nint)
-        nint[o] = nint_s[i];
+      const int64_t o = t0 + threadIdx.x;
+      __syncthreads();
+      if(o < n)
+        {
+          const uint32_t i       = iperm[o];
+          const double4 r        = res_s[i];
+          a[3 * threadIdx.x + 0] = r.x;
+          a[3 * threadIdx.x + 1] = r.y;
+          a[3 * threadIdx.x + 2] = r.z;
+          if(pot)
+            pot[o] = r.w;
+          if(nint)
+            nint[o] = nint_s[i];
+        }
+      __syncthreads();
+      const int cnt = (int)(3 * (n - t0 < kOutTile ? n - t0 : kOutTile));
+      for(int q = threadIdx.x; q < cnt; q += kOutTile)
+        acc[3 * t0 + q] = a[q];
     }
 }
 
@@ -350,7 +365,7 @@ int32_t gpugrav_destroy(gpugrav_ctx *c)
                         &c->sort_tmp, &c->s_pm, &c->s_ix, &c->s_iy, &c->s_iz, &c->s_st, &c->s_cd, &c->s_tl, &c->s_tlnode,
                         &c->cnt, &c->base, &c->hcnt, &c->hack_list, &c->hack_scratch, &c->counters, &c->top, &c->skel,
                         &c->n_suns, &c->n_depth, &c->n_cl, &c->n_sm, &c->n_maxsoft, &c->n_size, &c->n_father, &c->n_sibling,
-                        &c->n_next, &c->n_dfs, &c->n_count, &c->n_arrived, &c->n_off, &c->p_next, &c->p_father, &c->p_off, &c->w_sm, &c->w_cl, &c->w_link, &c->g_scan, &c->g_sm, &c->g_rel, &c->g_kids, &c->g_pm, &c->g_pst, &c->g_stack, &c->acc_s, &c->pot_s,
+                        &c->n_next, &c->n_dfs, &c->n_count, &c->n_arrived, &c->n_off, &c->p_next, &c->p_father, &c->p_off, &c->w_sm, &c->w_cl, &c->w_link, &c->g_scan, &c->g_sm, &c->g_rel, &c->g_kids, &c->g_pm, &c->g_pst, &c->g_stack, &c->res_s,
                         &c->nint_s, &c->oldacc_s, &c->oldacc_in, &c->out_acc, &c->out_pot, &c->out_nint, &c->scratch,
                         &c->g_groups, &c->g_ngroups, &c->g_gpd, &c->g_gseg, &c->g_gflag, &c->g_gid, &c->t_cd, &c->t_pd, &c->m_sys, &c->m_doms,
                         &c->pm_pos, &c->pm_mass, &c->pm_acc, &c->pm_pot, &c->ewd, &c->ewd32, &c->n_mpt, &c->w_mpt,
@@ -678,7 +693,7 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
   cudaStream_t st = c->stream;
   const int64_t n    = c->n;
   const int64_t nout = active ? nt : n;
-  if(c->acc_s.ensure(n * 3 * sizeof(double)) != cudaSuccess || c->pot_s.ensure(n * sizeof(double)) != cudaSuccess ||
+  if(c->res_s.ensure(n * sizeof(double4)) != cudaSuccess ||
      c->nint_s.ensure(n * sizeof(int32_t)) != cudaSuccess || c->oldacc_s.ensure(n * sizeof(float)) != cudaSuccess ||
      c->oldacc_in.ensure(n * sizeof(float)) != cudaSuccess || (active && c->t_in.ensure(nt * sizeof(int32_t) + 16) != cudaSuccess))
     return fail(c, GPUGRAV_ERR_OOM, "gpugrav_walk: device allocation");
@@ -807,8 +822,8 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
     CK(gg::targets_scatter(c, nt, a, b, d_acc, d_pot, d_nint), "scatter");
   else
     {
-      k_scatter_out<<<grid_for(n, 256), 256, 0, st>>>(c->acc_s.as<double>(), c->pot_s.as<double>(), c->nint_s.as<int32_t>(),
-                                                      c->perm.as<uint32_t>(), n, d_acc, d_pot, d_nint);
+      k_gather_out<<<grid_for(n, kOutTile), kOutTile, 0, st>>>(c->res_s.as<double4>(), c->nint_s.as<int32_t>(),
+                                                               c->iperm.as<uint32_t>(), n, d_acc, d_pot, d_nint);
       CK(cudaGetLastError(), "scatter");
     }
   if(mem == GPUGRAV_MEM_HOST)

@@ -219,7 +219,8 @@ struct gpugrav_ctx
   int32_t slice = 0, nslices = 1;             // target slice of the walks (gpugrav_set_target_slice)
   // active targets of the current walk (gpugrav_walk_targets): sorted particle positions in key order
   // (t_pos_alt) and their places in the caller's list (t_idx_alt); w_tlist is null for a walk of every particle
-  gg::DevBuf iperm, t_in, t_pos, t_pos_alt, t_idx, t_idx_alt;
+  gg::DevBuf iperm;                           // sorted position of each particle (caller order)
+  gg::DevBuf t_in, t_pos, t_pos_alt, t_idx, t_idx_alt;
   const int32_t *w_tlist = nullptr;
   // cost-balanced slices (gpugrav_set_target_slice_cost): per-particle cost in caller order, per-unit
   // costs and their prefix sums, the slice range computed on the device
@@ -249,7 +250,7 @@ struct gpugrav_ctx
   size_t w32_smem    = 0;
   bool want_pot       = true;  // potential requested by the current walk call
   int walk32_tpl      = 0;     // targets per lane of the group walk: 0 auto, 1 or 2 (GPUGRAV_WALK32_TPL)
-  gg::DevBuf acc_s, pot_s, nint_s, oldacc_s, oldacc_in;  // per target (sorted), inputs
+  gg::DevBuf res_s, nint_s, oldacc_s, oldacc_in;  // per target (sorted): (acceleration, potential) double4, count; inputs
   gg::DevBuf out_acc, out_pot, out_nint;      // caller order staging for host copies
   gg::DevBuf scratch;                         // reductions
   gg::DevBuf dir_buf, dir_io;                 // direct summation: working space; targets and results

@@ -260,7 +260,7 @@ __global__ void k_srv_bh(const int *__restrict__ ngroups, const SysDev *__restri
 
 // store forces, kick the stepping systems, OldAcc = |a| for the next relative pass
 __global__ void k_srv_post(const int64_t *__restrict__ dntot, const int32_t *__restrict__ m_sys, const SysDev *__restrict__ sys,
-                           const int64_t *__restrict__ s2p, const double *__restrict__ acc_s, double4 *__restrict__ vel,
+                           const int64_t *__restrict__ s2p, const double4 *__restrict__ res_s, double4 *__restrict__ vel,
                            double4 *__restrict__ acc, float *__restrict__ oldacc)
 {
   const int64_t ntot = *dntot;
@@ -268,7 +268,8 @@ __global__ void k_srv_post(const int64_t *__restrict__ dntot, const int32_t *__r
     {
       const int64_t p  = s2p[j];
       const SysDev &S  = sys[m_sys[j]];
-      double4 a        = make_double4(acc_s[3 * j + 0], acc_s[3 * j + 1], acc_s[3 * j + 2], 0.0);
+      double4 a        = res_s[j];
+      a.w              = 0.0;
       acc[p]           = a;
       oldacc[p]        = (float)sqrt(a.x * a.x + a.y * a.y + a.z * a.z);
       if(S.state == ST_STEP)
@@ -417,8 +418,7 @@ cudaError_t serve_reserve(gpugrav_serve *s)
   GG_TRY(c->s_st.ensure(n + 16));
   GG_TRY(c->m_sys.ensure(n * 4));
   GG_TRY(c->oldacc_s.ensure(n * 4));
-  GG_TRY(c->acc_s.ensure(n * 24));
-  GG_TRY(c->pot_s.ensure(n * 8));
+  GG_TRY(c->res_s.ensure(n * sizeof(double4)));
   GG_TRY(c->nint_s.ensure(n * 4));
   size_t tb = 0, t2 = 0;
   GG_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
@@ -790,8 +790,8 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
      c->perm.ensure(ntot * 4) != cudaSuccess || c->s_pm.ensure(ntot * sizeof(double4)) != cudaSuccess ||
      c->s_ix.ensure(ntot * 8) != cudaSuccess || c->s_iy.ensure(ntot * 8) != cudaSuccess || c->s_iz.ensure(ntot * 8) != cudaSuccess ||
      c->s_st.ensure(ntot + 16) != cudaSuccess || c->m_sys.ensure(ntot * 4) != cudaSuccess ||
-     c->oldacc_s.ensure(ntot * 4) != cudaSuccess || c->acc_s.ensure(ntot * 24) != cudaSuccess ||
-     c->pot_s.ensure(ntot * 8) != cudaSuccess || c->nint_s.ensure(ntot * 4) != cudaSuccess)
+     c->oldacc_s.ensure(ntot * 4) != cudaSuccess || c->res_s.ensure(ntot * sizeof(double4)) != cudaSuccess ||
+     c->nint_s.ensure(ntot * 4) != cudaSuccess)
     return sfail(s, GPUGRAV_ERR_OOM, "tick buffers");
   SCK(cudaMemsetAsync(s->ext.p, 0xFF, (size_t)nsys * 6 * 8, st), "extent");
   SCK(cudaMemset2DAsync(s->ext.as<unsigned long long>() + 3, 6 * 8, 0, 3 * 8, nsys, st), "extent");
@@ -850,7 +850,7 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
   // until a buffer is reallocated.
   const std::vector<const void *> key = {c->g_sm.p,     c->g_rel.p,    c->g_kids.p,   c->g_pm.p,          c->g_pst.p,
                                          c->s_pm.p,     c->s_st.p,     c->oldacc_s.p, c->g_groups.p,      c->g_stack.p,
-                                         c->acc_s.p,    c->pot_s.p,    c->nint_s.p,   c->scratch.p,       c->counters.p,
+                                         c->res_s.p,    c->nint_s.p,   c->scratch.p,       c->counters.p,
                                          c->m_sys.p,    s->s2p.p,      s->sysdev.p,   s->ntot_dev.p,      s->vel.p,
                                          s->acc.p,      s->oldacc.p,   c->g_ngroups.p, c->w32_kernel,
                                          (const void *)(intptr_t)c->w32_blocks};
@@ -867,7 +867,7 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
       k_srv_bh<<<148 * 4, 256, 0, st>>>(c->g_ngroups.as<int>(), dsys, c->g_groups.as<int4>());
       cudaError_t e2 = gg::walk32_launch(c);
       k_srv_post<<<148 * 8, 256, 0, st>>>(s->ntot_dev.as<int64_t>(), c->m_sys.as<int32_t>(), dsys, s->s2p.as<int64_t>(),
-                                          c->acc_s.as<double>(), s->vel.as<double4>(), s->acc.as<double4>(), s->oldacc.as<float>());
+                                          c->res_s.as<double4>(), s->vel.as<double4>(), s->acc.as<double4>(), s->oldacc.as<float>());
       cudaError_t e3 = cudaGetLastError();
       cudaError_t e4 = cudaStreamEndCapture(st, &g);
       SCK(e1 != cudaSuccess ? e1 : e2 != cudaSuccess ? e2 : e3 != cudaSuccess ? e3 : e4, "capture");

@@ -22,13 +22,6 @@ int grid_for(int64_t n, int threads)
   return (int)(b < 1 ? 1 : b);
 }
 
-// iperm[caller index] = sorted position
-__global__ void k_inv_perm(int64_t n, const uint32_t *__restrict__ perm, uint32_t *__restrict__ iperm)
-{
-  for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    iperm[perm[i]] = (uint32_t)i;
-}
-
 // sorted position of every listed target (flag bit 1: index out of range)
 __global__ void k_target_pos(int64_t nt, const int32_t *__restrict__ targets, int64_t n, const uint32_t *__restrict__ iperm,
                              uint32_t *__restrict__ pos, uint32_t *__restrict__ idx, int *__restrict__ flag)
@@ -58,19 +51,19 @@ __global__ void k_target_dups(int64_t nt, const uint32_t *__restrict__ pos, int 
 // results of the active list back to the caller's list order; entries outside [a, b) of the
 // active list (another rank's target slice) are written as zero
 __global__ void k_scatter_targets(int64_t nt, const uint32_t *__restrict__ tpos, const uint32_t *__restrict__ tidx, int64_t a,
-                                  int64_t b, const double *__restrict__ acc_s, const double *__restrict__ pot_s,
-                                  const int32_t *__restrict__ nint_s, double *__restrict__ acc, double *__restrict__ pot,
+                                  int64_t b, const double4 *__restrict__ res_s, const int32_t *__restrict__ nint_s, double *__restrict__ acc, double *__restrict__ pot,
                                   int32_t *__restrict__ nint)
 {
   for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nt; i += (int64_t)gridDim.x * blockDim.x)
     {
       const int64_t o = tidx[i], s = tpos[i];
       const bool in   = i >= a && i < b;
-      acc[3 * o + 0]  = in ? acc_s[3 * s + 0] : 0.0;
-      acc[3 * o + 1]  = in ? acc_s[3 * s + 1] : 0.0;
-      acc[3 * o + 2]  = in ? acc_s[3 * s + 2] : 0.0;
+      const double4 r = in ? res_s[s] : make_double4(0, 0, 0, 0);
+      acc[3 * o + 0]  = r.x;
+      acc[3 * o + 1]  = r.y;
+      acc[3 * o + 2]  = r.z;
       if(pot)
-        pot[o] = in ? pot_s[s] : 0.0;
+        pot[o] = r.w;
       if(nint)
         nint[o] = in ? nint_s[s] : 0;
     }
@@ -83,14 +76,12 @@ cudaError_t targets_stage(gpugrav_ctx *c, int64_t nt, const int32_t *d_targets, 
 {
   cudaStream_t st = c->stream;
   const int64_t n = c->n;
-  GG_TRY(c->iperm.ensure(n * sizeof(uint32_t)));
   GG_TRY(c->t_pos.ensure(nt * sizeof(uint32_t) + 16));
   GG_TRY(c->t_pos_alt.ensure(nt * sizeof(uint32_t) + 16));
   GG_TRY(c->t_idx.ensure(nt * sizeof(uint32_t) + 16));
   GG_TRY(c->t_idx_alt.ensure(nt * sizeof(uint32_t) + 16));
   int *flag = c->counters.as<int>() + 16;
   GG_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
-  k_inv_perm<<<grid_for(n, 256), 256, 0, st>>>(n, c->perm.as<uint32_t>(), c->iperm.as<uint32_t>());
   k_target_pos<<<grid_for(nt, 256), 256, 0, st>>>(nt, d_targets, n, c->iperm.as<uint32_t>(), c->t_pos.as<uint32_t>(),
                                                   c->t_idx.as<uint32_t>(), flag);
   int bits = 1;
@@ -112,8 +103,7 @@ cudaError_t targets_stage(gpugrav_ctx *c, int64_t nt, const int32_t *d_targets, 
 cudaError_t targets_scatter(gpugrav_ctx *c, int64_t nt, int64_t a, int64_t b, double *acc, double *pot, int32_t *nint)
 {
   k_scatter_targets<<<grid_for(nt, 256), 256, 0, c->stream>>>(nt, c->t_pos_alt.as<uint32_t>(), c->t_idx_alt.as<uint32_t>(), a, b,
-                                                             c->acc_s.as<double>(), c->pot_s.as<double>(),
-                                                             c->nint_s.as<int32_t>(), acc, pot, nint);
+                                                             c->res_s.as<double4>(), c->nint_s.as<int32_t>(), acc, pot, nint);
   return cudaGetLastError();
 }
 }  // namespace gg

@@ -139,7 +139,7 @@ struct W32Const
   const float4 *ewd;       // Ewald correction (fx, fy, fz, pot) per table entry (pure periodic tree)
   float ewd_fac;           // 2 EN / L
   int mns;                 // MULTIPLE_NODE_SOFTENING: nodes used per softening type
-  const float *mpt;        // per-type node masses, breadth-first order, nsoft each
+  const float *mpt;        // per-type node masses in layout order, nsoft each
   int nsoft;
   int minangle;            // ACTIVATE_MINIMUM_OPENING_ANGLE
   // FP64 form only (the FP32 kernels do not copy these into shared memory)
@@ -828,8 +828,7 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
                                                         const int64_t *__restrict__ slice_rng,
                                                         const W32Const *__restrict__ wcp,
                                                         int *__restrict__ stack_base, int *__restrict__ work,
-                                                        double *__restrict__ acc_out, double *__restrict__ pot_out,
-                                                        int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total,
+                                                        double4 *__restrict__ res_out, int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total,
                                                         int *__restrict__ err)
 {
   constexpr int kWarps = Shape<R, PERIODIC, TPL>::warps;
@@ -1169,7 +1168,7 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
           pexc           = pinc - npx;
           q0             = 0;
           WALK_STAT(2, ptot);
-          // node children of opened nodes -> stack (contiguous in breadth-first order)
+          // node children of opened nodes -> stack (contiguous)
           const int cinc = both >> 16;
           const int ctot = tot >> 16;
           if(sp + ctot <= kStackCap)
@@ -1189,12 +1188,9 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
           const int s = lane + 32 * k;
           if(s < cnt)
             {
-              const int64_t t    = tlist ? (int64_t)tlist[t0 + s] : t0 + s;
-              acc_out[3 * t + 0] = dsum[(4 * k + 0) * 32];
-              acc_out[3 * t + 1] = dsum[(4 * k + 1) * 32];
-              acc_out[3 * t + 2] = dsum[(4 * k + 2) * 32];
-              if(POT)
-                pot_out[t] = dsum[(4 * k + 3) * 32];
+              const int64_t t = tlist ? (int64_t)tlist[t0 + s] : t0 + s;
+              res_out[t]  = make_double4(dsum[(4 * k + 0) * 32], dsum[(4 * k + 1) * 32], dsum[(4 * k + 2) * 32],
+                                         POT ? dsum[(4 * k + 3) * 32] : 0.0);
               nint_out[t] = T[k].ni;
             }
         }
@@ -1338,8 +1334,7 @@ __global__ void k_grp_plain(int64_t n, int cap, int4 *__restrict__ groups, int *
 // outputs (sorted order) of the targets outside this slice set to zero; the slice's target range
 // is [start of group g_begin, start of group g_end) with the FP32 group table, else n*s/ns..
 __global__ void k_slice_mask(int64_t n, int slice, int nslices, const int4 *__restrict__ groups, const int *__restrict__ ngroups,
-                             const int64_t *__restrict__ slice_rng, double *__restrict__ acc, double *__restrict__ pot,
-                             int32_t *__restrict__ nint)
+                             const int64_t *__restrict__ slice_rng, double4 *__restrict__ res, int32_t *__restrict__ nint)
 {
   int64_t t_begin, t_end;
   if(slice_rng)
@@ -1362,9 +1357,7 @@ __global__ void k_slice_mask(int64_t n, int slice, int nslices, const int4 *__re
   for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     if(i < t_begin || i >= t_end)
       {
-        acc[3 * i] = acc[3 * i + 1] = acc[3 * i + 2] = 0.0;
-        if(pot)
-          pot[i] = 0.0;
+        res[i]  = make_double4(0, 0, 0, 0);
         nint[i] = 0;
       }
 }
@@ -1649,7 +1642,7 @@ cudaError_t walk32_launch(gpugrav_ctx *c)
                                               c->g_groups.as<int4>(), c->w_tlist, c->slice, c->nslices,
                                               c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr,
                                               (const W32Const *)c->scratch.p,
-                                              c->g_stack.as<int>(), work, c->acc_s.as<double>(), c->pot_s.as<double>(),
+                                              c->g_stack.as<int>(), work, c->res_s.as<double4>(),
                                               c->nint_s.as<int32_t>(), (unsigned long long *)(c->counters.as<int>() + 32), err);
   return cudaGetLastError();
 }
@@ -1764,8 +1757,8 @@ cudaError_t slice_mask_stage(gpugrav_ctx *c, bool fp32)
     return cudaSuccess;
   k_slice_mask<<<grid_for(c->n, 256), 256, 0, c->stream>>>(c->n, c->slice, c->nslices, fp32 ? c->g_groups.as<int4>() : nullptr,
                                                            fp32 ? c->g_ngroups.as<int>() : nullptr,
-                                                           c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr, c->acc_s.as<double>(),
-                                                           c->want_pot ? c->pot_s.as<double>() : nullptr, c->nint_s.as<int32_t>());
+                                                           c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr, c->res_s.as<double4>(),
+                                                           c->nint_s.as<int32_t>());
   return cudaGetLastError();
 }
 

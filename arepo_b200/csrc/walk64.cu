@@ -55,8 +55,7 @@ __global__ void __launch_bounds__(32 * kWarps, 12) k_walk64(const double4 *__res
                                                         const double4 *__restrict__ tpm, const uint8_t *__restrict__ tst,
                                                         const float *__restrict__ oldacc, int64_t t_begin, int64_t t_end,
                                                         const int32_t *__restrict__ tlist, const WalkConst *__restrict__ wcp,
-                                                        double *__restrict__ acc_out, double *__restrict__ pot_out,
-                                                        int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total)
+                                                        double4 *__restrict__ res_out, int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total)
 {
   __shared__ WalkConst w;
   for(int t = threadIdx.x; t < (int)(sizeof(WalkConst) / 4); t += blockDim.x)
@@ -278,11 +277,8 @@ __global__ void __launch_bounds__(32 * kWarps, 12) k_walk64(const double4 *__res
 
   if(valid)
     {
-      acc_out[3 * tgt + 0] = acc_x;
-      acc_out[3 * tgt + 1] = acc_y;
-      acc_out[3 * tgt + 2] = acc_z;
-      pot_out[tgt]         = pot;
-      nint_out[tgt]        = ninteractions;
+      res_out[tgt]  = make_double4(acc_x, acc_y, acc_z, pot);
+      nint_out[tgt] = ninteractions;
     }
   // interaction total for the timing report
   unsigned long long v = valid ? (unsigned long long)ninteractions : 0ull;
@@ -314,8 +310,7 @@ cudaError_t walk64_stage(gpugrav_ctx *c, const WalkConst &wc)
   kern<<<(unsigned)blocks, 32 * kWarps, 0, c->stream>>>(
       c->w_sm.as<double4>(), c->w_cl.as<double4>(), c->w_link.as<int2>(), (uint32_t)c->n_entries, c->s_pm.as<double4>(),
       c->s_st.as<uint8_t>(), c->oldacc_s.as<float>(), t_begin, t_end, c->w_tlist, c->wconst.as<WalkConst>(),
-      c->acc_s.as<double>(), c->pot_s.as<double>(),
-      c->nint_s.as<int32_t>(), (unsigned long long *)(c->counters.as<int>() + 32));
+      c->res_s.as<double4>(), c->nint_s.as<int32_t>(), (unsigned long long *)(c->counters.as<int>() + 32));
   return cudaGetLastError();
 }
 }  // namespace gg
