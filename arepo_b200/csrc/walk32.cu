@@ -136,7 +136,7 @@ struct W32Const
   float theta2, erracc;
   int periodic, bh;
   float soft[GPUGRAV_MAX_SOFTTYPES + 1];
-  const float4 *ewd;       // Ewald correction (fx, fy, fz, pot) per table entry (pure periodic tree)
+  const float4 *ewd;       // Ewald correction (fx, fy, fz, pot) per cell corner (pure periodic tree)
   float ewd_fac;           // 2 EN / L
   int mns;                 // MULTIPLE_NODE_SOFTENING: nodes used per softening type
   const float *mpt;        // per-type node masses in layout order, nsoft each
@@ -343,21 +343,33 @@ struct Tgt
   int ni;
 };
 
+// 32 bytes in one load (32-byte aligned)
+__device__ __forceinline__ void load2(const float4 *p, float4 &a, float4 &b)
+{
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
 // Ewald correction (force, potential) for the separation (dx, dy, dz) = source - target:
 // the trilinear interpolation and sign flips of ewald_corr (src/gravity/forcetree_ewald.c:268-342)
-// in FP32 on the float4 table.
+// in FP32 on the table of cell corners (k_ewald_cells).
 __device__ __forceinline__ float4 ewald_corr32(float dx, float dy, float dz, const W32Const &w)
 {
-  constexpr int m = kEwaldN + 1;
+  constexpr int n = kEwaldN;
   const float sx = dx < 0.0f ? 1.0f : -1.0f, sy = dy < 0.0f ? 1.0f : -1.0f, sz = dz < 0.0f ? 1.0f : -1.0f;
   float u = fabsf(dx) * w.ewd_fac, v = fabsf(dy) * w.ewd_fac, s = fabsf(dz) * w.ewd_fac;
-  const int i = min((int)u, kEwaldN - 1), j = min((int)v, kEwaldN - 1), k = min((int)s, kEwaldN - 1);
+  const int i = min((int)u, n - 1), j = min((int)v, n - 1), k = min((int)s, n - 1);
   u -= i;
   v -= j;
   s -= k;
-  const float4 *t = w.ewd + ((i * m + j) * m + k);
-  const float4 a0 = __ldg(t), a1 = __ldg(t + 1), a2 = __ldg(t + m), a3 = __ldg(t + m + 1);
-  const float4 b0 = __ldg(t + m * m), b1 = __ldg(t + m * m + 1), b2 = __ldg(t + m * m + m), b3 = __ldg(t + m * m + m + 1);
+  // the cell's corners, two (32 bytes) per load
+  const float4 *t = w.ewd + (size_t)((i * n + j) * n + k) * 8;
+  float4 a0, a1, a2, a3, b0, b1, b2, b3;
+  load2(t, a0, a1);
+  load2(t + 2, a2, a3);
+  load2(t + 4, b0, b1);
+  load2(t + 6, b2, b3);
   const float f1 = (1 - u) * (1 - v) * (1 - s), f2 = (1 - u) * (1 - v) * s, f3 = (1 - u) * v * (1 - s), f4 = (1 - u) * v * s;
   const float f5 = u * (1 - v) * (1 - s), f6 = u * (1 - v) * s, f7 = u * v * (1 - s), f8 = u * v * s;
   float4 r;
