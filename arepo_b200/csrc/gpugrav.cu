@@ -761,6 +761,11 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
   CK(cudaMemsetAsync(c->counters.as<int>() + 14, 0, 4, st), "reset counters");
   cudaEventRecord(c->ev[8], st);
   cudaError_t we = cudaSuccess;
+  if(active)
+    {
+      c->w_tlist    = c->t_pos_alt.as<int32_t>();
+      c->w_ntargets = nt;
+    }
   if(fp32)
     {
       we = gg::walk32_prepare(c, wc);
@@ -780,23 +785,13 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
       c->slice_rng_on = false;
       if(!active && we == cudaSuccess)
         we = gg::slice_cost_stage(c, true);  // cost-balanced slice range, if costs are set
-      if(active)
-        {
-          c->w_tlist    = c->t_pos_alt.as<int32_t>();
-          c->w_ntargets = nt;
-        }
       if(we == cudaSuccess)
         we = gg::walk32_launch(c);
     }
   else
     {
       c->slice_rng_on = false;
-      if(active)
-        {
-          c->w_tlist    = c->t_pos_alt.as<int32_t>();
-          c->w_ntargets = nt;
-        }
-      else
+      if(!active)
         we = gg::slice_cost_stage(c, false);
       if(we == cudaSuccess)
         we = gg::walk64_stage(c, wc);

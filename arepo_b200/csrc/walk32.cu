@@ -528,12 +528,11 @@ namespace
 // them), in blocks of kUnroll entries evaluated without branches.  CHECK (near list): a block in
 // which some pair lies inside the softening length (the targets' own particles, close neighbours)
 // is revisited for those pairs.  MASK: per-pair Rcut mask and count (see far()).
-template <typename R, bool PERIODIC, bool POT, int TPL, bool EWALD, bool CHECK, bool MASK>
+template <typename R, bool PERIODIC, bool POT, int TPL, bool EWALD, bool CHECK, bool MASK, int U = kUnroll<TPL>>
 __device__ __forceinline__ void evaluate_region(const V4<R> *__restrict__ LP, const R *__restrict__ LH, int nl, Tgt<R> (&T)[TPL],
                                                 const W32Const &w, TabRef tab)
 {
   int j = 0;
-  constexpr int U = kUnroll<TPL>;
   for(; j + U <= nl; j += U)
     {
       V4<R> e[U];
@@ -717,7 +716,9 @@ struct List
 
 // Evaluates and empties the list, then folds the batch partials into the lane's FP64 sums (shared
 // memory, dsum[(4k + c) * 32] for target k and component c = x, y, z, potential).
-template <typename R, bool PERIODIC, bool POT, int TPL, bool EWALD = false>
+// NU: entries per block of the near list; a block's softened pairs follow its others, so the order of the
+// sums depends on it (a split group keeps that of the whole one).
+template <typename R, bool PERIODIC, bool POT, int TPL, bool EWALD, int NU>
 __device__ __forceinline__ void evaluate(List<R> &L, Tgt<R> (&T)[TPL], double *dsum, const W32Const &w, TabRef tab)
 {
   WALK_STAT(4, L.na);
@@ -734,7 +735,7 @@ __device__ __forceinline__ void evaluate(List<R> &L, Tgt<R> (&T)[TPL], double *d
       if(PERIODIC)  // without Rcut no entry is a border entry
         evaluate_region<R, PERIODIC, POT, TPL, EWALD, false, true>(L.P + Cap<R>::list - L.nb, nullptr, L.nb, T, w, tab);
     }
-  evaluate_region<R, PERIODIC, POT, TPL, EWALD, true, true>(L.NP, L.NH, L.nn, T, w, tab);
+  evaluate_region<R, PERIODIC, POT, TPL, EWALD, true, true, NU>(L.NP, L.NH, L.nn, T, w, tab);
 #pragma unroll
   for(int k = 0; k < TPL; k++)
     {
@@ -830,7 +831,10 @@ struct BlockSh
   __align__(16) unsigned char w_raw[kW32Bytes<R>];
 };
 
-template <bool PERIODIC, bool POT, int TPL, bool EWALD = false, typename R = float>
+// SPLIT (two targets per lane, few groups): a group goes to two warps; both make its whole traversal, which
+// gives both the same lists, and each evaluates one target per lane.  While there are fewer groups than
+// half the warps the walk takes as long as its slowest warp, and the evaluation is most of that.
+template <bool PERIODIC, bool POT, int TPL, bool EWALD = false, typename R = float, bool SPLIT = false>
 __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, PERIODIC, TPL>::blocks) k_walk32(const double4 *__restrict__ g_sm, const float4 *__restrict__ g_rel,
                                                         const int4 *__restrict__ g_kids, const double4 *__restrict__ g_pm,
                                                         const uint8_t *__restrict__ g_pst, const double4 *__restrict__ tpm,
@@ -877,12 +881,15 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
   // (or the cost-balanced range computed on the device, slice_rng[0..1])
   const int g_begin = slice_rng ? (int)slice_rng[0] : (int)(ng * slice / nslices);
   const int g_end   = slice_rng ? (int)slice_rng[1] : (int)(ng * (slice + 1) / nslices);
-  // a warp's first group is its number, counted over the blocks first so that a small walk spreads
-  // over the SMs; the next ones come from the counter
-  int grp = g_begin + warp * (int)gridDim.x + (int)blockIdx.x;
+  // a warp's first unit (group, or half of one) is its number, counted over the blocks first so that a
+  // small walk spreads over the SMs; the next ones come from the counter
+  constexpr int UPG = SPLIT ? 2 : 1;  // units per group
+  constexpr int TE  = TPL / UPG;      // targets per lane that this warp evaluates
+  int unit          = warp * (int)gridDim.x + (int)blockIdx.x;
 
   while(true)
     {
+      const int grp = g_begin + unit / UPG, half = SPLIT ? unit & 1 : 0;
       if(grp >= g_end)
         break;
       // group of up to 32*TPL consecutive targets; lane holds targets t0 + lane + 32k.  A group lies
@@ -944,11 +951,18 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
           T[k].x = (R)(p[k].x - gx), T[k].y = (R)(p[k].y - gy), T[k].z = (R)(p[k].z - gz);
           const int sk = lane + 32 * k < cnt ? lane + 32 * k : 0;
           T[k].h       = (R)w.soft[tst[tlist ? (int64_t)tlist[t0 + sk] : t0 + sk]];
-          T[k].ax = T[k].ay = T[k].az = T[k].pot = R(0);
+        }
+      // the targets that this warp evaluates
+      Tgt<R> E[TE];
+#pragma unroll
+      for(int k = 0; k < TE; k++)
+        {
+          E[k]    = SPLIT && half ? T[TPL - 1] : T[k];
+          E[k].ax = E[k].ay = E[k].az = E[k].pot = R(0);
 #pragma unroll
           for(int c = 0; c < 4; c++)
             dsum[(4 * k + c) * 32] = 0.0;
-          T[k].ni = 0;
+          E[k].ni = 0;
         }
 
       int sp = 1;
@@ -979,7 +993,7 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
             {
               WALK_STAT(0, queued);
               WALK_STAT(10, 1);
-              evaluate<R, PERIODIC, POT, TPL, EWALD>(L, T, dsum, w, tab);
+              evaluate<R, PERIODIC, POT, TE, EWALD, kUnroll<TPL>>(L, E, dsum, w, tab);
               __syncwarp();
             }
           if(t_next < t_end)
@@ -1195,22 +1209,22 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
           __syncwarp();
         }
 #pragma unroll
-      for(int k = 0; k < TPL; k++)
+      for(int k = 0; k < TE; k++)
         {
-          const int s = lane + 32 * k;
+          const int s = lane + 32 * (SPLIT ? half : k);
           if(s < cnt)
             {
               const int64_t t = tlist ? (int64_t)tlist[t0 + s] : t0 + s;
               res_out[t]  = make_double4(dsum[(4 * k + 0) * 32], dsum[(4 * k + 1) * 32], dsum[(4 * k + 2) * 32],
                                          POT ? dsum[(4 * k + 3) * 32] : 0.0);
-              nint_out[t] = T[k].ni;
+              nint_out[t] = E[k].ni;
             }
         }
       // the group's interactions (idle slots count none)
       unsigned long long gtot = 0;
 #pragma unroll
-      for(int k = 0; k < TPL; k++)
-        gtot += lane + 32 * k < cnt ? (unsigned long long)T[k].ni : 0ull;
+      for(int k = 0; k < TE; k++)
+        gtot += lane + 32 * (SPLIT ? half : k) < cnt ? (unsigned long long)E[k].ni : 0ull;
       for(int o = 16; o > 0; o >>= 1)
         gtot += __shfl_xor_sync(0xffffffffu, gtot, o);
       int nextg = 0;
@@ -1219,7 +1233,7 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
           ws.total += gtot;
           nextg = atomicAdd(work, 1);
         }
-      grp = g_begin + kWarps * (int)gridDim.x + __shfl_sync(0xffffffffu, nextg, 0);
+      unit = kWarps * (int)gridDim.x + __shfl_sync(0xffffffffu, nextg, 0);
     }
   if(lane == 0 && ws.total)
     atomicAdd(total, ws.total);
@@ -1585,11 +1599,11 @@ struct Walk32Plan
   int warps;
   size_t smem;
 };
-template <bool PERIODIC, int TPL, bool EWALD = false, typename R = float>
+template <bool PERIODIC, int TPL, bool EWALD = false, typename R = float, bool SPLIT = false>
 Walk32Plan plan_of(bool pot)
 {
-  return {pot ? k_walk32<PERIODIC, true, TPL, EWALD, R> : k_walk32<PERIODIC, false, TPL, EWALD, R>, Shape<R, PERIODIC, TPL>::warps,
-          sizeof(BlockSh<R, PERIODIC, TPL>)};
+  return {pot ? k_walk32<PERIODIC, true, TPL, EWALD, R, SPLIT> : k_walk32<PERIODIC, false, TPL, EWALD, R, SPLIT>,
+          Shape<R, PERIODIC, TPL>::warps, sizeof(BlockSh<R, PERIODIC, TPL>)};
 }
 
 // Everything that must happen before the walk launch and may not be captured in a graph
@@ -1621,10 +1635,15 @@ cudaError_t walk32_prepare(gpugrav_ctx *c, const WalkConst &wc)
   const bool fp64     = c->prm.precision == GPUGRAV_PREC_FP64_GROUP;
   if(fp64 && wc.ewald)
     return cudaErrorNotSupported;
+  // two warps per group while all of them run at once (24 warps per SM in either form); an active list may
+  // be cut into somewhat more groups, whose second halves then follow in a second round
+  const int64_t targets = c->w_ntargets > 0 ? c->w_ntargets : c->n;
+  const bool split      = !fp64 && !wc.ewald && tpl == 2 && 2 * ((targets / c->nslices + 63) / 64) <= 24 * sms;
   const Walk32Plan plan =
       fp64 ? (tpl == 2 ? (periodic ? plan_of<true, 2, false, double>(pot) : plan_of<false, 2, false, double>(pot))
                        : (periodic ? plan_of<true, 1, false, double>(pot) : plan_of<false, 1, false, double>(pot)))
       : wc.ewald ? plan_of<false, 1, true>(pot)
+      : split    ? (periodic ? plan_of<true, 2, false, float, true>(pot) : plan_of<false, 2, false, float, true>(pot))
       : tpl == 2 ? (periodic ? plan_of<true, 2>(pot) : plan_of<false, 2>(pot))
                  : (periodic ? plan_of<true, 1>(pot) : plan_of<false, 1>(pot));
   GG_TRY(cudaFuncSetAttribute(plan.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
