@@ -265,7 +265,7 @@ cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent)
   const int64_t n = c->n;
   if((e = c->scratch.ensure(kExtBlocks * 6 * sizeof(double) + 64)) != cudaSuccess)
     return e;
-  if((e = c->counters.ensure(64 * sizeof(int))) != cudaSuccess)
+  if((e = c->counters.ensure(kCounters * sizeof(int))) != cudaSuccess)
     return e;
   if((e = c->key.ensure(n * sizeof(u128))) != cudaSuccess || (e = c->key_alt.ensure(n * sizeof(u128))) != cudaSuccess ||
      (e = c->idx.ensure(n * sizeof(uint32_t))) != cudaSuccess || (e = c->perm.ensure(n * sizeof(uint32_t))) != cudaSuccess)

@@ -164,6 +164,7 @@ int grid_for(int64_t n, int threads)
   return (int)(b < 1 ? 1 : b);
 }
 
+constexpr int64_t kStagedDirect = 16384;  // gravity_direct: host arrays of up to this many particles go through one block
 constexpr size_t kDirectKeep = (size_t)256 << 20;  // working space of gpugrav_direct kept between calls
 
 struct DeviceGuard
@@ -343,7 +344,7 @@ int32_t gpugrav_create(gpugrav_ctx **out, int32_t device, const gpugrav_params *
         return GPUGRAV_ERR_CUDA;
       }
   if(c->bconst.ensure(sizeof(BuildConst)) != cudaSuccess || c->wconst.ensure(sizeof(WalkConst)) != cudaSuccess ||
-     c->counters.ensure(64 * sizeof(int)) != cudaSuccess)
+     c->counters.ensure(kCounters * sizeof(int)) != cudaSuccess)
     {
       delete c;
       return GPUGRAV_ERR_OOM;
@@ -375,6 +376,7 @@ int32_t gpugrav_destroy(gpugrav_ctx *c)
   for(auto *b : bufs)
     b->release();
   c->pinned.release();
+  c->stage.release();
   for(auto &e : c->ev)
     if(e)
       cudaEventDestroy(e);
@@ -457,7 +459,10 @@ int32_t gpugrav_load(gpugrav_ctx *c, int64_t n, const double *pos, const double 
   cudaEventRecord(c->ev[1], st);
 
   // softening types must index ForceSoftening[0..nsofttypes-1]: validated on the host copy when given
-  BuildConst bc;
+  gg::HostIo *io = c->io();
+  if(!io)
+    return fail(c, GPUGRAV_ERR_OOM, "gpugrav_load: pinned allocation");
+  BuildConst &bc = io->bc;
   memset(&bc, 0, sizeof(bc));
   bc.n        = n;
   bc.periodic = c->prm.periodic;
@@ -474,15 +479,15 @@ int32_t gpugrav_load(gpugrav_ctx *c, int64_t n, const double *pos, const double 
     }
   CK(cudaMemcpyAsync(c->bconst.p, &bc, sizeof(bc), cudaMemcpyHostToDevice, st), "upload constants");
 
-  int flags = 0;
   CK(gg::domain_stage(c, dom == nullptr), "domain stage");
   cudaEventRecord(c->ev[2], st);
   CK(gg::sort_lead_stage(c, n, c->counters.as<int>()), "key sort");
   cudaEventRecord(c->ev[3], st);
   CK(gg::gather_stage(c), "gather");
   CK(cudaMemcpyAsync(&bc, c->bconst.p, sizeof(bc), cudaMemcpyDeviceToHost, st), "download domain");
-  CK(cudaMemcpyAsync(&flags, c->counters.p, sizeof(int), cudaMemcpyDeviceToHost, st), "download flags");
+  CK(cudaMemcpyAsync(io->counters, c->counters.p, sizeof(int), cudaMemcpyDeviceToHost, st), "download flags");
   CK(cudaStreamSynchronize(st), "domain stage");
+  const int flags = io->counters[0];
   if(flags & 2)
     return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_load: non-finite particle position");
   if(flags & 1)
@@ -523,7 +528,8 @@ int32_t gpugrav_build(gpugrav_ctx *c, const gpugrav_topnode *top, int32_t ntop)
         return fail(c, GPUGRAV_ERR_OOM, "top nodes");
       c->top_host.assign(top, top + ntop);
       CK(cudaMemcpyAsync(c->top.p, top, ntop * sizeof(gpugrav_topnode), cudaMemcpyHostToDevice, st), "upload top nodes");
-      c->ntop = ntop;
+      c->ntop    = ntop;
+      c->top_dev = false;
     }
   else
     {
@@ -535,11 +541,11 @@ int32_t gpugrav_build(gpugrav_ctx *c, const gpugrav_topnode *top, int32_t ntop)
   cudaEventRecord(c->ev[5], st);
   int s = 0;
   CK(gg::build_stage(c, &s), "tree build");
+  if(s == GPUGRAV_ERR_TOPNODES && c->top_dev && c->ntop < 0)
+    return fail(c, s, "gpugrav_build: top-level tree could not be refined (PEANOGRID too coarse)");
   if(s != GPUGRAV_OK)
     return fail(c, s, s == GPUGRAV_ERR_TOPNODES ? "gpugrav_build: invalid top-level tree"
                                                 : "gpugrav_build: tree build self-check failed");
-  cudaEventRecord(c->ev[6], st);
-  CK(cudaStreamSynchronize(st), "tree build");
   c->timings.toptree_ms = elapsed(c->ev[4], c->ev[5]);
   c->timings.build_ms   = elapsed(c->ev[5], c->ev[6]);
   c->built              = true;
@@ -697,7 +703,10 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
      c->nint_s.ensure(n * sizeof(int32_t)) != cudaSuccess || c->oldacc_s.ensure(n * sizeof(float)) != cudaSuccess ||
      c->oldacc_in.ensure(n * sizeof(float)) != cudaSuccess || (active && c->t_in.ensure(nt * sizeof(int32_t) + 16) != cudaSuccess))
     return fail(c, GPUGRAV_ERR_OOM, "gpugrav_walk: device allocation");
-  WalkConst wc;
+  gg::HostIo *io = c->io();
+  if(!io)
+    return fail(c, GPUGRAV_ERR_OOM, "gpugrav_walk: pinned allocation");
+  WalkConst &wc = io->wc;
   make_walk_const(c->prm, &wc);
   if(wc.ewald)
     {
@@ -829,14 +838,19 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
       if(ninter)
         CK(cudaMemcpyAsync(ninter, d_nint, nout * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "download interactions");
     }
-  unsigned long long tot = 0;
-  int walk_err = 0;
-  CK(cudaMemcpyAsync(&tot, c->counters.as<int>() + 32, 8, cudaMemcpyDeviceToHost, st), "interaction total");
-  CK(cudaMemcpyAsync(&walk_err, c->counters.as<int>() + 14, 4, cudaMemcpyDeviceToHost, st), "walk flags");
+  // counters[13]: layout self-check, [14]: walk flags, [32..33]: interaction total
+  CK(cudaMemcpyAsync(io->counters, c->counters.p, kCounters * sizeof(int), cudaMemcpyDeviceToHost, st), "walk flags");
   cudaEventRecord(c->ev[10], st);
   CK(cudaStreamSynchronize(st), "walk");
-  if(walk_err)
+  if(fp32 && io->counters[13])
+    {
+      c->layout32_valid = false;
+      return fail(c, GPUGRAV_ERR_CUDA, "fp32 walk: layout self-check failed");
+    }
+  if(io->counters[14])
     return fail(c, GPUGRAV_ERR_DEEP_TREE, "gpugrav_walk: traversal stack of the FP32 walk exhausted");
+  unsigned long long tot = 0;
+  memcpy(&tot, io->counters + 32, sizeof(tot));
   c->timings.walk_ms              = elapsed(c->ev[8], c->ev[9]);
   c->timings.download_ms          = elapsed(c->ev[9], c->ev[10]);
   c->timings.interactions         = (int64_t)tot;
@@ -855,7 +869,10 @@ int gravity_direct_impl(gpugrav_ctx *c, int64_t n, const double *pos, const doub
   DeviceGuard g(c->device);
   cudaStream_t st = c->stream;
   c->loaded = c->built = false;  // the particle buffers are reused
-  WalkConst wc;
+  gg::HostIo *io = c->io();
+  if(!io)
+    return fail(c, GPUGRAV_ERR_OOM, "gpugrav_gravity_direct: pinned allocation");
+  WalkConst &wc = io->wc;
   make_walk_const(c->prm, &wc);
   if(wc.ewald)
     {
@@ -867,6 +884,39 @@ int gravity_direct_impl(gpugrav_ctx *c, int64_t n, const double *pos, const doub
   const uint8_t *d_st = softtype;
   double *d_acc = acc, *d_pot = pot;
   int32_t *d_nint = ninter;
+  if(mem == GPUGRAV_MEM_HOST && n <= kStagedDirect)
+    {
+      // small sets, where each separate copy costs more than the kernel: one transfer each way through pinned
+      // memory, positions | masses | accelerations | potentials | flag | types in one block
+      const size_t out = (size_t)n * 32, flag_at = out + (size_t)n * 32, bytes = flag_at + 16 + (size_t)n;
+      if(c->stage.ensure(bytes) != cudaSuccess || c->dir_io.ensure(bytes) != cudaSuccess)
+        return fail(c, GPUGRAV_ERR_OOM, "gpugrav_gravity_direct: staging");
+      char *h = (char *)c->stage.p, *d = c->dir_io.as<char>();
+      memcpy(h, pos, n * 24);
+      memcpy(h + n * 24, mass, n * 8);
+      *(int *)(h + flag_at) = 0;
+      memcpy(h + flag_at + 16, softtype, n);
+      CK(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st), "upload");
+      cudaEventRecord(c->ev[8], st);
+      CK(gg::gravity_direct_stage(c, n, (double *)d, (double *)(d + n * 24), (uint8_t *)(d + flag_at + 16), (double *)(d + out),
+                                  (double *)(d + out + n * 24), nullptr, (int *)(d + flag_at)),
+         "direct summation");
+      cudaEventRecord(c->ev[9], st);
+      CK(cudaMemcpyAsync(h + out, d + out, flag_at + 4 - out, cudaMemcpyDeviceToHost, st), "download");
+      CK(cudaStreamSynchronize(st), "direct summation");
+      if(*(int *)(h + flag_at))
+        return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_gravity_direct: softening type >= nsofttypes");
+      memcpy(acc, h + out, n * 24);
+      if(pot)
+        memcpy(pot, h + out + n * 24, n * 8);
+      if(ninter)
+        for(int64_t i = 0; i < n; i++)
+          ninter[i] = (int32_t)n;
+      c->timings.walk_ms              = elapsed(c->ev[8], c->ev[9]);
+      c->timings.interactions         = n * n;
+      c->timings.walk_kernel_launches = 1;
+      return GPUGRAV_OK;
+    }
   if(mem == GPUGRAV_MEM_HOST)
     {
       if(c->pos_in.ensure(n * 24) != cudaSuccess || c->mass_in.ensure(n * 8) != cudaSuccess || c->st_in.ensure(n + 16) != cudaSuccess ||
@@ -1097,6 +1147,14 @@ int32_t gpugrav_get_topnodes(gpugrav_ctx *c, gpugrav_topnode *top, int32_t capac
     return GPUGRAV_ERR_INVALID;
   if(!c->built)
     return fail(c, GPUGRAV_ERR_STATE, "no tree built");
+  if(c->top_dev)
+    {
+      DeviceGuard g(c->device);
+      c->top_host.resize(c->ntop);
+      CK(cudaMemcpyAsync(c->top_host.data(), c->top.p, c->ntop * sizeof(gpugrav_topnode), cudaMemcpyDeviceToHost, c->stream), "top nodes");
+      CK(cudaStreamSynchronize(c->stream), "top nodes");
+      c->top_dev = false;
+    }
   *ntop = (int32_t)c->top_host.size();
   if(top)
     {

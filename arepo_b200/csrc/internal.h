@@ -52,6 +52,7 @@ struct BuildConst
 };
 
 constexpr int kSortFlag     = 24;  // gpugrav_ctx::counters: sort_lead_stage's flag in the serving loop
+constexpr int kTopCount     = 40;  // gpugrav_ctx::counters: nodes of the library's top tree (< 0: it could not be refined)
 constexpr int kNeedFullSort = 1;   // build_stage status: the particles are not in full key order yet
 
 // Walk constants
@@ -156,6 +157,26 @@ struct DevBuf
   }
 };
 
+// validated top tree (device copy filled by k_skeleton)
+struct SkelInfo
+{
+  int32_t ntop_nodes;  // nodes created (NTopnodes)
+  int32_t nleaves;
+  int32_t status;      // 0 ok, <0 invalid top tree
+  int32_t max_top_depth;
+};
+
+constexpr int kCounters = 64;  // ints in gpugrav_ctx::counters
+struct HostIo
+{
+  BuildConst bc;
+  WalkConst wc;
+  alignas(64) unsigned char w32[8192];  // constants of the group walk
+  int counters[kCounters];
+  SkelInfo skel;
+  int32_t mdyn;             // nodes below the top tree
+};
+
 struct PinnedBuf
 {
   void *p    = nullptr;
@@ -191,7 +212,9 @@ struct gpugrav_ctx
   int32_t max_depth  = 0;
   int32_t hack_cells = 0;
   gpugrav_domain dom{};
-  std::vector<gpugrav_topnode> top_host;
+  std::vector<gpugrav_topnode> top_host;  // the caller's top tree, or the library's once it has been asked for
+  bool top_dev = false;                   // library-built top tree: on the device, top_host not filled yet
+  int32_t ntop_cap = 0;                   // ... and the bound on its nodes
 
   // ---- device buffers ----
   gg::DevBuf bconst, wconst;
@@ -256,7 +279,10 @@ struct gpugrav_ctx
   gg::DevBuf out_acc, out_pot, out_nint;      // caller order staging for host copies
   gg::DevBuf scratch;                         // reductions
   gg::DevBuf dir_buf, dir_io;                 // direct summation: working space; targets and results
-  gg::PinnedBuf pinned;
+  gg::PinnedBuf pinned, stage;  // HostIo; arrays of small direct sums
+  // Pinned block for the small transfers of a call: what several kernels leave for the host comes back
+  // together, with one wait, and constants go out without staging.  Every call that uses it ends with a wait.
+  gg::HostIo *io() { return pinned.ensure(sizeof(gg::HostIo)) == cudaSuccess ? (gg::HostIo *)pinned.p : nullptr; }
 
   cudaEvent_t ev[20] = {};
   gpugrav_timings timings{};

@@ -884,14 +884,16 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
   SCK(cudaGraphLaunch(s->graph, st), "walk graph");
   cudaEventRecord(c->ev[15], st);
   s->graph_replays++;
-  int walk_err                = 0;
-  unsigned long long inter    = 0;
-  SCK(cudaMemcpyAsync(&walk_err, c->counters.as<int>() + 14, 4, cudaMemcpyDeviceToHost, st), "walk flags");
-  SCK(cudaMemcpyAsync(&inter, c->counters.as<int>() + 32, 8, cudaMemcpyDeviceToHost, st), "walk flags");
+  int *flags = c->io()->counters;  // pinned (the build has made it)
+  SCK(cudaMemcpyAsync(flags, c->counters.p, kCounters * sizeof(int), cudaMemcpyDeviceToHost, st), "walk flags");
   SCK(cudaMemsetAsync(c->counters.as<int>() + 32, 0, 8, st), "walk flags");
   SCK(cudaStreamSynchronize(st), "tick");
+  unsigned long long inter = 0;
+  memcpy(&inter, flags + 32, sizeof(inter));
   c->mark("s3 walk graph");
-  if(walk_err)
+  if(flags[13])
+    return sfail(s, GPUGRAV_ERR_CUDA, "layout self-check failed");
+  if(flags[14])
     return sfail(s, GPUGRAV_ERR_DEEP_TREE, "walk stack exhausted");
 
   // ---- state machine, completion ----

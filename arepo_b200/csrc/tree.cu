@@ -32,14 +32,6 @@ namespace
 __constant__ PhTable c_ph_tree;
 int g_ph_tree_ready[64] = {0};
 
-struct SkelInfo
-{
-  int32_t ntop_nodes;  // nodes created (NTopnodes)
-  int32_t nleaves;
-  int32_t status;      // 0 ok, <0 invalid top tree
-  int32_t max_top_depth;
-};
-
 __device__ __forceinline__ int morton_slot(uint64_t x, uint64_t y, uint64_t z, int depth)
 {
   // child index inside a node of depth (depth-1): bits 52-depth, x | y<<1 | z<<2 (src/gravity/forcetree.c:854-855)
@@ -389,7 +381,7 @@ __global__ void __launch_bounds__(kTopThreads) k_toptree(const u128 *__restrict_
 // 35 us from global memory); validation and output are everyone's.
 // ------------------------------------------------------------------------------
 constexpr int kSkelThreads = 128, kSkelShared = 256;
-__global__ void __launch_bounds__(kSkelThreads) k_skeleton(const gpugrav_topnode *__restrict__ top_g, int ntop, const BuildConst *__restrict__ bc,
+__global__ void __launch_bounds__(kSkelThreads) k_skeleton(const gpugrav_topnode *__restrict__ top_g, int ntop, const int *__restrict__ ntop_dev, const BuildConst *__restrict__ bc,
                                                            int32_t *__restrict__ suns, double4 *__restrict__ cl_g, uint8_t *__restrict__ depth,
                                                            int32_t *__restrict__ father, int32_t *__restrict__ leafnode,
                                                            int32_t *__restrict__ nodetop, SkelInfo *info)
@@ -397,6 +389,8 @@ __global__ void __launch_bounds__(kSkelThreads) k_skeleton(const gpugrav_topnode
   __shared__ gpugrav_topnode top_sh[kSkelShared];
   __shared__ double4 cl_sh[kSkelShared];
   __shared__ int s_leaves, s_bad;
+  if(ntop_dev)
+    ntop = *ntop_dev;  // the library's top tree
   const bool fits            = ntop <= kSkelShared;
   const gpugrav_topnode *top = fits ? top_sh : top_g;
   double4 *cl                = fits ? cl_sh : cl_g;
@@ -423,7 +417,7 @@ __global__ void __launch_bounds__(kSkelThreads) k_skeleton(const gpugrav_topnode
   for(int64_t q = threadIdx.x; q < 8 * (int64_t)ntop; q += kSkelThreads)
     suns[q] = -1;
   __syncthreads();
-  if(s_bad)
+  if(s_bad || ntop < 1)
     {
       if(threadIdx.x == 0)
         info->status = -2;
@@ -500,7 +494,8 @@ __global__ void __launch_bounds__(kSkelThreads) k_skeleton(const gpugrav_topnode
 
 // top leaf of every sorted particle: walk TopNodes with MortonToPeanoSubnode
 // (src/gravity/forcetree.c:507-522)
-__global__ void k_topleaf(const gpugrav_topnode *__restrict__ top, const int32_t *__restrict__ leafnode, int64_t n,
+__global__ void k_topleaf(const gpugrav_topnode *__restrict__ top, const int32_t *__restrict__ leafnode,
+                          const SkelInfo *__restrict__ info, int64_t n,
                           const uint64_t *__restrict__ ix, const uint64_t *__restrict__ iy, const uint64_t *__restrict__ iz,
                           uint8_t *__restrict__ tl, int32_t *__restrict__ tlnode)
 {
@@ -508,6 +503,13 @@ __global__ void k_topleaf(const gpugrav_topnode *__restrict__ top, const int32_t
     {
       uint64_t x = ix[i], y = iy[i], z = iz[i];
       int no = 0, levels = 0;
+      if(info->status < 0)
+        {
+          // invalid top tree: the build stops after the host has read the status
+          tl[i]     = 0;
+          tlnode[i] = 0;
+          continue;
+        }
       while(top[no].daughter >= 0 && levels < 52)
         {
           int b      = 51 - levels;
@@ -1117,35 +1119,31 @@ cudaError_t ensure_ph(int device)
 }
 }  // namespace
 
+// The node count stays on the device (counters[kTopCount]); the host allocates for the bound.
 cudaError_t toptree_stage(gpugrav_ctx *c, int *status)
 {
   GG_TRY(ensure_ph(c->device));
   const int max_top = kMaxTop;
-  GG_TRY(c->top.ensure(max_top * sizeof(gpugrav_topnode)));
-  GG_TRY(c->scratch.ensure(max_top * (sizeof(TopTmp) + 3 * sizeof(int)) + 256));
-  GG_TRY(c->counters.ensure(64 * sizeof(int)));
-  char *s     = (char *)c->scratch.p;
-  TopTmp *T   = (TopTmp *)s;
-  int *queue  = (int *)(s + max_top * sizeof(TopTmp));
-  int *list   = queue + max_top;
-  int *result = c->counters.as<int>() + 8;
-  k_toptree<<<1, kTopThreads, 0, c->stream>>>(c->key.as<u128>(), c->perm.as<uint32_t>(), c->n, c->prm.top_node_factor, c->prm.multiple_domains, T, queue,
-                                              list, list + max_top, c->top.as<gpugrav_topnode>(), max_top, result);
-  GG_TRY(cudaGetLastError());
-  int r = 0;
-  GG_TRY(cudaMemcpyAsync(&r, result, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  GG_TRY(cudaStreamSynchronize(c->stream));
-  if(r < 0)
+  const int a = 1 + 2 * 4, b = (int)(c->prm.top_node_factor * c->prm.multiple_domains);
+  c->ntop_cap = 2 * (a > b ? a : b) + 8;  // k_toptree's limit and one refinement more
+  *status     = GPUGRAV_OK;
+  if(c->ntop_cap > max_top)
     {
       *status = GPUGRAV_ERR_TOPNODES;
       return cudaSuccess;
     }
-  c->ntop = r;
-  c->top_host.resize(r);
-  GG_TRY(cudaMemcpyAsync(c->top_host.data(), c->top.p, r * sizeof(gpugrav_topnode), cudaMemcpyDeviceToHost, c->stream));
-  GG_TRY(cudaStreamSynchronize(c->stream));
-  *status = GPUGRAV_OK;
-  return cudaSuccess;
+  GG_TRY(c->top.ensure(max_top * sizeof(gpugrav_topnode)));
+  GG_TRY(c->scratch.ensure(max_top * (sizeof(TopTmp) + 3 * sizeof(int)) + 256));
+  GG_TRY(c->counters.ensure(kCounters * sizeof(int)));
+  char *s     = (char *)c->scratch.p;
+  TopTmp *T   = (TopTmp *)s;
+  int *queue  = (int *)(s + max_top * sizeof(TopTmp));
+  int *list   = queue + max_top;
+  k_toptree<<<1, kTopThreads, 0, c->stream>>>(c->key.as<u128>(), c->perm.as<uint32_t>(), c->n, c->prm.top_node_factor,
+                                              c->prm.multiple_domains, T, queue, list, list + max_top, c->top.as<gpugrav_topnode>(),
+                                              max_top, c->counters.as<int>() + kTopCount);
+  c->top_dev = true;
+  return cudaGetLastError();
 }
 
 // Builds the whole tree: skeleton, nodes, moments, threading, walk layout.
@@ -1184,7 +1182,7 @@ cudaError_t build_reserve(gpugrav_ctx *c, int64_t n, int64_t nn, int32_t ntop)
   GG_TRY(c->cnt.ensure((n + 16) * sizeof(int32_t)));
   GG_TRY(c->base.ensure((n + 16) * sizeof(int32_t)));
   GG_TRY(c->hack_list.ensure((n + 16) * sizeof(int32_t)));
-  GG_TRY(c->counters.ensure(64 * sizeof(int)));
+  GG_TRY(c->counters.ensure(kCounters * sizeof(int)));
   GG_TRY(c->skel.ensure(sizeof(SkelInfo) + (size_t)(ntop + 8) * 2 * sizeof(int32_t)));
   GG_TRY(node_arrays(c, nn + 16));
   size_t tb = 0;
@@ -1246,10 +1244,14 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
 {
   GG_TRY(ensure_ph(c->device));
   const int64_t n    = c->n;
-  const int32_t ntop = c->ntop;
+  const bool lib_top = !c->multi && c->top_dev;      // top tree built by toptree_stage: its size is on the device
+  int32_t ntop       = lib_top ? c->ntop_cap : c->ntop;  // ... and this its bound until the host has read it
   cudaStream_t st    = c->stream;
   int launches       = 0;
   *status            = GPUGRAV_OK;
+  HostIo *io         = c->io();
+  if(!io)
+    return cudaErrorMemoryAllocation;
   c->mark(nullptr);
 
   GG_TRY(c->s_cd.ensure(n + 16));
@@ -1258,7 +1260,7 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
   GG_TRY(c->cnt.ensure((n + 16) * sizeof(int32_t)));
   GG_TRY(c->base.ensure((n + 16) * sizeof(int32_t)));
   GG_TRY(c->hack_list.ensure((n + 16) * sizeof(int32_t)));
-  GG_TRY(c->counters.ensure(64 * sizeof(int)));
+  GG_TRY(c->counters.ensure(kCounters * sizeof(int)));
   GG_TRY(c->skel.ensure(sizeof(SkelInfo) + (size_t)(ntop + 8) * 2 * sizeof(int32_t)));
   int *counters     = c->counters.as<int>();
   SkelInfo *sinfo   = (SkelInfo *)c->skel.p;
@@ -1283,19 +1285,12 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
     }
   else
     {
-      k_skeleton<<<1, kSkelThreads, 0, st>>>(c->top.as<gpugrav_topnode>(), ntop, c->bconst.as<BuildConst>(), c->n_suns.as<int32_t>(),
-                                    c->n_cl.as<double4>(), c->n_depth.as<uint8_t>(), c->n_father.as<int32_t>(), leafnode, nodetop, sinfo);
+      k_skeleton<<<1, kSkelThreads, 0, st>>>(c->top.as<gpugrav_topnode>(), ntop, lib_top ? counters + kTopCount : nullptr,
+                                    c->bconst.as<BuildConst>(), c->n_suns.as<int32_t>(), c->n_cl.as<double4>(),
+                                    c->n_depth.as<uint8_t>(), c->n_father.as<int32_t>(), leafnode, nodetop, sinfo);
       launches++;
-      SkelInfo si;
-      GG_TRY(cudaMemcpyAsync(&si, sinfo, sizeof(si), cudaMemcpyDeviceToHost, st));
-      GG_TRY(cudaStreamSynchronize(st));
-      if(si.status < 0 || si.ntop_nodes != ntop)
-        {
-          *status = GPUGRAV_ERR_TOPNODES;
-          return cudaSuccess;
-        }
-      c->nleaves = si.nleaves;
-      k_topleaf<<<grid_for(n, 256), 256, 0, st>>>(c->top.as<gpugrav_topnode>(), leafnode, n, c->s_ix.as<uint64_t>(),
+      GG_TRY(cudaMemcpyAsync(&io->skel, sinfo, sizeof(SkelInfo), cudaMemcpyDeviceToHost, st));
+      k_topleaf<<<grid_for(n, 256), 256, 0, st>>>(c->top.as<gpugrav_topnode>(), leafnode, sinfo, n, c->s_ix.as<uint64_t>(),
                                                    c->s_iy.as<uint64_t>(), c->s_iz.as<uint64_t>(), c->s_tl.as<uint8_t>(),
                                                    c->s_tlnode.as<int32_t>());
       launches++;
@@ -1327,9 +1322,31 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
   GG_TRY(cudaMemsetAsync(counters, 0, 16 * sizeof(int), st));
   k_count<<<grid_for(n + 1, 256), 256, 0, st>>>(a, c->cnt.as<int32_t>(), c->hack_list.as<int32_t>(), counters);
   launches++;
-  int hc[kSortFlag + 1];
-  GG_TRY(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, st));
+  // numbering: exclusive scan of the per-particle node counts (again where cells are replayed below)
+  auto number_nodes = [&]() -> cudaError_t {
+    size_t tb = 0;
+    GG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, c->cnt.as<int32_t>(), c->base.as<int32_t>(), (int)(n + 1), st));
+    GG_TRY(c->sort_tmp.ensure(tb));
+    GG_TRY(cub::DeviceScan::ExclusiveSum(c->sort_tmp.p, tb, c->cnt.as<int32_t>(), c->base.as<int32_t>(), (int)(n + 1), st));
+    launches++;
+    return cudaMemcpyAsync(&io->mdyn, c->base.as<int32_t>() + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+  };
+  GG_TRY(number_nodes());
+  int *hc = io->counters;
+  GG_TRY(cudaMemcpyAsync(hc, counters, kCounters * sizeof(int), cudaMemcpyDeviceToHost, st));
   GG_TRY(cudaStreamSynchronize(st));
+  if(!c->multi)
+    {
+      if(lib_top)
+        ntop = c->ntop = hc[kTopCount];
+      if(ntop < 1 || io->skel.status < 0 || io->skel.ntop_nodes != ntop)
+        {
+          *status = GPUGRAV_ERR_TOPNODES;
+          return cudaSuccess;
+        }
+      c->nleaves = io->skel.nleaves;
+      a.ntop     = ntop;
+    }
   if(c->multi && hc[kSortFlag])
     {
       *status = kNeedFullSort;  // the serving loop sorts the full keys and builds again
@@ -1359,18 +1376,14 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
       launches += 2;
     }
 
-  c->mark("b2 count+hack");
-  // 3. numbering: exclusive scan of per-particle node counts
-  {
-    size_t tb = 0;
-    GG_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, c->cnt.as<int32_t>(), c->base.as<int32_t>(), (int)(n + 1), st));
-    GG_TRY(c->sort_tmp.ensure(tb));
-    GG_TRY(cub::DeviceScan::ExclusiveSum(c->sort_tmp.p, tb, c->cnt.as<int32_t>(), c->base.as<int32_t>(), (int)(n + 1), st));
-    launches++;
-  }
-  int32_t mdyn = 0;
-  GG_TRY(cudaMemcpyAsync(&mdyn, c->base.as<int32_t>() + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  GG_TRY(cudaStreamSynchronize(st));
+  if(nh > 0)
+    {
+      GG_TRY(number_nodes());
+      GG_TRY(cudaStreamSynchronize(st));
+    }
+  const int32_t mdyn = io->mdyn;
+  c->mark("b2 count+scan");
+  // 3. node storage
   const int64_t nn = (int64_t)ntop + mdyn;
   if(n + nn >= (int64_t)INT32_MAX)
     {
@@ -1381,7 +1394,6 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
   c->n_entries = n + nn;
   a.nn         = nn;
 
-  c->mark("b3 scan");
   // grow node arrays, keeping the skeleton written by k_skeleton
   if((size_t)nn * 8 * sizeof(int32_t) > c->n_suns.cap || (size_t)nn * sizeof(double4) > c->n_cl.cap ||
      (size_t)nn + 16 > c->n_depth.cap || (size_t)nn * sizeof(int32_t) > c->n_father.cap)
@@ -1396,8 +1408,9 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
         k_roots<<<grid_for(ntop, 128), 128, 0, st>>>(ntop, mdoms, c->n_suns.as<int32_t>(), c->n_cl.as<double4>(),
                                                       c->n_depth.as<uint8_t>(), c->n_father.as<int32_t>());
       else
-        k_skeleton<<<1, kSkelThreads, 0, st>>>(c->top.as<gpugrav_topnode>(), ntop, c->bconst.as<BuildConst>(), c->n_suns.as<int32_t>(),
-                                      c->n_cl.as<double4>(), c->n_depth.as<uint8_t>(), c->n_father.as<int32_t>(), leafnode, nodetop, sinfo);
+        k_skeleton<<<1, kSkelThreads, 0, st>>>(c->top.as<gpugrav_topnode>(), ntop, nullptr, c->bconst.as<BuildConst>(),
+                                      c->n_suns.as<int32_t>(), c->n_cl.as<double4>(), c->n_depth.as<uint8_t>(),
+                                      c->n_father.as<int32_t>(), leafnode, nodetop, sinfo);
       launches++;
     }
 
@@ -1441,11 +1454,12 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
   c->mark("b6 threading+layout64");
   c->timings.build_kernel_launches = launches;
   GG_TRY(cudaGetLastError());
-  int out[9] = {};  // counters[4]: deepest level, [12]: self-check flags
-  GG_TRY(cudaMemcpyAsync(out, counters + 4, sizeof(out), cudaMemcpyDeviceToHost, st));
+  cudaEventRecord(c->ev[6], st);
+  // counters[4]: deepest level, [12]: self-check flags
+  GG_TRY(cudaMemcpyAsync(io->counters, counters, kCounters * sizeof(int), cudaMemcpyDeviceToHost, st));
   GG_TRY(cudaStreamSynchronize(st));
-  c->max_depth  = out[0];
-  const int err = out[8];
+  c->max_depth  = io->counters[4];
+  const int err = io->counters[12];
   if(err)
     {
       c->err  = "tree build self-check failed (flags " + std::to_string(err) + ")";

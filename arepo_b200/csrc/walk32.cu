@@ -845,7 +845,7 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
                                                         const W32Const *__restrict__ wcp,
                                                         int *__restrict__ stack_base, int *__restrict__ work,
                                                         double4 *__restrict__ res_out, int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total,
-                                                        int *__restrict__ err)
+                                                        int *__restrict__ err, const int *__restrict__ layout_err)
 {
   constexpr int kWarps = Shape<R, PERIODIC, TPL>::warps;
   constexpr bool WRAP  = PERIODIC || EWALD;  // nearest images in a periodic box
@@ -867,6 +867,8 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
     }
   __syncthreads();
 
+  if(*layout_err)
+    return;  // the layout's self-check failed: its indices cannot be trusted
   int *stack = stack_base + ((int64_t)blockIdx.x * kWarps + warp) * kStackCap;
   WarpSh<R, TPL> &ws = sh.warp[warp];
   List<R> L;
@@ -1577,11 +1579,6 @@ cudaError_t layout32_stage(gpugrav_ctx *c)
                                                    mns ? c->n_mpt.as<double>() : nullptr, c->prm.nsofttypes,
                                                    mns ? c->g_mpt.as<float>() : nullptr);
   GG_TRY(cudaGetLastError());
-  int e = 0;
-  GG_TRY(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  GG_TRY(cudaStreamSynchronize(st));
-  if(e)
-    return cudaErrorUnknown;
   c->mark("l1 layout32");
   GG_TRY(groups_stage(c));
   c->mark("l2 groups");
@@ -1613,7 +1610,11 @@ cudaError_t walk32_prepare(gpugrav_ctx *c, const WalkConst &wc)
   if(!c->layout32_valid)
     GG_TRY(layout32_stage(c));
   cudaStream_t st = c->stream;
-  W32Const w;
+  HostIo *io = c->io();
+  if(!io)
+    return cudaErrorMemoryAllocation;
+  static_assert(sizeof(W32Const) <= sizeof(io->w32), "pinned block");
+  W32Const &w = *(W32Const *)io->w32;
   make_w32(wc, &w);
   if(wc.ewald)
     {
@@ -1624,7 +1625,6 @@ cudaError_t walk32_prepare(gpugrav_ctx *c, const WalkConst &wc)
     w.mpt = c->g_mpt.as<float>();
   GG_TRY(c->scratch.ensure(sizeof(W32Const) + 256));
   GG_TRY(cudaMemcpyAsync(c->scratch.p, &w, sizeof(w), cudaMemcpyHostToDevice, st));
-  GG_TRY(cudaStreamSynchronize(st));  // `w` lives on this stack frame
   int dev = 0, sms = 0, per_sm = 0;
   GG_TRY(cudaGetDevice(&dev));
   GG_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1674,7 +1674,7 @@ cudaError_t walk32_launch(gpugrav_ctx *c)
                                               c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr,
                                               (const W32Const *)c->scratch.p,
                                               c->g_stack.as<int>(), work, c->res_s.as<double4>(),
-                                              c->nint_s.as<int32_t>(), (unsigned long long *)(c->counters.as<int>() + 32), err);
+                                              c->nint_s.as<int32_t>(), (unsigned long long *)(c->counters.as<int>() + 32), err, c->counters.as<int>() + 13);
   return cudaGetLastError();
 }
 
