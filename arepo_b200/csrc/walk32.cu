@@ -543,24 +543,21 @@ __device__ __forceinline__ void evaluate_region(const V4<R> *__restrict__ LP, co
           e[u]  = LP[j + u];
           hj[u] = CHECK ? LH[j + u] : R(0);
         }
-      bool soft = false;
+      unsigned soft = 0;
 #pragma unroll
       for(int u = 0; u < U; u++)
 #pragma unroll
         for(int k = 0; k < TPL; k++)
-          soft |= far<R, PERIODIC, POT, EWALD, CHECK, MASK>(e[u], hj[u], T[k], w, tab);
-      if(CHECK && soft)
-        {
-#pragma unroll 1
-          for(int u = 0; u < U; u++)
-            {
-              const V4<R> eu = LP[j + u];
-              const R hu     = LH[j + u];
-#pragma unroll
-              for(int k = 0; k < TPL; k++)
-                near<R, PERIODIC, POT>(eu, hu, T[k], w, tab);
-            }
-        }
+          soft |= far<R, PERIODIC, POT, EWALD, CHECK, MASK>(e[u], hj[u], T[k], w, tab) ? 1u << (u * TPL + k) : 0u;
+      if(CHECK)
+        for(; soft; soft &= soft - 1)
+          {
+            const int b = __ffs(soft) - 1;
+            if(TPL == 2 && (b & 1))
+              near<R, PERIODIC, POT>(LP[j + b / TPL], LH[j + b / TPL], T[TPL - 1], w, tab);
+            else
+              near<R, PERIODIC, POT>(LP[j + b / TPL], LH[j + b / TPL], T[0], w, tab);
+          }
     }
   for(; j < nl; j++)
     {
@@ -616,23 +613,24 @@ struct Sum2
   f2 ax, ay, az, pot;
 };
 
-// far() without CHECK for the lane's two targets at once (outside every target's softening length); N: the
-// targets' negated positions
-template <bool PERIODIC, bool POT, bool MASK>
-__device__ __forceinline__ void far2(const float4 e, const f2 (&N)[3], Tgt<float> (&T)[2], Sum2 &S, const W32Const &w, TabRef tab, f2 afac,
-                                     f2 big)
+// far() for the lane's two targets at once; N: their negated positions.  CHECK (near list, hj the entry's
+// softening): bit k of the result says that target k lies inside the softening length (masked here).
+template <bool PERIODIC, bool POT, bool MASK, bool CHECK>
+__device__ __forceinline__ unsigned far2(const float4 e, const float hj, const f2 (&N)[3], Tgt<float> (&T)[2], Sum2 &S, const W32Const &w,
+                                         TabRef tab, f2 afac, f2 big)
 {
   const f2 dx = add2(pk(e.x, e.x), N[0]), dy = add2(pk(e.y, e.y), N[1]), dz = add2(pk(e.z, e.z), N[2]);
   const f2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
   float r2a, r2b;
   upk(r2, r2a, r2b);
-  const float ra = rsqrt_normal(r2a), rb = rsqrt_normal(r2b);
+  const float ra = rsqrt_normal(CHECK ? fmaxf(r2a, 1.0e-30f) : r2a), rb = rsqrt_normal(CHECK ? fmaxf(r2b, 1.0e-30f) : r2b);
   const f2 rinv = pk(ra, rb);
+  const f2 r    = mul2(r2, rinv);
   float ma = e.w, mb = e.w;
+  f2 ff = 0, fpt = pk(-1.0f, -1.0f);
   if(PERIODIC)
     {
-      const f2 r = mul2(r2, rinv);
-      f2 tb      = fma2_rd(r, afac, big);
+      f2 tb = fma2_rd(r, afac, big);
       float ta, tc;
       upk(tb, ta, tc);
       if(MASK)
@@ -649,56 +647,95 @@ __device__ __forceinline__ void far2(const float4 e, const f2 (&N)[3], Tgt<float
       const float4 qa = tab.row[(__float_as_int(ta) - 0x4B400000) * kCopies], qb = tab.row[(__float_as_int(tc) - 0x4B400000) * kCopies];
       float wa, wb;
       upk(fma2(r, afac, fma2(tb, pk(-1.0f, -1.0f), big)), wa, wb);
-      const f2 ff = pk(fmaf(wa, qa.y, qa.x), fmaf(wb, qb.y, qb.x));
-      const f2 mr = mul2(pk(ma, mb), rinv);
-      const f2 fm = mul2(mr, fma2(rinv, rinv, ff));
-      S.ax        = fma2(dx, fm, S.ax);
-      S.ay        = fma2(dy, fm, S.ay);
-      S.az        = fma2(dz, fm, S.az);
-      if(POT)
-        S.pot = fma2(mr, pk(fmaf(wa, qa.w, qa.z), fmaf(wb, qb.w, qb.z)), S.pot);
+      ff  = pk(fmaf(wa, qa.y, qa.x), fmaf(wb, qb.y, qb.x));
+      fpt = pk(fmaf(wa, qa.w, qa.z), fmaf(wb, qb.w, qb.z));
     }
-  else
+  else if(MASK)
     {
-      const f2 mr = mul2(pk(ma, mb), rinv);
-      const f2 fm = mul2(mr, mul2(rinv, rinv));
-      S.ax        = fma2(dx, fm, S.ax);
-      S.ay        = fma2(dy, fm, S.ay);
-      S.az        = fma2(dz, fm, S.az);
-      if(POT)
-        S.pot = fma2(mr, pk(-1.0f, -1.0f), S.pot);
+      T[0].ni++;
+      T[1].ni++;
     }
+  unsigned soft = 0;
+  if(CHECK)
+    {
+      float r_a, r_b;
+      upk(r, r_a, r_b);
+      const bool sa = r_a < fmaxf(T[0].h, hj), sb = r_b < fmaxf(T[1].h, hj);
+      ma   = sa ? 0.0f : ma;
+      mb   = sb ? 0.0f : mb;
+      soft = (sa ? 1u : 0u) | (sb ? 2u : 0u);
+    }
+  const f2 mr = mul2(pk(ma, mb), rinv);
+  const f2 fm = mul2(mr, PERIODIC ? fma2(rinv, rinv, ff) : mul2(rinv, rinv));
+  S.ax        = fma2(dx, fm, S.ax);
+  S.ay        = fma2(dy, fm, S.ay);
+  S.az        = fma2(dz, fm, S.az);
+  if(POT)
+    S.pot = fma2(mr, fpt, S.pot);
+  return soft;
 }
 
-// evaluate_region without CHECK for two FP32 targets per lane
-template <bool PERIODIC, bool POT, bool MASK>
-__device__ __forceinline__ void evaluate_region2(const float4 *__restrict__ LP, int nl, Tgt<float> (&T)[2], const W32Const &w, TabRef tab)
+// evaluate_region for two FP32 targets per lane
+template <bool PERIODIC, bool POT, bool MASK, bool CHECK>
+__device__ __forceinline__ void evaluate_region2(const float4 *__restrict__ LP, const float *__restrict__ LH, int nl, Tgt<float> (&T)[2],
+                                                 const W32Const &w, TabRef tab)
 {
   constexpr int U = kUnroll<2>;
   Sum2 S;
-  S.ax  = pk(T[0].ax, T[1].ax);
-  S.ay  = pk(T[0].ay, T[1].ay);
-  S.az  = pk(T[0].az, T[1].az);
-  S.pot = pk(T[0].pot, T[1].pot);
+  auto pack = [&]() {
+    S.ax  = pk(T[0].ax, T[1].ax);
+    S.ay  = pk(T[0].ay, T[1].ay);
+    S.az  = pk(T[0].az, T[1].az);
+    S.pot = pk(T[0].pot, T[1].pot);
+  };
+  auto unpack = [&]() {
+    upk(S.ax, T[0].ax, T[1].ax);
+    upk(S.ay, T[0].ay, T[1].ay);
+    upk(S.az, T[0].az, T[1].az);
+    upk(S.pot, T[0].pot, T[1].pot);
+  };
+  // the pairs of the last entries that lie inside the softening length (bit 2 u + k)
+  auto softened = [&](int j, unsigned bits) {
+    unpack();
+#pragma unroll 1
+    for(; bits; bits &= bits - 1)
+      {
+        const int b = __ffs(bits) - 1;
+        if(b & 1)
+          near<float, PERIODIC, POT>(LP[j + (b >> 1)], LH[j + (b >> 1)], T[1], w, tab);
+        else
+          near<float, PERIODIC, POT>(LP[j + (b >> 1)], LH[j + (b >> 1)], T[0], w, tab);
+      }
+    pack();
+  };
+  pack();
   const f2 afac = pk(w.asmthfac, w.asmthfac), big = pk(12582912.0f, 12582912.0f);
   const f2 N[3] = {pk(-T[0].x, -T[1].x), pk(-T[0].y, -T[1].y), pk(-T[0].z, -T[1].z)};
   int j         = 0;
   for(; j + U <= nl; j += U)
     {
       float4 e[U];
+      float hj[U];
 #pragma unroll
       for(int u = 0; u < U; u++)
-        e[u] = LP[j + u];
+        {
+          e[u]  = LP[j + u];
+          hj[u] = CHECK ? LH[j + u] : 0.0f;
+        }
+      unsigned bits = 0;
 #pragma unroll
       for(int u = 0; u < U; u++)
-        far2<PERIODIC, POT, MASK>(e[u], N, T, S, w, tab, afac, big);
+        bits |= far2<PERIODIC, POT, MASK, CHECK>(e[u], hj[u], N, T, S, w, tab, afac, big) << (2 * u);
+      if(CHECK && bits)
+        softened(j, bits);
     }
   for(; j < nl; j++)
-    far2<PERIODIC, POT, MASK>(LP[j], N, T, S, w, tab, afac, big);
-  upk(S.ax, T[0].ax, T[1].ax);
-  upk(S.ay, T[0].ay, T[1].ay);
-  upk(S.az, T[0].az, T[1].az);
-  upk(S.pot, T[0].pot, T[1].pot);
+    {
+      const unsigned bits = far2<PERIODIC, POT, MASK, CHECK>(LP[j], CHECK ? LH[j] : 0.0f, N, T, S, w, tab, afac, big);
+      if(CHECK && bits)
+        softened(j, bits);
+    }
+  unpack();
 }
 
 // The warp's interaction list in shared memory.  Main buffer: entries outside the softening length of
@@ -725,17 +762,18 @@ __device__ __forceinline__ void evaluate(List<R> &L, Tgt<R> (&T)[TPL], double *d
   WALK_STAT(5, L.nb);
   if constexpr(TPL == 2 && sizeof(R) == 4)
     {
-      evaluate_region2<PERIODIC, POT, false>(L.P, L.na, T, w, tab);
+      evaluate_region2<PERIODIC, POT, false, false>(L.P, nullptr, L.na, T, w, tab);
       if(PERIODIC)
-        evaluate_region2<PERIODIC, POT, true>(L.P + Cap<R>::list - L.nb, L.nb, T, w, tab);
+        evaluate_region2<PERIODIC, POT, true, false>(L.P + Cap<R>::list - L.nb, nullptr, L.nb, T, w, tab);
+      evaluate_region2<PERIODIC, POT, true, true>(L.NP, L.NH, L.nn, T, w, tab);
     }
   else
     {
       evaluate_region<R, PERIODIC, POT, TPL, EWALD, false, false>(L.P, nullptr, L.na, T, w, tab);
       if(PERIODIC)  // without Rcut no entry is a border entry
         evaluate_region<R, PERIODIC, POT, TPL, EWALD, false, true>(L.P + Cap<R>::list - L.nb, nullptr, L.nb, T, w, tab);
+      evaluate_region<R, PERIODIC, POT, TPL, EWALD, true, true, NU>(L.NP, L.NH, L.nn, T, w, tab);
     }
-  evaluate_region<R, PERIODIC, POT, TPL, EWALD, true, true, NU>(L.NP, L.NH, L.nn, T, w, tab);
 #pragma unroll
   for(int k = 0; k < TPL; k++)
     {
