@@ -368,7 +368,7 @@ int32_t gpugrav_destroy(gpugrav_ctx *c)
                         &c->n_suns, &c->n_depth, &c->n_cl, &c->n_sm, &c->n_maxsoft, &c->n_size, &c->n_father, &c->n_sibling,
                         &c->n_next, &c->n_dfs, &c->n_count, &c->n_arrived, &c->n_off, &c->p_next, &c->p_father, &c->p_off, &c->w_sm, &c->w_cl, &c->w_link, &c->g_scan, &c->g_sm, &c->g_rel, &c->g_kids, &c->g_pm, &c->g_pst, &c->g_stack, &c->res_s,
                         &c->nint_s, &c->oldacc_s, &c->oldacc_in, &c->out_acc, &c->out_pot, &c->out_nint, &c->scratch,
-                        &c->g_groups, &c->g_ngroups, &c->g_gpd, &c->g_gseg, &c->g_gflag, &c->g_gid, &c->t_cd, &c->t_pd, &c->m_sys, &c->m_doms,
+                        &c->g_groups, &c->g_ngroups, &c->g_order, &c->g_gpd, &c->g_gseg, &c->g_gflag, &c->g_gid, &c->t_cd, &c->t_pd, &c->m_sys, &c->m_doms,
                         &c->pm_pos, &c->pm_mass, &c->pm_acc, &c->pm_pot, &c->ewd, &c->ewd32, &c->n_mpt, &c->w_mpt,
                         &c->g_mpt, &c->iperm, &c->t_in, &c->t_pos, &c->t_pos_alt, &c->t_idx, &c->t_idx_alt,
                         &c->cost_in, &c->cost_u, &c->cost_p, &c->slice_rng, &c->dir_buf, &c->dir_io};
@@ -794,6 +794,8 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
       c->slice_rng_on = false;
       if(!active && we == cudaSuccess)
         we = gg::slice_cost_stage(c, true);  // cost-balanced slice range, if costs are set
+      if(we == cudaSuccess)
+        we = gg::walk32_order(c, wc);
       if(we == cudaSuccess)
         we = gg::walk32_launch(c);
     }

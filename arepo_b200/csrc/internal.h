@@ -236,7 +236,7 @@ struct gpugrav_ctx
   gg::DevBuf g_sm, g_rel, g_kids;             // node: (CoM, mass) double4; (centre - CoM, len) float4; int4 links
   gg::DevBuf g_pm, g_pst;                     // particles in parent order: (x, y, z, m) double4; softening type
   gg::DevBuf g_stack;                         // per-warp traversal stacks
-  gg::DevBuf g_groups, g_ngroups;             // walk groups (first, count, root, criterion), their count
+  gg::DevBuf g_groups, g_ngroups, g_order;    // walk groups (first, count, root, criterion), their count, their order
   gg::DevBuf g_gpd, g_gseg, g_gflag, g_gid;   // group construction scratch
   gg::DevBuf t_cd, t_pd;                      // active list: pair depths of consecutive targets, their cell depths
   int32_t slice = 0, nslices = 1;             // target slice of the walks (gpugrav_set_target_slice)
@@ -271,6 +271,7 @@ struct gpugrav_ctx
   gg::DevBuf m_sys, m_doms;
   // FP32 walk launch plan (walk32_prepare)
   void *w32_kernel   = nullptr;
+  int *w32_order     = nullptr;  // order of the groups of this walk, or none
   int32_t w32_blocks = 0, w32_threads = 0;
   size_t w32_smem    = 0;
   bool want_pot       = true;  // potential requested by the current walk call
@@ -309,7 +310,7 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status);
 cudaError_t thread_stage(gpugrav_ctx *c);
 cudaError_t thread_ensure(gpugrav_ctx *c);
 cudaError_t walk64_stage(gpugrav_ctx *c, const WalkConst &wc);
-cudaError_t walk32_stage(gpugrav_ctx *c, const WalkConst &wc);
+cudaError_t walk32_order(gpugrav_ctx *c, const WalkConst &wc);
 cudaError_t walk32_prepare(gpugrav_ctx *c, const WalkConst &wc);
 cudaError_t walk32_launch(gpugrav_ctx *c);
 cudaError_t groups_stage(gpugrav_ctx *c);

@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
                                                         const uint8_t *__restrict__ g_pst, const double4 *__restrict__ tpm,
                                                         const uint8_t *__restrict__ tst, const float *__restrict__ oldacc,
                                                         const int *__restrict__ ngroups_dev, const int4 *__restrict__ groups,
-                                                        const int32_t *__restrict__ tlist, int slice, int nslices,
+                                                        const int *__restrict__ order, const int32_t *__restrict__ tlist, int slice, int nslices,
                                                         const int64_t *__restrict__ slice_rng,
                                                         const W32Const *__restrict__ wcp,
                                                         int *__restrict__ stack_base, int *__restrict__ work,
@@ -929,9 +929,10 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
 
   while(true)
     {
-      const int grp = g_begin + unit / UPG, half = SPLIT ? unit & 1 : 0;
-      if(grp >= g_end)
+      const int slot = g_begin + unit / UPG, half = SPLIT ? unit & 1 : 0;
+      if(slot >= g_end)
         break;
+      const int grp = order ? order[slot] : slot;
       // group of up to 32*TPL consecutive targets; lane holds targets t0 + lane + 32k.  A group lies
       // inside one system and walks that system's tree (root).
       const int4 G       = groups[grp];
@@ -1277,6 +1278,89 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
     }
   if(lane == 0 && ws.total)
     atomicAdd(total, ws.total);
+}
+
+// ---- order of the groups ----
+// A walk of several groups per warp ends when its last group does.  The cost of a group under the relative
+// criterion spans three orders of magnitude (a background particle amid a dense core opens the core: 180 ms
+// against 6 ms for the median group), and in key order expensive ones began as late as half-way: the last
+// third of the 328 ms walk of a 2^24-particle zoom box ran on 80 of 3552 warps.  So the groups go by falling
+// cost, as far as it can be told before the walk: by the binary exponent of their smallest OldAcc, which
+// opens the most, and by key within one exponent.  That walk takes 250 ms (240 ms for all warps busy to the
+// end).  Every group's result is its own; the order changes none.
+constexpr int kOrderBlock = 256;
+constexpr int kOrderRun   = 4;  // consecutive groups that stay together
+struct GroupOrder
+{
+  int hist[256], cursor[256];  // groups per exponent; the scatter's reservations
+};
+__device__ __forceinline__ void group_range(const int *ngroups_dev, int slice, int nslices, const int64_t *slice_rng, int &b, int &e)
+{
+  const int64_t ng = *ngroups_dev;
+  b                = slice_rng ? (int)slice_rng[0] : (int)(ng * slice / nslices);
+  e                = slice_rng ? (int)slice_rng[1] : (int)(ng * (slice + 1) / nslices);
+}
+__global__ void __launch_bounds__(kOrderBlock) k_order_key(const int *__restrict__ ngroups_dev, int slice, int nslices,
+                                                           const int64_t *__restrict__ slice_rng, const int4 *__restrict__ groups,
+                                                           const int32_t *__restrict__ tlist, const float *__restrict__ oldacc,
+                                                           uint8_t *__restrict__ key, GroupOrder *__restrict__ o)
+{
+  __shared__ int h[256];
+  for(int t = threadIdx.x; t < 256; t += blockDim.x)
+    h[t] = 0;
+  __syncthreads();
+  int b, e;
+  group_range(ngroups_dev, slice, nslices, slice_rng, b, e);
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (kOrderBlock / 32);
+  for(int r = blockIdx.x * (kOrderBlock / 32) + (threadIdx.x >> 5); b + r * kOrderRun < e; r += warps)
+    {
+      const int g0 = b + r * kOrderRun, g1 = g0 + kOrderRun < e ? g0 + kOrderRun : e;
+      // consecutive groups hold consecutive targets
+      const int4 last = groups[g1 - 1];
+      float a         = 3.0e38f;
+#pragma unroll 8
+      for(int k = groups[g0].x + lane; k < last.x + last.y; k += 32)
+        a = fminf(a, oldacc[tlist ? tlist[k] : k]);
+      a = wminf(a);
+      if(lane == 0)
+        {
+          const int x = (__float_as_int(a) >> 23) & 255;
+          key[r]      = (uint8_t)x;
+          atomicAdd(&h[x], g1 - g0);
+        }
+    }
+  __syncthreads();
+  for(int t = threadIdx.x; t < 256; t += blockDim.x)
+    if(h[t])
+      atomicAdd(&o->hist[t], h[t]);
+}
+__global__ void __launch_bounds__(kOrderBlock) k_order_scatter(const int *__restrict__ ngroups_dev, int slice, int nslices,
+                                                               const int64_t *__restrict__ slice_rng, const uint8_t *__restrict__ key,
+                                                               GroupOrder *__restrict__ o, int *__restrict__ order)
+{
+  static_assert(kOrderBlock == 256, "one thread per exponent");
+  typedef cub::BlockScan<int, kOrderBlock> Scan;
+  __shared__ typename Scan::TempStorage tmp;
+  __shared__ int cnt[256], base[256];
+  int start, b, e;
+  Scan(tmp).ExclusiveSum(o->hist[threadIdx.x], start);
+  group_range(ngroups_dev, slice, nslices, slice_rng, b, e);
+  const int runs = (e - b + kOrderRun - 1) / kOrderRun;
+  for(int r0 = blockIdx.x * kOrderBlock; r0 < runs; r0 += gridDim.x * kOrderBlock)
+    {
+      cnt[threadIdx.x] = 0;
+      __syncthreads();
+      const int r = r0 + threadIdx.x, x = r < runs ? key[r] : -1;
+      const int g0 = b + r * kOrderRun, g1 = g0 + kOrderRun < e ? g0 + kOrderRun : e;
+      const int at = x >= 0 ? atomicAdd(&cnt[x], g1 - g0) : 0;
+      __syncthreads();
+      base[threadIdx.x] = cnt[threadIdx.x] ? b + start + atomicAdd(&o->cursor[threadIdx.x], cnt[threadIdx.x]) : 0;
+      __syncthreads();
+      if(x >= 0)
+        for(int g = g0; g < g1; g++)
+          order[base[x] + at + g - g0] = g;
+      __syncthreads();
+    }
 }
 
 // ---- walk groups -------------------------------------------------------------------------
@@ -1689,6 +1773,7 @@ cudaError_t walk32_prepare(gpugrav_ctx *c, const WalkConst &wc)
   if(per_sm < 1)
     per_sm = 1;
   c->w32_kernel  = (void *)plan.kern;
+  c->w32_order   = nullptr;
   c->w32_threads = 32 * plan.warps;
   c->w32_smem    = plan.smem;
   c->w32_blocks  = sms * per_sm;
@@ -1708,7 +1793,7 @@ cudaError_t walk32_launch(gpugrav_ctx *c)
   kern<<<c->w32_blocks, c->w32_threads, c->w32_smem, st>>>(c->g_sm.as<double4>(), c->g_rel.as<float4>(), c->g_kids.as<int4>(),
                                               c->g_pm.as<double4>(), c->g_pst.as<uint8_t>(), c->s_pm.as<double4>(),
                                               c->s_st.as<uint8_t>(), c->oldacc_s.as<float>(), c->g_ngroups.as<int>(),
-                                              c->g_groups.as<int4>(), c->w_tlist, c->slice, c->nslices,
+                                              c->g_groups.as<int4>(), c->w32_order, c->w_tlist, c->slice, c->nslices,
                                               c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr,
                                               (const W32Const *)c->scratch.p,
                                               c->g_stack.as<int>(), work, c->res_s.as<double4>(),
@@ -1831,10 +1916,35 @@ cudaError_t slice_mask_stage(gpugrav_ctx *c, bool fp32)
   return cudaGetLastError();
 }
 
-cudaError_t walk32_stage(gpugrav_ctx *c, const WalkConst &wc)
+// the order of the groups of the walk to be launched (k_order_key)
+cudaError_t walk32_order(gpugrav_ctx *c, const WalkConst &wc)
 {
-  GG_TRY(walk32_prepare(c, wc));
-  return walk32_launch(c);
+  // Where some warps take more than one group (a walk that all runs at once needs no order), by the relative
+  // criterion (the geometric one, bh, does not look at OldAcc), in a tree deeper by four levels than an even
+  // set's of that size: the groups of an even set cost the same, and the 25 us of the two kernels and the
+  // neighbours' cache lines were lost there (2^24 particles of an early box, depth 8: 16.6 ms in key order,
+  // 16.8 ms in this one).
+  const int64_t targets = (c->w_ntargets > 0 ? c->w_ntargets : c->n) / c->nslices;
+  const size_t cap      = c->g_groups.cap / sizeof(int4);
+  const int levels      = c->max_depth - 4;
+  const bool deep       = levels > 20 || (levels > 0 && (int64_t)1 << (3 * levels) >= c->n);
+  if(wc.bh || !deep || targets / (32 * walk32_tpl(c)) <= (int64_t)c->w32_blocks * (c->w32_threads / 32))
+    return cudaSuccess;
+  if(c->g_order.ensure(sizeof(GroupOrder) + cap * (sizeof(int) + 1)) != cudaSuccess)
+    cudaGetLastError();  // no room: key order
+  else
+    {
+      GroupOrder *o      = c->g_order.as<GroupOrder>();
+      int *order         = (int *)(o + 1);
+      uint8_t *key       = (uint8_t *)(order + cap);
+      const int64_t *rng = c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr;
+      GG_TRY(cudaMemsetAsync(o, 0, sizeof(GroupOrder), c->stream));
+      k_order_key<<<148 * 8, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), c->slice, c->nslices, rng, c->g_groups.as<int4>(), c->w_tlist,
+                                                          c->oldacc_s.as<float>(), key, o);
+      k_order_scatter<<<148, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), c->slice, c->nslices, rng, key, o, order);
+      c->w32_order = order;
+    }
+  return cudaGetLastError();
 }
 }  // namespace gg
 
