@@ -4,10 +4,10 @@
 // with the reference's arithmetic operation for operation.  The tree is laid
 // out in the reference's traversal order (depth first, slots 0..7), so that
 // "nextnode" of an entry is the next entry and "sibling" is the entry after its
-// subtree (w_link.x).  A warp takes 32 consecutive targets in key order; each
+// subtree (w_link.x).  A warp takes up to 32 consecutive targets in key order; each
 // lane keeps its own position in its own traversal, and the warp always serves
 // the smallest position among its lanes: the entry is loaded once for the warp
-// and evaluated by exactly the lanes that are at it.  Every lane therefore sees
+// and tested by exactly the lanes that are at it.  Every lane therefore sees
 // the same interaction sequence, in the same order, as the reference walk for
 // its target -- the per-target results are bit-identical to the reference.
 #include "internal.h"
@@ -37,255 +37,232 @@ namespace
 
 __device__ __forceinline__ double nearest(double x, const WalkConst &w)
 {
-  // GRAVITY_NEAREST_X, src/main/allvars.h:602-608
-  if(!w.periodic)
-    return x;
-  return (x > w.half_box) ? (x - w.box) : ((x < -w.half_box) ? (x + w.box) : x);
+  // GRAVITY_NEAREST_X, src/main/allvars.h:602-608; selects, no branches
+  const double hb = w.periodic ? w.half_box : 1e300, lo = x - w.box, hi = x + w.box;
+  const bool a = x > hb, b = x < -hb;
+  return a ? lo : b ? hi : x;
 }
 
-constexpr int kWarps = 4;
+constexpr int kWarps  = 4;
+// Blocks per SM: 6 leave 80 registers a thread.  Even sets of 48^3 targets and zoom boxes of 240022 with
+// MULTIPLE_NODE_SOFTENING take (ms) 3.41 and 19.8 with 4, 2.35 and 19.4 with 6, 2.45 and 20.4 with 8.
+constexpr int kBlocks = 6;
 
-// EWALD (pure periodic tree) and MNS (MULTIPLE_NODE_SOFTENING) are compiled in only where used: the
-// TreePM and isolated walks keep the register budget of a kernel without them.  The walk is
-// latency-bound (lanes wait on the entry the warp serves), so occupancy beats spill-free code: on
-// the zoom box 12 blocks per SM (48 warps) walk 1.18x faster than 6 and 1.3x faster than 5.
+// The walk's tests of an internal node, src/gravity/forcetree_walk.c:196-330: opened (go on with the next
+// entry), or not -- then skipped with its subtree, and used unless it lies beyond Rcut (out).
+template <bool MNS>
+__device__ __forceinline__ void test_node(const double4 sm, const double4 cl, int type_fl, double pos_x, double pos_y, double pos_z,
+                                          double aold, double h_i, const WalkConst &w, bool &open, bool &out)
+{
+  // No short-circuit evaluation: the comparisons do not depend on one another and run side by side; a branch
+  // for each, taken by some lanes, made the test most of the walk: 32^3 targets took 1.28 ms, 0.95 ms
+  // without; a zoom box of 240022 30.5 ms, 19.4 ms without.
+  const double mass = sm.w;
+  const double dx = nearest(sm.x - pos_x, w), dy = nearest(sm.y - pos_y, w), dz = nearest(sm.z - pos_z, w);
+  const double cx = fabs(nearest(cl.x - pos_x, w)), cy = fabs(nearest(cl.y - pos_y, w)), cz = fabs(nearest(cl.z - pos_z, w));
+  const double r2  = dx * dx + dy * dy + dz * dz;
+  const double len = cl.w, len2 = len * len;
+  const double eff_dist = w.rcut + 0.5 * len;
+  out = (w.pm != 0) & (r2 > w.rcut2) & ((cx > eff_dist) | (cy > eff_dist) | (cz > eff_dist));
+  if(w.bh)
+    open = len2 > r2 * w.theta * w.theta;
+  else
+    {
+      // ACTIVATE_MINIMUM_OPENING_ANGLE adds a minimum angle to the mass test (forcetree_walk.c:266-271)
+      const double in = 0.60 * len;
+      open = (len2 > r2 * (1.2 * 1.2)) | ((mass * len2 > r2 * r2 * aold) & ((w.minangle == 0) | (len2 > r2 * (0.4 * 0.4)))) |
+             ((cx < in) & (cy < in) & (cz < in));
+    }
+  if(!MNS)
+    {
+      const double h_j = w.soft[type_fl & 0xff];
+      open             = open | ((h_j > h_i) & (r2 < h_j * h_j));
+    }
+  open = open && !out;
+}
+
+// One contribution of a walk entry (sm: centre of mass and mass, type_fl: softening type and node flag) to a
+// target, src/gravity/forcetree_walk.c:363-488, added with add(x, y, z, potential); type >= 0: the node's
+// mass of that softening type (MULTIPLE_NODE_SOFTENING, forcetree_walk.c:382-401).  False: beyond the table.
+template <bool EWALD, bool MNS, class Add>
+__device__ __forceinline__ bool interact(uint32_t e, int type, const double4 sm, int type_fl, double pos_x, double pos_y, double pos_z,
+                                         double h_i, const WalkConst &w, Add add)
+{
+  const double dx = nearest(sm.x - pos_x, w), dy = nearest(sm.y - pos_y, w), dz = nearest(sm.z - pos_z, w);
+  const double r2     = dx * dx + dy * dy + dz * dz;
+  double r            = sqrt(r2);
+  double factor_force = 0, factor_pot = 0;
+  if(w.pm)
+    {
+      double tabentry = w.asmthfac * r;
+      int tabindex    = (int)tabentry;
+      if(!(tabindex < kNtab))
+        return false;
+      double tabweight = tabentry - tabindex;
+      factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
+      factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];
+    }
+  double mass      = sm.w;
+  double h_j       = w.soft[type_fl & 0xff];
+  if(MNS && type >= 0)
+    {
+      mass = w.w_mpt[(int64_t)e * w.nsoft + type];
+      h_j  = w.soft[type];
+      if(!mass)
+        return true;
+    }
+  const double hmax = (h_j > h_i) ? h_j : h_i;
+  double fac, wp;
+  if(r >= hmax)
+    {
+      double rinv  = 1.0 / r;
+      double rinv3 = rinv * rinv * rinv;
+      if(w.pm)
+        {
+          fac = rinv3 + rinv * factor_force * w.asmthinv2;
+          wp  = rinv * factor_pot;
+        }
+      else
+        {
+          fac = rinv3;
+          wp  = -rinv;
+        }
+    }
+  else
+    {
+      double h_inv  = 1.0 / hmax;
+      double h3_inv = h_inv * h_inv * h_inv;
+      double u      = r * h_inv;
+      if(u < 0.5)
+        {
+          double u2 = u * u;
+          fac       = h3_inv * (SF1 + u2 * (SF2 * u + SF3));
+          wp        = h_inv * (SF4 + u2 * (SF5 + u2 * (SF6 * u + SF7)));
+        }
+      else
+        {
+          double u2 = u * u;
+          double u3 = u2 * u;
+          fac       = h3_inv * (SF8 + SF9 * u + SF10 * u2 + SF11 * u3 + SF12 / u3);
+          wp        = h_inv * (SF13 + SF14 / u + u2 * (SF1 + u * (SF15 + u * (SF16 + SF17 * u))));
+        }
+      if(w.pm && r > 0)
+        {
+          double rinv = 1.0 / r;
+          fac += rinv * factor_force * w.asmthinv2;
+          wp += rinv * (factor_pot + 1.0);
+        }
+    }
+  fac *= mass;
+  add(dx * fac, dy * fac, dz * fac, mass * wp);
+  if(EWALD)
+    {
+      // all further periodic images, src/gravity/forcetree_walk.c:469-477
+      double fcorr[3], pcorr;
+      ewald_corr(dx, dy, dz, w, fcorr, pcorr);
+      add(mass * fcorr[0], mass * fcorr[1], mass * fcorr[2], mass * pcorr);
+    }
+  return true;
+}
+
+// A warp takes up to 32 targets at a time, its first by number, the next from a counter: the walks of a dense
+// core and of the background differ by two orders of magnitude, and blocks of four fixed warps waited for
+// their longest.  The chain of one entry after the other bounds it: load, FP64 test, next entry, some 900
+// cycles.  Interactions are evaluated where they are found; waiting in queues and evaluated 32 at a time, they
+// were 1.2 times faster in a zoom box but 1.5 times slower in an even set of 2^18, whose warps the queues'
+// shared memory kept off the SM.
+//
+// EWALD (pure periodic tree: two contributions per entry) and MNS (MULTIPLE_NODE_SOFTENING) are compiled in
+// only where used.
 template <bool EWALD, bool MNS>
-__global__ void __launch_bounds__(32 * kWarps, 12) k_walk64(const double4 *__restrict__ w_sm, const double4 *__restrict__ w_cl,
+__global__ void __launch_bounds__(32 * kWarps, kBlocks) k_walk64(const double4 *__restrict__ w_sm, const double4 *__restrict__ w_cl,
                                                         const int2 *__restrict__ w_link, uint32_t n_entries,
                                                         const double4 *__restrict__ tpm, const uint8_t *__restrict__ tst,
                                                         const float *__restrict__ oldacc, int64_t t_begin, int64_t t_end,
                                                         const int32_t *__restrict__ tlist, const WalkConst *__restrict__ wcp,
-                                                        double4 *__restrict__ res_out, int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total)
+                                                        int tpu, int *__restrict__ work, double4 *__restrict__ res_out,
+                                                        int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total)
 {
   __shared__ WalkConst w;
   for(int t = threadIdx.x; t < (int)(sizeof(WalkConst) / 4); t += blockDim.x)
     ((int *)&w)[t] = ((const int *)wcp)[t];
   __syncthreads();
 
-  const int lane  = threadIdx.x & 31;
-  // position in the walk's target range; the target itself (sorted particle index) is the same
-  // position, or its entry in the list of active targets
-  const int64_t slot = t_begin + ((int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5)) * 32 + lane;
-  const bool valid   = slot < t_end;
-  const int64_t tgt  = valid && tlist ? (int64_t)tlist[slot] : slot;
-
-  double pos_x = 0, pos_y = 0, pos_z = 0, aold = 0, h_i = 0;
-  if(valid)
+  const int lane           = threadIdx.x & 31;
+  const int64_t units      = (t_end - t_begin + tpu - 1) / tpu;
+  unsigned long long count = 0;
+  for(int64_t u = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < units;)
     {
-      double4 p = tpm[tgt];
-      pos_x     = p.x;
-      pos_y     = p.y;
-      pos_z     = p.z;
-      aold      = w.erracc * (double)oldacc[tgt];
-      h_i       = w.soft[tst[tgt]];
-    }
-  double acc_x = 0, acc_y = 0, acc_z = 0, pot = 0;
-  int ninteractions = 0;
-  uint32_t next     = valid ? 0u : n_entries;  // entry 0 is the root (Tree_MaxPart)
+      // position in the walk's target range; the target itself (sorted particle index) is the same
+      // position, or its entry in the list of active targets
+      const int64_t slot = t_begin + u * tpu + lane;
+      const bool valid   = lane < tpu && slot < t_end;
+      const int64_t tgt  = valid && tlist ? (int64_t)tlist[slot] : slot;
 
-  while(true)
-    {
-      const uint32_t i = __reduce_min_sync(0xffffffffu, next);
-      if(i >= n_entries)
-        break;
-      const int2 link  = w_link[i];
-      const double4 sm = w_sm[i];
-      const bool node  = (link.y & kNodeFlag) != 0;
-      double4 cl       = make_double4(0, 0, 0, 0);
-      if(node)
-        cl = w_cl[i];
-      if(next != i)
-        continue;
-
-      double dx, dy, dz, r2, mass, hmax;
-      bool split = false;  // MULTIPLE_NODE_SOFTENING: node used per softening type
-      if(!node)
+      double pos_x = 0, pos_y = 0, pos_z = 0, aold = 0, h_i = 0;
+      if(valid)
         {
-          // single particle, src/gravity/forcetree_walk.c:178-195
-          dx         = nearest(sm.x - pos_x, w);
-          dy         = nearest(sm.y - pos_y, w);
-          dz         = nearest(sm.z - pos_z, w);
-          r2         = dx * dx + dy * dy + dz * dz;
-          mass       = sm.w;
-          double h_j = w.soft[link.y & 0xff];
-          hmax       = (h_j > h_i) ? h_j : h_i;
-          next       = i + 1;
+          double4 p = tpm[tgt];
+          pos_x     = p.x;
+          pos_y     = p.y;
+          pos_z     = p.z;
+          aold      = w.erracc * (double)oldacc[tgt];
+          h_i       = w.soft[tst[tgt]];
         }
-      else
-        {
-          // internal node, src/gravity/forcetree_walk.c:196-330
-          mass = sm.w;
-          dx   = nearest(sm.x - pos_x, w);
-          dy   = nearest(sm.y - pos_y, w);
-          dz   = nearest(sm.z - pos_z, w);
-          r2   = dx * dx + dy * dy + dz * dz;
-          const double len = cl.w;
-          if(w.pm && r2 > w.rcut2)
-            {
-              double eff_dist = w.rcut + 0.5 * len;
-              double dist     = nearest(cl.x - pos_x, w);
-              bool out        = (dist < -eff_dist || dist > eff_dist);
-              if(!out)
-                {
-                  dist = nearest(cl.y - pos_y, w);
-                  out  = (dist < -eff_dist || dist > eff_dist);
-                }
-              if(!out)
-                {
-                  dist = nearest(cl.z - pos_z, w);
-                  out  = (dist < -eff_dist || dist > eff_dist);
-                }
-              if(out)
-                {
-                  next = (uint32_t)link.x;
-                  continue;
-                }
-            }
-          if(w.bh)
-            {
-              if(len * len > r2 * w.theta * w.theta)
-                {
-                  next = i + 1;
-                  continue;
-                }
-            }
-          else
-            {
-              double len2 = len * len;
-              if(len2 > r2 * (1.2 * 1.2))
-                {
-                  next = i + 1;
-                  continue;
-                }
-              // ACTIVATE_MINIMUM_OPENING_ANGLE adds a minimum angle to the mass test (forcetree_walk.c:266-271)
-              if(mass * len2 > r2 * r2 * aold && (!w.minangle || len2 > r2 * (0.4 * 0.4)))
-                {
-                  next = i + 1;
-                  continue;
-                }
-              if(fabs(nearest(cl.x - pos_x, w)) < 0.60 * len && fabs(nearest(cl.y - pos_y, w)) < 0.60 * len &&
-                 fabs(nearest(cl.z - pos_z, w)) < 0.60 * len)
-                {
-                  next = i + 1;
-                  continue;
-                }
-            }
-          double h_j = w.soft[link.y & 0xff];
-          if(h_j > h_i)
-            {
-              if(MNS)
-                split = true;  // src/gravity/forcetree_walk.c:296-308
-              else if(r2 < h_j * h_j)
-                {
-                  next = i + 1;
-                  continue;
-                }
-              hmax = h_j;
-            }
-          else
-            hmax = h_i;
-          next = (uint32_t)link.x;
-        }
+      double acc_x = 0, acc_y = 0, acc_z = 0, pot = 0;
+      int ninteractions = 0;
+      auto add_own = [&](double tx, double ty, double tz, double tp) {
+        acc_x += tx;
+        acc_y += ty;
+        acc_z += tz;
+        pot += tp;
+      };
+      uint32_t next = valid ? 0u : n_entries;  // entry 0 is the root (Tree_MaxPart)
 
-      // multipole (monopole) interaction, src/gravity/forcetree_walk.c:363-488
-      if(mass)
+      while(true)
         {
-          double r            = sqrt(r2);
-          double factor_force = 0, factor_pot = 0;
-          if(w.pm)
+          const uint32_t i = __reduce_min_sync(0xffffffffu, next);
+          if(i >= n_entries)
+            break;
+          const int2 link  = w_link[i];
+          const double4 sm = w_sm[i], cl = w_cl[i];
+          const bool node  = (link.y & kNodeFlag) != 0;
+          bool open = false, out = false;
+          if(node)
+            test_node<MNS>(sm, cl, link.y, pos_x, pos_y, pos_z, aold, h_i, w, open, out);
+          const bool here = next == i, take = here && !open && !out && sm.w != 0;
+          if(here)
+            next = node && !open ? (uint32_t)link.x : i + 1;
+          // MULTIPLE_NODE_SOFTENING: a node is used per softening type, src/gravity/forcetree_walk.c:296-308
+          const bool split = MNS && node && w.soft[link.y & 0xff] > h_i;
+          if(take)
             {
-              double tabentry = w.asmthfac * r;
-              int tabindex    = (int)tabentry;
-              if(!(tabindex < kNtab))
-                continue;
-              double tabweight = tabentry - tabindex;
-              factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
-              factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];
-            }
-          // per softening type under MULTIPLE_NODE_SOFTENING (forcetree_walk.c:382-401), else once
-          const int t0 = (MNS && split) ? 0 : -1, t1 = (MNS && split) ? w.nsoft : 0;
-          for(int type = t0; type < t1; type++)
-            {
-              if(type >= 0)
-                {
-                  mass             = w.w_mpt[(int64_t)i * w.nsoft + type];
-                  const double hjt = w.soft[type];
-                  hmax             = (hjt > h_i) ? hjt : h_i;
-                }
-              if(!mass)
-                continue;
-              double fac, wp;
-              if(r >= hmax)
-                {
-                  double rinv  = 1.0 / r;
-                  double rinv3 = rinv * rinv * rinv;
-                  if(w.pm)
-                    {
-                      fac = rinv3 + rinv * factor_force * w.asmthinv2;
-                      wp  = rinv * factor_pot;
-                    }
-                  else
-                    {
-                      fac = rinv3;
-                      wp  = -rinv;
-                    }
-                }
+              bool did = false;
+              if(MNS && split)
+                for(int t = 0; t < w.nsoft; t++)
+                  did = interact<EWALD, MNS>(i, t, sm, link.y, pos_x, pos_y, pos_z, h_i, w, add_own);
               else
-                {
-                  double h_inv  = 1.0 / hmax;
-                  double h3_inv = h_inv * h_inv * h_inv;
-                  double u      = r * h_inv;
-                  if(u < 0.5)
-                    {
-                      double u2 = u * u;
-                      fac       = h3_inv * (SF1 + u2 * (SF2 * u + SF3));
-                      wp        = h_inv * (SF4 + u2 * (SF5 + u2 * (SF6 * u + SF7)));
-                    }
-                  else
-                    {
-                      double u2 = u * u;
-                      double u3 = u2 * u;
-                      fac       = h3_inv * (SF8 + SF9 * u + SF10 * u2 + SF11 * u3 + SF12 / u3);
-                      wp        = h_inv * (SF13 + SF14 / u + u2 * (SF1 + u * (SF15 + u * (SF16 + SF17 * u))));
-                    }
-                  if(w.pm && r > 0)
-                    {
-                      double rinv = 1.0 / r;
-                      fac += rinv * factor_force * w.asmthinv2;
-                      wp += rinv * (factor_pot + 1.0);
-                    }
-                }
-              pot += mass * wp;
-              fac *= mass;
-              acc_x += dx * fac;
-              acc_y += dy * fac;
-              acc_z += dz * fac;
-              if(EWALD)
-                {
-                  // all further periodic images, src/gravity/forcetree_walk.c:469-477
-                  double fcorr[3], pcorr;
-                  ewald_corr(dx, dy, dz, w, fcorr, pcorr);
-                  acc_x += mass * fcorr[0];
-                  acc_y += mass * fcorr[1];
-                  acc_z += mass * fcorr[2];
-                  pot += mass * pcorr;
-                }
+                did = interact<EWALD, false>(i, -1, sm, link.y, pos_x, pos_y, pos_z, h_i, w, add_own);
+              ninteractions += did ? 1 : 0;
             }
-          ninteractions++;
         }
-    }
 
-  if(valid)
-    {
-      res_out[tgt]  = make_double4(acc_x, acc_y, acc_z, pot);
-      nint_out[tgt] = ninteractions;
+      if(valid)
+        {
+          res_out[tgt]  = make_double4(acc_x, acc_y, acc_z, pot);
+          nint_out[tgt] = ninteractions;
+          count += (unsigned long long)ninteractions;
+        }
+      int taken = 0;
+      if(lane == 0)
+        taken = atomicAdd(work, 1);
+      u = (int64_t)kWarps * gridDim.x + __shfl_sync(0xffffffffu, taken, 0);
     }
   // interaction total for the timing report
-  unsigned long long v = valid ? (unsigned long long)ninteractions : 0ull;
   for(int o = 16; o > 0; o >>= 1)
-    v += __shfl_xor_sync(0xffffffffu, v, o);
-  if(lane == 0 && v)
-    atomicAdd(total, v);
+    count += __shfl_xor_sync(0xffffffffu, count, o);
+  if(lane == 0 && count)
+    atomicAdd(total, count);
 }
 }  // namespace
 
@@ -303,13 +280,23 @@ cudaError_t walk64_stage(gpugrav_ctx *c, const WalkConst &wc)
       t_begin = rng[2];
       t_end   = rng[3];
     }
-  const int64_t warps   = (t_end - t_begin + 31) / 32;
-  const int64_t blocks  = warps > 0 ? (warps + kWarps - 1) / kWarps : 1;
   auto kern = wc.ewald ? (wc.mns ? k_walk64<true, true> : k_walk64<true, false>)
                        : (wc.mns ? k_walk64<false, true> : k_walk64<false, false>);
-  kern<<<(unsigned)blocks, 32 * kWarps, 0, c->stream>>>(
+  int sms = 0, per_sm = 0;
+  GG_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  GG_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarps, 0));
+  // Targets per warp: as few as keep all warps running at once, 4 to 32.  The walk of a set that does not fill
+  // the chip takes as long as its longest warp, and that steps on the union of its targets' entries (ms with
+  // 4 / 8 / 16 / 32: 4096 targets 0.18 / 0.20 / 0.25 / 0.31, 15625 0.62 / 0.48 / 0.54 / 0.60, 32768
+  // 1.56 / 1.25 / 0.84 / 0.95); once there are more warps than fit, shared steps count (110592 targets: 3.75
+  // with 16, 2.35 with 32).
+  const int64_t resident = (int64_t)sms * (per_sm > 0 ? per_sm : 1) * kWarps, need = (t_end - t_begin + resident - 1) / resident;
+  const int tpu          = need < 4 ? 4 : (need > 32 ? 32 : (int)need);
+  int *work = c->counters.as<int>() + 20;
+  GG_TRY(cudaMemsetAsync(work, 0, sizeof(int), c->stream));
+  kern<<<sms * (per_sm > 0 ? per_sm : 1), 32 * kWarps, 0, c->stream>>>(
       c->w_sm.as<double4>(), c->w_cl.as<double4>(), c->w_link.as<int2>(), (uint32_t)c->n_entries, c->s_pm.as<double4>(),
-      c->s_st.as<uint8_t>(), c->oldacc_s.as<float>(), t_begin, t_end, c->w_tlist, c->wconst.as<WalkConst>(),
+      c->s_st.as<uint8_t>(), c->oldacc_s.as<float>(), t_begin, t_end, c->w_tlist, c->wconst.as<WalkConst>(), tpu, work,
       c->res_s.as<double4>(), c->nint_s.as<int32_t>(), (unsigned long long *)(c->counters.as<int>() + 32));
   return cudaGetLastError();
 }
