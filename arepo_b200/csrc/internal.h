@@ -259,7 +259,7 @@ struct gpugrav_ctx
   bool ewd_user  = false;
   // periodic PM long-range force (pm.cu): mesh size of the cuFFT plans, plans, meshes, particles
   int32_t pm_grid = 0, pm_plan_f = 0, pm_plan_b = 0;
-  gg::DevBuf pm_rho, pm_rhok, pm_pos, pm_mass, pm_acc, pm_pot, pm_tab, pm_force;
+  gg::DevBuf pm_rho, pm_rhok, pm_pos, pm_mass, pm_acc, pm_pot, pm_tab, pm_force, pm_sort;
   int32_t pm_tab_n  = 0;                      // mesh, box and Asmth that pm_tab belongs to
   double pm_tab_box = 0, pm_tab_asmth = 0;
   int group_slack = 99;                       // group cuts between cells (< 64) or key order only (GPUGRAV_GROUP_SLACK)
