@@ -10,6 +10,8 @@
 // and tested by exactly the lanes that are at it.  Every lane therefore sees
 // the same interaction sequence, in the same order, as the reference walk for
 // its target -- the per-target results are bit-identical to the reference.
+#include <type_traits>
+
 #include "internal.h"
 
 namespace gg
@@ -45,8 +47,11 @@ __device__ __forceinline__ double nearest(double x, const WalkConst &w)
 
 constexpr int kWarps  = 4;
 // Blocks per SM: 6 leave 80 registers a thread.  Even sets of 48^3 targets and zoom boxes of 240022 with
-// MULTIPLE_NODE_SOFTENING take (ms) 3.41 and 19.8 with 4, 2.35 and 19.4 with 6, 2.45 and 20.4 with 8.
-constexpr int kBlocks = 6;
+// MULTIPLE_NODE_SOFTENING take (ms) 3.41 and 19.8 with 4, 2.35 and 19.4 with 6, 2.45 and 20.4 with 8.  Walks of
+// many units per warp, whose trees lie farther away, want more warps: 128^3 targets take 19.6 with 6 and 17.8
+// with 8, 2^21 of a zoom box 75.4 and 73.9 (with 12: 17.6 and 78.9).
+constexpr int kBlocks = 6, kBlocksLarge = 8;
+constexpr int kLarge  = 8;  // units per warp of a large walk (2^19 of a zoom box: 30.0 with 6 blocks, 32.2 with 8)
 
 // The walk's tests of an internal node, src/gravity/forcetree_walk.c:196-330: opened (go on with the next
 // entry), or not -- then skipped with its subtree, and used unless it lies beyond Rcut (out).
@@ -174,8 +179,8 @@ __device__ __forceinline__ bool interact(uint32_t e, int type, const double4 sm,
 //
 // EWALD (pure periodic tree: two contributions per entry) and MNS (MULTIPLE_NODE_SOFTENING) are compiled in
 // only where used.
-template <bool EWALD, bool MNS>
-__global__ void __launch_bounds__(32 * kWarps, kBlocks) k_walk64(const double4 *__restrict__ w_sm, const double4 *__restrict__ w_cl,
+template <bool EWALD, bool MNS, int BLOCKS>
+__global__ void __launch_bounds__(32 * kWarps, BLOCKS) k_walk64(const double4 *__restrict__ w_sm, const double4 *__restrict__ w_cl,
                                                         const int2 *__restrict__ w_link, uint32_t n_entries,
                                                         const double4 *__restrict__ tpm, const uint8_t *__restrict__ tst,
                                                         const float *__restrict__ oldacc, int64_t t_begin, int64_t t_end,
@@ -280,10 +285,15 @@ cudaError_t walk64_stage(gpugrav_ctx *c, const WalkConst &wc)
       t_begin = rng[2];
       t_end   = rng[3];
     }
-  auto kern = wc.ewald ? (wc.mns ? k_walk64<true, true> : k_walk64<true, false>)
-                       : (wc.mns ? k_walk64<false, true> : k_walk64<false, false>);
   int sms = 0, per_sm = 0;
   GG_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  auto plan = [&](auto blocks) {
+    constexpr int B = decltype(blocks)::value;
+    return wc.ewald ? (wc.mns ? k_walk64<true, true, B> : k_walk64<true, false, B>)
+                    : (wc.mns ? k_walk64<false, true, B> : k_walk64<false, false, B>);
+  };
+  const bool large = (t_end - t_begin) / 32 >= (int64_t)kLarge * kBlocks * kWarps * sms;
+  auto kern        = large ? plan(std::integral_constant<int, kBlocksLarge>()) : plan(std::integral_constant<int, kBlocks>());
   GG_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarps, 0));
   // Targets per warp: as few as keep all warps running at once, 4 to 32.  The walk of a set that does not fill
   // the chip takes as long as its longest warp, and that steps on the union of its targets' entries (ms with
