@@ -122,14 +122,14 @@ __device__ __forceinline__ void direct_pair(double dx, double dy, double dz, dou
     }
 }
 
-// A warp sums kTgt targets (consecutive in key order) over the batches of 32 tiles blockIdx.y,
+// A warp sums kTgt targets (consecutive in key order) over the batches of up to 32 tiles blockIdx.y,
 // blockIdx.y + gridDim.y, ...: each lane compares one tile's box with the targets, then the warp visits the
 // tiles that can hold a pair closer than the split's reach (PM: rskip; else every tile), one source per
 // lane.  Lane sums are added over the warp at the end.
 constexpr int kDirectWarps = 4;
 template <bool PM, bool EWALD>
 __global__ void __launch_bounds__(32 * kDirectWarps) k_direct(const double4 *__restrict__ pm, const uint8_t *__restrict__ st, int64_t n,
-                                                              const TileBox *__restrict__ box, int64_t ntile,
+                                                              const TileBox *__restrict__ box, int64_t ntile, int batch,
                                                               const int32_t *__restrict__ targets, int64_t nt,
                                                               const WalkConst *__restrict__ wcp, int cut, double rskip2,
                                                               double4 *__restrict__ partial)
@@ -153,10 +153,10 @@ __global__ void __launch_bounds__(32 * kDirectWarps) k_direct(const double4 *__r
       h_i[k]      = w.soft[st[i]];
       a[k]        = make_double4(0, 0, 0, 0);
     }
-  for(int64_t b = (int64_t)blockIdx.y * 32; b < ntile; b += (int64_t)gridDim.y * 32)
+  for(int64_t b = (int64_t)blockIdx.y * batch; b < ntile; b += (int64_t)gridDim.y * batch)
     {
       unsigned near = 0;
-      if(b + lane < ntile)
+      if(lane < batch && b + lane < ntile)
         {
           near = (1u << kTgt) - 1u;
           if(PM)
@@ -449,9 +449,14 @@ cudaError_t direct_stage(gpugrav_ctx *c, const WalkConst &wc, int64_t nt, const 
   const int64_t n     = c->n;
   const int64_t ntile = (n + kTileSrc - 1) / kTileSrc, nwarp = (nt + kTgt - 1) / kTgt;
   // enough warps for several waves whatever the number of targets (at least 8 chunks, at most one
-  // batch of 32 tiles each)
+  // batch of tiles each: 32, or down to 4 while there is not a warp per SM: one target among 3271 sources took
+  // 154 us with batches of 32, four warps in all, and 89 with 4; more chunks than that cost the last sum
+  // more than they save: one among 100000 162 us with 98 chunks, 180 with 782)
+  int batch = 32;
+  while(batch > 4 && nwarp * ((ntile + batch - 1) / batch) < 148)
+    batch /= 2;
   int64_t chunks         = 148 * 128 / nwarp;
-  const int64_t nbatch   = (ntile + 31) / 32;
+  const int64_t nbatch   = (ntile + batch - 1) / batch;
   chunks                 = chunks < 8 ? 8 : chunks;
   chunks                 = chunks > nbatch ? nbatch : chunks;
   // scratch: boxes | chunk sums | sorted positions and places (before and after the sort) | sort space
@@ -477,7 +482,7 @@ cudaError_t direct_stage(gpugrav_ctx *c, const WalkConst &wc, int64_t nt, const 
     k_tile_box<<<(unsigned)((ntile + 7) / 8 < 2368 ? (ntile + 7) / 8 : 2368), 256, 0, st>>>(c->s_pm.as<double4>(), n, ntile, box);
   auto kern = wc.pm ? k_direct<true, false> : wc.ewald ? k_direct<false, true> : k_direct<false, false>;
   kern<<<dim3((unsigned)((nwarp + kDirectWarps - 1) / kDirectWarps), (unsigned)chunks), 32 * kDirectWarps, 0, st>>>(
-      c->s_pm.as<double4>(), c->s_st.as<uint8_t>(), n, box, ntile, ts2, nt, c->wconst.as<WalkConst>(), cut,
+      c->s_pm.as<double4>(), c->s_st.as<uint8_t>(), n, box, ntile, batch, ts2, nt, c->wconst.as<WalkConst>(), cut,
       reach * reach * (1.0 + 1e-9), part);
   k_direct_reduce<<<(unsigned)((nt + 255) / 256), 256, 0, st>>>(part, (int)chunks, nt, pl2, d_acc, d_pot);
   return cudaGetLastError();
