@@ -5,7 +5,7 @@
 // periodic nearest image, the relative criterion (ErrTolForceAcc x OldAcc) after
 // a Barnes-Hut pass.  Different arithmetic organisation:
 //
-//  * a warp walks the tree for a group of 32 targets that are consecutive in key
+//  * a warp walks the tree for a group of up to 64 targets that are consecutive in key
 //    order (compact in space); nodes are tested 32 at a time, one per lane,
 //    against the group's bounding box with the reference's tests made
 //    conservative for the whole group (a node is accepted only if every target of
