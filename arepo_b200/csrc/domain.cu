@@ -258,7 +258,8 @@ cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent)
   if(!g_ph_ready)
     {
       PhTable t = ph_make_table();
-      if((e = cudaMemcpyToSymbol(c_ph, &t, sizeof(t))) != cudaSuccess)
+      if((e = cudaMemcpyToSymbolAsync(c_ph, &t, sizeof(t), 0, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess ||
+         (e = cudaStreamSynchronize(c->stream)) != cudaSuccess)  // other contexts' streams read it from now on
         return e;
       g_ph_ready = true;
     }

@@ -148,7 +148,8 @@ const std::vector<double> &ewald_unit_table()
 }
 
 // tables of the context scaled to its box (fcorr / L^2, potcorr / L, forcetree_ewald.c:239-251):
-// FP64 (fx | fy | fz | pot) for the FP64 walk and the direct sum, cells of float4 corners for the FP32 walk.  `user` (may be null): the caller's already scaled tables.
+// FP64 (fx | fy | fz | pot) for the FP64 walk and the direct sum, cells of float4 corners for the FP32 walk.
+// `user` (may be null): the caller's already scaled tables.
 cudaError_t ewald_upload(gpugrav_ctx *c, const double *user)
 {
   const int m = kEwaldN + 1;
@@ -168,10 +169,12 @@ cudaError_t ewald_upload(gpugrav_ctx *c, const double *user)
   constexpr int corners = 8 * kEwaldN * kEwaldN * kEwaldN;
   GG_TRY(c->ewd.ensure(4 * total * sizeof(double)));
   GG_TRY(c->ewd32.ensure(corners * sizeof(float4)));
-  GG_TRY(cudaMemcpy(c->ewd.p, t.data(), 4 * total * sizeof(double), cudaMemcpyHostToDevice));
+  // on the context's stream, which the kernel below reads behind (a plain cudaMemcpy of pageable memory may
+  // return before its last piece has arrived, and the stream does not wait for the default one)
+  GG_TRY(cudaMemcpyAsync(c->ewd.p, t.data(), 4 * total * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   k_ewald_cells<<<(corners + 255) / 256, 256, 0, c->stream>>>(c->ewd.as<double>(), c->ewd32.as<float4>());
   GG_TRY(cudaGetLastError());
-  GG_TRY(cudaStreamSynchronize(c->stream));
+  GG_TRY(cudaStreamSynchronize(c->stream));  // `t` lives on this stack frame
   c->ewd_box  = user ? -1.0 : c->prm.box_size;
   c->ewd_user = user != nullptr;
   return cudaSuccess;

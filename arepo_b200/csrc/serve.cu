@@ -538,17 +538,19 @@ int32_t gpugrav_serve_create(gpugrav_serve **out, int32_t device, const gpugrav_
   int prev         = 0;
   cudaGetDevice(&prev);
   cudaSetDevice(device);
+  bool ok = true;
   if(device < 64 && !g_ph_srv_ready[device])
     {
       PhTable t = ph_make_table();
-      cudaMemcpyToSymbol(c_ph_srv, &t, sizeof(t));
-      g_ph_srv_ready[device] = 1;
+      ok        = cudaMemcpyToSymbolAsync(c_ph_srv, &t, sizeof(t), 0, cudaMemcpyHostToDevice, s->st) == cudaSuccess &&
+           cudaStreamSynchronize(s->st) == cudaSuccess;  // other servers' streams read it from now on
+      g_ph_srv_ready[device] = ok ? 1 : 0;
     }
   // particle pool sized by max_particles; admission also keeps the estimated device
   // footprint of the particles in flight under the budget
   s->pool_cap           = cfg->max_particles;
   s->bytes_per_particle = 700;  // pool + sorted arrays + tree + walk layout, measured upper estimate
-  bool ok = s->pos.ensure(s->pool_cap * sizeof(double4)) == cudaSuccess &&
+  ok = ok && s->pos.ensure(s->pool_cap * sizeof(double4)) == cudaSuccess &&
             s->vel.ensure(s->pool_cap * sizeof(double4)) == cudaSuccess &&
             s->acc.ensure(s->pool_cap * sizeof(double4)) == cudaSuccess &&
             s->oldacc.ensure(s->pool_cap * sizeof(float)) == cudaSuccess &&
@@ -568,7 +570,8 @@ int32_t gpugrav_serve_create(gpugrav_serve **out, int32_t device, const gpugrav_
       bc.box      = p.box_size;
       for(int i = 0; i <= p.nsofttypes; i++)
         bc.soft[i] = p.force_softening[i];
-      ok = cudaMemcpy(ctx->bconst.p, &bc, sizeof(bc), cudaMemcpyHostToDevice) == cudaSuccess;
+      ok = cudaMemcpyAsync(ctx->bconst.p, &bc, sizeof(bc), cudaMemcpyHostToDevice, s->st) == cudaSuccess &&
+           cudaStreamSynchronize(s->st) == cudaSuccess;
     }
   // working memory of a tick over a full pool, allocated once here instead of during the first
   // large ticks (one node per particle: the trees of these systems need about half that)

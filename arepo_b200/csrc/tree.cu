@@ -1107,12 +1107,14 @@ int grid_for(int64_t n, int threads)
   return (int)(b < 1 ? 1 : b);
 }
 
-cudaError_t ensure_ph(int device)
+cudaError_t ensure_ph(int device, cudaStream_t st)
 {
   if(device >= 0 && device < 64 && g_ph_tree_ready[device])
     return cudaSuccess;
   PhTable t     = ph_make_table();
-  cudaError_t e = cudaMemcpyToSymbol(c_ph_tree, &t, sizeof(t));
+  cudaError_t e = cudaMemcpyToSymbolAsync(c_ph_tree, &t, sizeof(t), 0, cudaMemcpyHostToDevice, st);
+  if(e == cudaSuccess)
+    e = cudaStreamSynchronize(st);  // other contexts' streams read it from now on
   if(e == cudaSuccess && device >= 0 && device < 64)
     g_ph_tree_ready[device] = 1;
   return e;
@@ -1122,7 +1124,7 @@ cudaError_t ensure_ph(int device)
 // The node count stays on the device (counters[kTopCount]); the host allocates for the bound.
 cudaError_t toptree_stage(gpugrav_ctx *c, int *status)
 {
-  GG_TRY(ensure_ph(c->device));
+  GG_TRY(ensure_ph(c->device, c->stream));
   const int max_top = kMaxTop;
   const int a = 1 + 2 * 4, b = (int)(c->prm.top_node_factor * c->prm.multiple_domains);
   c->ntop_cap = 2 * (a > b ? a : b) + 8;  // k_toptree's limit and one refinement more
@@ -1242,7 +1244,7 @@ cudaError_t thread_ensure(gpugrav_ctx *c)
 
 cudaError_t build_stage(gpugrav_ctx *c, int *status)
 {
-  GG_TRY(ensure_ph(c->device));
+  GG_TRY(ensure_ph(c->device, c->stream));
   const int64_t n    = c->n;
   const bool lib_top = !c->multi && c->top_dev;      // top tree built by toptree_stage: its size is on the device
   int32_t ntop       = lib_top ? c->ntop_cap : c->ntop;  // ... and this its bound until the host has read it
