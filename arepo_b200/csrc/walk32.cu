@@ -1034,6 +1034,7 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
             {
               WALK_STAT(0, queued);
               WALK_STAT(10, 1);
+              __syncwarp();  // every lane reads the entries that the others have put
               evaluate<R, PERIODIC, POT, TE, EWALD, kUnroll<TPL>>(L, E, dsum, w, tab);
               __syncwarp();
             }
