@@ -327,7 +327,7 @@ __device__ __forceinline__ void short_range(double r, const W32Const &w, TabRef,
   const double te = r * w.asmthfac_d;
   int i           = (int)te;
   if(CLAMP)
-    i = min(i, kNtab - 1);
+    i = (int)min((unsigned)i, (unsigned)kNtab - 1u);  // also the conversion of a NaN (r2 = 0, no softening)
   const double tw = te - i;
   const double4 t = w.tab64[i];
   ff              = fma(tw, t.y, t.x);
@@ -812,7 +812,9 @@ __device__ __forceinline__ void push(List<R> &L, bool keep, const V4<R> e, R h, 
   if(PERIODIC)
     {
       const float fx = fabsf((float)e.x) + bx, fy = fabsf((float)e.y) + by, fz = fabsf((float)e.z) + bz;
-      const bool all = fmaf(fx, fx, fmaf(fy, fy, fz * fz)) < w.rcut2_all;
+      // the unmasked evaluation indexes the table by r = r2 / sqrt(r2), which takes a normal r2: without
+      // softening (hn = 0) a target's own entry goes where the index is clamped
+      const bool all = fmaf(fx, fx, fmaf(fy, fy, fz * fz)) < w.rcut2_all && d2 >= 4.0e-38f;
       ka             = __ballot_sync(0xffffffffu, keep && all);
       kb             = __ballot_sync(0xffffffffu, keep && !all);
       at             = all ? L.na + __popc(ka & lt_mask) : Cap<R>::list - 1 - (L.nb + __popc(kb & lt_mask));
@@ -1533,6 +1535,7 @@ void make_w32(const WalkConst &wc, W32Const *w)
   w->half_box  = wc.half_box;
   w->rcut      = (float)wc.rcut;
   w->rcut2     = (float)wc.rcut2;
+  w->rcut2_d   = wc.rcut2;
   // margin for the rounding of the FP32 separations and the box extents (relative ~1e-6)
   w->rcut2_all = (float)(wc.rcut2 * (1.0 - 1.0 / 4096.0));
   w->asmthfac  = (float)wc.asmthfac;
@@ -1557,7 +1560,6 @@ void make_w32(const WalkConst &wc, W32Const *w)
       const double q0 = wc.tab_pot[i], q1 = (i < kNtab) ? wc.tab_pot[i + 1] : wc.tab_pot[i];
       w->tab64[i]     = make_double4(d0, d1 - d0, q0, q1 - q0);
     }
-  w->rcut2_d    = wc.rcut2;
   w->asmthfac_d = wc.asmthfac;
 }
 }  // namespace
