@@ -1534,10 +1534,14 @@ void make_w32(const WalkConst &wc, W32Const *w)
   w->box       = wc.box;
   w->half_box  = wc.half_box;
   w->rcut      = (float)wc.rcut;
-  w->rcut2     = (float)wc.rcut2;
-  w->rcut2_d   = wc.rcut2;
+  // pairs end where the table does, if that is before Rcut (RcutCells x Asmth < Rcut), as tabindex >= NTAB
+  // does in the reference; Rcut and the table's end usually agree to rounding
+  const double rtab  = wc.pm ? kNtab / wc.asmthfac : wc.rcut;
+  const double rcut2 = rtab * (1.0 + 1e-6) < wc.rcut ? rtab * rtab : wc.rcut2;
+  w->rcut2     = (float)rcut2;
+  w->rcut2_d   = rcut2;
   // margin for the rounding of the FP32 separations and the box extents (relative ~1e-6)
-  w->rcut2_all = (float)(wc.rcut2 * (1.0 - 1.0 / 4096.0));
+  w->rcut2_all = (float)(rcut2 * (1.0 - 1.0 / 4096.0));
   w->asmthfac  = (float)wc.asmthfac;
   const double finv = wc.pm ? wc.asmthinv2 : 1.0;
   w->theta2    = (float)(wc.theta * wc.theta);

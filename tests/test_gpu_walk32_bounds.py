@@ -1,6 +1,6 @@
 """Accepted parameters that leave the range the group walk's table was made for, in FP32 and in the walk's FP64
 form: particles without softening, which meet their own entry at distance zero (the reference's result for
-them is not finite; the others' and the massless ones' are)."""
+them is not finite; the others' and the massless ones' are), and an Rcut beyond the table's end."""
 import numpy as np
 import pytest
 
@@ -37,3 +37,19 @@ def test_particles_without_softening(softening, n, theta, precision, periodic, c
     # the group opens at least the nodes that each of its targets does: within the criterion's own error
     scale = np.sqrt(np.mean(np.sum(ref[ok] ** 2, axis=1)))
     assert np.sqrt(np.mean(np.sum((acc - ref)[ok] ** 2, axis=1))) <= 0.03 * scale
+
+
+@pytest.mark.parametrize("precision", [L.PREC_FP32, L.PREC_FP64_GROUP])
+@pytest.mark.parametrize("n,theta", [(2000, 0.0), (2000, 0.7), (120003, 0.0)])
+def test_rcut_beyond_the_table(n, theta, precision, cuda_lib):
+    """Pairs beyond RcutCells x Asmth contribute nothing, whatever Rcut says."""
+    rng = np.random.default_rng(n + 1)
+    pos, mass, st = rng.uniform(0, 1, (n, 3)), rng.uniform(0.5, 1.5, n) / n, np.ones(n, np.uint8)
+    acc, pot, ni = _walk(precision, pos, mass, st, rcut=1.5 * 4.5 * 0.05, theta=theta)
+    one, pot1, ni1 = _walk(precision, pos, mass, st, theta=theta)
+    # the same pairs and targets; only nodes whose cell lies between the two radii are visited besides, which
+    # changes how the sums are batched
+    scale = np.sqrt(np.mean(np.sum(one**2, axis=1)))
+    assert np.max(np.linalg.norm(acc - one, axis=1)) <= 1e-5 * scale + 1e-5 * np.max(np.linalg.norm(one, axis=1))
+    assert np.max(np.abs(pot - pot1)) <= 1e-5 * np.max(np.abs(pot1))
+    assert np.sum(ni != ni1) <= n // 100  # a pair at the table's end may fall on the other side by rounding
