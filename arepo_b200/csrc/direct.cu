@@ -275,8 +275,12 @@ __device__ __forceinline__ void direct_terms(const double4 s, double h_j, double
     {
       double tabentry = w.asmthfac * r;
       int tabindex    = (int)tabentry;
-      if(tabindex >= kNtab)
-        return;
+      if((unsigned)tabindex >= (unsigned)kNtab)
+        {
+          if(tabindex >= 0)
+            return;
+          tabindex = 0;  // r is NaN (a non-finite position): so will the sums be
+        }
       double tabweight = tabentry - tabindex;
       factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
       factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];

@@ -101,8 +101,12 @@ __device__ __forceinline__ bool interact(uint32_t e, int type, const double4 sm,
     {
       double tabentry = w.asmthfac * r;
       int tabindex    = (int)tabentry;
-      if(!(tabindex < kNtab))
-        return false;
+      if((unsigned)tabindex >= (unsigned)kNtab)
+        {
+          if(tabindex >= 0)
+            return false;
+          tabindex = 0;  // r is NaN (a non-finite mass in the node): so will the sum be
+        }
       double tabweight = tabentry - tabindex;
       factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
       factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];
