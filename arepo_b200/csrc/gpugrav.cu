@@ -785,9 +785,11 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
               we               = gg::groups_active_stage(c, nt, cap);
               c->groups_active = true;
             }
-          else if(c->groups_active)
+          else if(c->groups_active || c->group_cap != cap)
             {
-              we               = gg::groups_stage(c);  // the table of every particle again
+              // the table of every particle again, or for another number of targets per lane (which follows
+              // the parameters, and those may change on a built tree)
+              we               = gg::groups_stage(c);
               c->groups_active = false;
             }
         }

@@ -253,6 +253,7 @@ struct gpugrav_ctx
   bool slice_rng_on = false;
   int64_t w_ntargets     = 0;
   bool groups_active     = false;  // the FP32 group table describes an active list, not every particle
+  int group_cap = 0;                          // most targets per group in the table of every particle
   // Ewald correction tables (ewald.cu): FP64 and float4 copies, scaled to ewd_box (or the caller's)
   gg::DevBuf ewd, ewd32;
   double ewd_box = 0;

@@ -1606,8 +1606,8 @@ cudaError_t groups_stage(gpugrav_ctx *c)
 {
   const int64_t n = c->n;
   cudaStream_t st = c->stream;
-  const bool ewald = c->prm.periodic && !(c->prm.asmth > 0);  // the Ewald variant walks one target per lane
   const int cap    = 32 * walk32_tpl(c);
+  c->group_cap     = cap;
   GG_TRY(cudaMemsetAsync(c->g_ngroups.p, 0, sizeof(int), st));
   if(n == 0)
     return cudaSuccess;
