@@ -737,7 +737,6 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
   // active list: sorted positions in key order (targets_stage checks range and duplicates)
   const bool fp32 = c->prm.precision != GPUGRAV_PREC_FP64;  // the group walk (FP32, or its FP64 form)
   const int cap   = 32 * gg::walk32_tpl(c);                    // group size
-  int64_t a = 0, b = nout;  // this call's target slice of the active list
   c->w_tlist    = nullptr;
   c->w_ntargets = 0;
   if(active)
@@ -754,17 +753,6 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
         return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_walk_targets: target index outside [0, n)");
       if(flags & 2)
         return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_walk_targets: a particle is listed twice");
-      if(fp32)
-        {
-          const int64_t ng = (nt + cap - 1) / cap, gb = ng * c->slice / c->nslices, ge = ng * (c->slice + 1) / c->nslices;
-          a = gb * cap;
-          b = ge * cap < nt ? ge * cap : nt;
-        }
-      else
-        {
-          a = nt * c->slice / c->nslices;
-          b = nt * (c->slice + 1) / c->nslices;
-        }
     }
   CK(cudaMemsetAsync(c->counters.as<int>() + 32, 0, 8, st), "reset counters");
   CK(cudaMemsetAsync(c->counters.as<int>() + 14, 0, 4, st), "reset counters");
@@ -827,7 +815,7 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
       d_nint = ninter ? c->out_nint.as<int32_t>() : nullptr;
     }
   if(active)
-    CK(gg::targets_scatter(c, nt, a, b, d_acc, d_pot, d_nint), "scatter");
+    CK(gg::targets_scatter(c, nt, fp32, d_acc, d_pot, d_nint), "scatter");
   else
     {
       k_gather_out<<<grid_for(n, kOutTile), kOutTile, 0, st>>>(c->res_s.as<double4>(), c->nint_s.as<int32_t>(),

@@ -321,7 +321,7 @@ cudaError_t timestep_stage(gpugrav_ctx *c, const gpugrav_timestep_params *tp, in
 cudaError_t active_stage(gpugrav_ctx *c, int64_t n, const int8_t *bin, const uint8_t *d_sync, int32_t *list, int64_t *d_count);
 cudaError_t targets_stage(gpugrav_ctx *c, int64_t nt, const int32_t *d_targets, int *flags);
 cudaError_t groups_active_stage(gpugrav_ctx *c, int64_t nt, int cap);
-cudaError_t targets_scatter(gpugrav_ctx *c, int64_t nt, int64_t a, int64_t b, double *acc, double *pot, int32_t *nint);
+cudaError_t targets_scatter(gpugrav_ctx *c, int64_t nt, bool groups, double *acc, double *pot, int32_t *nint);
 cudaError_t slice_mask_stage(gpugrav_ctx *c, bool fp32);
 cudaError_t slice_cost_stage(gpugrav_ctx *c, bool fp32);
 const std::vector<double> &ewald_unit_table();

@@ -48,12 +48,21 @@ __global__ void k_target_dups(int64_t nt, const uint32_t *__restrict__ pos, int 
       atomicOr(flag, 2);
 }
 
-// results of the active list back to the caller's list order; entries outside [a, b) of the
-// active list (another rank's target slice) are written as zero
-__global__ void k_scatter_targets(int64_t nt, const uint32_t *__restrict__ tpos, const uint32_t *__restrict__ tidx, int64_t a,
-                                  int64_t b, const double4 *__restrict__ res_s, const int32_t *__restrict__ nint_s, double *__restrict__ acc, double *__restrict__ pot,
-                                  int32_t *__restrict__ nint)
+// results of the active list back to the caller's list order; entries outside this target slice
+// (another rank's) are written as zero.  The slice is a range of walk groups where the walk has them
+// (groups not null; their number is known on the device only), else of targets.
+__global__ void k_scatter_targets(int64_t nt, const uint32_t *__restrict__ tpos, const uint32_t *__restrict__ tidx, int slice,
+                                  int nslices, const int4 *__restrict__ groups, const int *__restrict__ ngroups,
+                                  const double4 *__restrict__ res_s, const int32_t *__restrict__ nint_s,
+                                  double *__restrict__ acc, double *__restrict__ pot, int32_t *__restrict__ nint)
 {
+  int64_t a = nt * slice / nslices, b = nt * (slice + 1) / nslices;
+  if(groups)
+    {
+      const int64_t ng = *ngroups, ga = ng * slice / nslices, gb = ng * (slice + 1) / nslices;
+      a = ga < ng ? groups[ga].x : nt;
+      b = gb < ng ? groups[gb].x : nt;
+    }
   for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nt; i += (int64_t)gridDim.x * blockDim.x)
     {
       const int64_t o = tidx[i], s = tpos[i];
@@ -100,10 +109,12 @@ cudaError_t targets_stage(gpugrav_ctx *c, int64_t nt, const int32_t *d_targets, 
   return cudaSuccess;
 }
 
-cudaError_t targets_scatter(gpugrav_ctx *c, int64_t nt, int64_t a, int64_t b, double *acc, double *pot, int32_t *nint)
+cudaError_t targets_scatter(gpugrav_ctx *c, int64_t nt, bool groups, double *acc, double *pot, int32_t *nint)
 {
-  k_scatter_targets<<<grid_for(nt, 256), 256, 0, c->stream>>>(nt, c->t_pos_alt.as<uint32_t>(), c->t_idx_alt.as<uint32_t>(), a, b,
-                                                             c->res_s.as<double4>(), c->nint_s.as<int32_t>(), acc, pot, nint);
+  k_scatter_targets<<<grid_for(nt, 256), 256, 0, c->stream>>>(nt, c->t_pos_alt.as<uint32_t>(), c->t_idx_alt.as<uint32_t>(), c->slice,
+                                                             c->nslices, groups ? c->g_groups.as<int4>() : nullptr,
+                                                             groups ? c->g_ngroups.as<int>() : nullptr, c->res_s.as<double4>(),
+                                                             c->nint_s.as<int32_t>(), acc, pot, nint);
   return cudaGetLastError();
 }
 }  // namespace gg
