@@ -481,6 +481,19 @@ __global__ void __launch_bounds__(kSkelThreads) k_skeleton(const gpugrav_topnode
       s_leaves            = numnodes;
     }
   __syncthreads();
+  if(!ntop_dev)
+    // a caller's top tree: particles descend by its morton_to_peano, nodes were made by the curve
+    for(int k = threadIdx.x; k < s_leaves; k += kSkelThreads)
+      {
+        const gpugrav_topnode &tn = top[nodetop[k]];
+        for(int q = 0; q < 8 && tn.daughter >= 0 && !s_bad; q++)
+          {
+            const int64_t c = suns[8 * (int64_t)k + q] - bc->n;
+            if(c < 1 || c >= s_leaves || nodetop[c] != tn.daughter + tn.morton_to_peano[q])
+              s_bad = 1;
+          }
+      }
+  __syncthreads();
   for(int l = threadIdx.x; l < nleaves; l += kSkelThreads)
     if(leafnode[l] < 0)
       s_bad = 1;
@@ -871,6 +884,9 @@ __global__ void k_children(int64_t nn, int32_t n, const int32_t *__restrict__ su
     atomicMax(deepest, d);
 }
 
+// ancestors of a node: a replayed cell's chain has up to 4096 (replay_cell's bound), below the tree's levels
+constexpr int kMaxChain = 4096 + 64;
+
 // ---- moments (force_update_node_recursive, src/gravity/forcetree.c:1266-1392) ----
 // Every thread starts at a node without node children and goes up as long as it is the last to arrive at
 // the parent, so that the whole tree takes one launch; what other threads wrote is read from L2.  One
@@ -880,12 +896,13 @@ __global__ void __launch_bounds__(128) k_moments(int64_t nn, int32_t n, const in
                                                  int32_t *__restrict__ arrived, const int32_t *__restrict__ father,
                                                  const double4 *__restrict__ pm, const uint8_t *__restrict__ st,
                                                  const double4 *__restrict__ cl, double4 *sm, uint8_t *maxsoft, int32_t *size,
-                                                 const BuildConst *__restrict__ bc, double *mpt)
+                                                 const BuildConst *__restrict__ bc, double *mpt, int *err)
 {
   int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if(k >= nn || (count[k] & 15) != 0)
+  // after a failed self-check some fathers and children are not set: the build ends without following any
+  if(k >= nn || *err || (count[k] & 15) != 0)
     return;
-  while(true)
+  for(int g = 0; g < kMaxChain; g++)
     {
       int32_t c[8];
       load_suns(suns, k, c);
@@ -976,18 +993,20 @@ __global__ void __launch_bounds__(128) k_moments(int64_t nn, int32_t n, const in
         return;
       __threadfence();
     }
+  atomicOr(err, 16);  // no root above: the build's self-check
 }
 
 // ---- threading and depth-first positions ----
 constexpr int32_t kInherit = -2;     // the link is the father's sibling
-constexpr int kMaxChain    = 4096;   // ancestors of a node (the replay of coincident points has the same bound)
 
 // per node: its children's offsets from its own position and the links among them
 __global__ void k_offsets(int64_t nn, int32_t n, const int32_t *__restrict__ suns, const int32_t *__restrict__ size,
                           const int32_t *__restrict__ father, int32_t *__restrict__ noff, int32_t *__restrict__ nsib,
                           int32_t *__restrict__ nnext, int32_t *__restrict__ poff, int32_t *__restrict__ pnext,
-                          int32_t *__restrict__ pfather)
+                          int32_t *__restrict__ pfather, const int *__restrict__ err)
 {
+  if(*err)
+    return;
   for(int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nn; k += (int64_t)gridDim.x * blockDim.x)
     {
       int32_t c[8];
@@ -1033,8 +1052,10 @@ __global__ void k_offsets(int64_t nn, int32_t n, const int32_t *__restrict__ sun
 // per node: position = offsets of the node and its ancestors; an inherited sibling is that of the nearest
 // ancestor that has one (a concurrent thread may have resolved it already: the same value)
 __global__ void k_thread(int64_t nn, int32_t n, const int32_t *__restrict__ father, const int32_t *__restrict__ noff, int32_t *nsib,
-                         int32_t *__restrict__ nnext, int32_t *__restrict__ ndfs)
+                         int32_t *__restrict__ nnext, int32_t *__restrict__ ndfs, int *err)
 {
+  if(*err)
+    return;
   for(int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nn; k += (int64_t)gridDim.x * blockDim.x)
     {
       int32_t pos = noff[k], sib = nsib[k];
@@ -1046,6 +1067,8 @@ __global__ void k_thread(int64_t nn, int32_t n, const int32_t *__restrict__ fath
             sib = __ldcg(nsib + (p - n));
           p = father[p - n];
         }
+      if(p >= 0)
+        atomicOr(err, 16);
       ndfs[k] = pos;
       nsib[k] = sib;
       if(nnext[k] == kInherit)
@@ -1213,9 +1236,10 @@ cudaError_t thread_stage(gpugrav_ctx *c)
   k_offsets<<<grid_for(nn, 256), 256, 0, st>>>(nn, (int32_t)n, c->n_suns.as<int32_t>(), c->n_size.as<int32_t>(),
                                                c->n_father.as<int32_t>(), c->n_off.as<int32_t>(), c->n_sibling.as<int32_t>(),
                                                c->n_next.as<int32_t>(), c->p_off.as<int32_t>(), c->p_next.as<int32_t>(),
-                                               c->p_father.as<int32_t>());
+                                               c->p_father.as<int32_t>(), c->counters.as<int>() + 12);
   k_thread<<<grid_for(nn, 256), 256, 0, st>>>(nn, (int32_t)n, c->n_father.as<int32_t>(), c->n_off.as<int32_t>(),
-                                              c->n_sibling.as<int32_t>(), c->n_next.as<int32_t>(), c->n_dfs.as<int32_t>());
+                                              c->n_sibling.as<int32_t>(), c->n_next.as<int32_t>(), c->n_dfs.as<int32_t>(),
+                                              c->counters.as<int>() + 12);
   k_layout<<<grid_for(ne, 256), 256, 0, st>>>(n, nn, c->s_pm.as<double4>(), c->s_st.as<uint8_t>(), c->p_off.as<int32_t>(),
                                                c->p_father.as<int32_t>(), c->p_next.as<int32_t>(), c->n_sibling.as<int32_t>(),
                                                c->n_sm.as<double4>(), c->n_cl.as<double4>(), c->n_maxsoft.as<uint8_t>(),
@@ -1441,7 +1465,7 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
                                                           c->n_arrived.as<int32_t>(), c->n_father.as<int32_t>(), c->s_pm.as<double4>(),
                                                           c->s_st.as<uint8_t>(), c->n_cl.as<double4>(), c->n_sm.as<double4>(),
                                                           c->n_maxsoft.as<uint8_t>(), c->n_size.as<int32_t>(),
-                                                          c->bconst.as<BuildConst>(), mns ? c->n_mpt.as<double>() : nullptr);
+                                                          c->bconst.as<BuildConst>(), mns ? c->n_mpt.as<double>() : nullptr, a.err);
   launches += 2;
   c->mark("b5 moments");
   // 6. threading and the layout of the FP64 walk; the group walk needs neither (several systems are
