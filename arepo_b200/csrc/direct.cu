@@ -275,12 +275,10 @@ __device__ __forceinline__ void direct_terms(const double4 s, double h_j, double
     {
       double tabentry = w.asmthfac * r;
       int tabindex    = (int)tabentry;
-      if((unsigned)tabindex >= (unsigned)kNtab)
-        {
-          if(tabindex >= 0)
-            return;
-          tabindex = 0;  // r is NaN (a non-finite position): so will the sums be
-        }
+      if(tabindex >= kNtab)
+        return;
+      static_assert((kNtab & (kNtab + 1)) == 0, "all bits set");
+      tabindex &= kNtab;  // INT_MIN where r is NaN (a non-finite position): entry 0, and the sums will be NaN
       double tabweight = tabentry - tabindex;
       factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
       factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];

@@ -101,12 +101,11 @@ __device__ __forceinline__ bool interact(uint32_t e, int type, const double4 sm,
     {
       double tabentry = w.asmthfac * r;
       int tabindex    = (int)tabentry;
-      if((unsigned)tabindex >= (unsigned)kNtab)
-        {
-          if(tabindex >= 0)
-            return false;
-          tabindex = 0;  // r is NaN (a non-finite mass in the node): so will the sum be
-        }
+      if(!(tabindex < kNtab))
+        return false;
+      // INT_MIN where r is NaN (a non-finite mass in the node): entry 0, and the sum will be NaN
+      static_assert((kNtab & (kNtab + 1)) == 0, "all bits set");
+      tabindex &= kNtab;
       double tabweight = tabentry - tabindex;
       factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
       factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];
