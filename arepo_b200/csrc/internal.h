@@ -351,6 +351,12 @@ inline int walk32_tpl(const gpugrav_ctx *c)
     return 1;
   return (c->walk32_tpl == 2 || !c->multi) ? 2 : 1;
 }
+// the built tree is deeper by `more` levels than an even set's of as many particles would be
+inline bool deep_tree(const gpugrav_ctx *c, int more)
+{
+  const int levels = c->max_depth - more;
+  return levels > 20 || (levels > 0 && (int64_t)1 << (3 * levels) >= c->n);
+}
 // GPUGRAV_OK or GPUGRAV_ERR_INVALID: ABI version, softening table (finite, >= 0, zero end entry),
 // box size, TreePM split (asmth, rcut, rcut_cells > 0 unless asmth == 0), tolerances, flags
 int validate_params(const gpugrav_params *p);

@@ -1933,9 +1933,7 @@ cudaError_t walk32_order(gpugrav_ctx *c, const WalkConst &wc)
   // 16.8 ms in this one).
   const int64_t targets = (c->w_ntargets > 0 ? c->w_ntargets : c->n) / c->nslices;
   const size_t cap      = c->g_groups.cap / sizeof(int4);
-  const int levels      = c->max_depth - 4;
-  const bool deep       = levels > 20 || (levels > 0 && (int64_t)1 << (3 * levels) >= c->n);
-  if(wc.bh || !deep || targets / (32 * walk32_tpl(c)) <= (int64_t)c->w32_blocks * (c->w32_threads / 32))
+  if(wc.bh || !deep_tree(c, 4) || targets / (32 * walk32_tpl(c)) <= (int64_t)c->w32_blocks * (c->w32_threads / 32))
     return cudaSuccess;
   if(c->g_order.ensure(sizeof(GroupOrder) + cap * (sizeof(int) + 1)) != cudaSuccess)
     cudaGetLastError();  // no room: key order

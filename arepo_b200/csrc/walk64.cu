@@ -37,64 +37,61 @@ namespace
 #define SF16 9.6
 #define SF17 (-2.133333333333)
 
+// GRAVITY_NEAREST_X, src/main/allvars.h:602-608: x - box or x + box beyond half a box; a select, no branches
+template <bool PER>
 __device__ __forceinline__ double nearest(double x, const WalkConst &w)
 {
-  // GRAVITY_NEAREST_X, src/main/allvars.h:602-608; selects, no branches
-  const double hb = w.periodic ? w.half_box : 1e300, lo = x - w.box, hi = x + w.box;
-  const bool a = x > hb, b = x < -hb;
-  return a ? lo : b ? hi : x;
+  return PER ? x - (fabs(x) > w.half_box ? copysign(w.box, x) : 0.0) : x;
 }
 
 constexpr int kWarps  = 4;
-// Blocks per SM: 6 leave 80 registers a thread.  Even sets of 48^3 targets and zoom boxes of 240022 with
-// MULTIPLE_NODE_SOFTENING take (ms) 3.41 and 19.8 with 4, 2.35 and 19.4 with 6, 2.45 and 20.4 with 8.  Walks of
-// many units per warp, whose trees lie farther away, want more warps: 128^3 targets take 19.6 with 6 and 17.8
-// with 8, 2^21 of a zoom box 75.4 and 73.9 (with 12: 17.6 and 78.9).
-constexpr int kBlocks = 6, kBlocksLarge = 8;
-constexpr int kLarge  = 8;  // units per warp of a large walk (2^19 of a zoom box: 30.0 with 6 blocks, 32.2 with 8)
+// Blocks per SM: 6 leave 80 registers a thread, 8 hide more of the loads' latency, 10 hold more warps at once
+// (walk64_stage chooses).  Walk (ms) with 6 / 8 / 10: even 48^3 0.99 / 1.11 / 1.37, 53^3 1.75 / 1.34 / 1.70, 57^3
+// 2.05 / 2.13 / 1.92, 61^3 2.39 / 2.48 / 2.66, 80^3 5.77 / 5.28 / 5.59, 128^3 19.5 / 17.9 / 18.5; zoom box 150000
+// 17.5 / 19.5 / 21.3, 240022 22.4 / 24.9 / 27.2, 2^19 29.3 / 32.7 / 34.9, 2^21 71.5 / 71.4 / 76.3, 2^24 (tolerance 2e-5)
+// - / 3868 / -; Plummer 150000 5.7 / 6.1 / 6.2, 2^20 17.5 / 17.2 / 17.3.
+constexpr int kBlocks = 6, kBlocksMore = 8, kBlocksMost = 10;
+constexpr int kLarge  = 8;  // units per warp from which the walk of a clustered set takes kBlocksMore
 
 // The walk's tests of an internal node, src/gravity/forcetree_walk.c:196-330: opened (go on with the next
 // entry), or not -- then skipped with its subtree, and used unless it lies beyond Rcut (out).
-template <bool MNS>
-__device__ __forceinline__ void test_node(const double4 sm, const double4 cl, int type_fl, double pos_x, double pos_y, double pos_z,
-                                          double aold, double h_i, const WalkConst &w, bool &open, bool &out)
+template <bool MNS, bool PER>
+__device__ __forceinline__ void test_node(double mass, const double4 cl, int type_fl, double r2, double pos_x, double pos_y,
+                                          double pos_z, double aold, double h_i, const WalkConst &w, bool &open, bool &out)
 {
   // No short-circuit evaluation: the comparisons do not depend on one another and run side by side; a branch
-  // for each, taken by some lanes, made the test most of the walk: 32^3 targets took 1.28 ms, 0.95 ms
-  // without; a zoom box of 240022 30.5 ms, 19.4 ms without.
-  const double mass = sm.w;
-  const double dx = nearest(sm.x - pos_x, w), dy = nearest(sm.y - pos_y, w), dz = nearest(sm.z - pos_z, w);
-  const double cx = fabs(nearest(cl.x - pos_x, w)), cy = fabs(nearest(cl.y - pos_y, w)), cz = fabs(nearest(cl.z - pos_z, w));
-  const double r2  = dx * dx + dy * dy + dz * dz;
+  // for each, taken by some lanes, made the test most of the walk of sets that fill the chip about once
+  // (32^3 targets 1.28 ms, 0.87 without; a zoom box of 240022 32 ms, 22 without).
   const double len = cl.w, len2 = len * len;
-  const double eff_dist = w.rcut + 0.5 * len;
-  out = (w.pm != 0) & (r2 > w.rcut2) & ((cx > eff_dist) | (cy > eff_dist) | (cz > eff_dist));
+  const bool beyond = PER && (w.pm != 0) & (r2 > w.rcut2);
   if(w.bh)
     open = len2 > r2 * w.theta * w.theta;
   else
-    {
-      // ACTIVATE_MINIMUM_OPENING_ANGLE adds a minimum angle to the mass test (forcetree_walk.c:266-271)
-      const double in = 0.60 * len;
-      open = (len2 > r2 * (1.2 * 1.2)) | ((mass * len2 > r2 * r2 * aold) & ((w.minangle == 0) | (len2 > r2 * (0.4 * 0.4)))) |
-             ((cx < in) & (cy < in) & (cz < in));
-    }
+    // ACTIVATE_MINIMUM_OPENING_ANGLE adds a minimum angle to the mass test (forcetree_walk.c:266-271)
+    open = (len2 > r2 * (1.2 * 1.2)) | ((mass * len2 > r2 * r2 * aold) & ((w.minangle == 0) | (len2 > r2 * (0.4 * 0.4))));
   if(!MNS)
     {
       const double h_j = w.soft[type_fl & 0xff];
       open             = open | ((h_j > h_i) & (r2 < h_j * h_j));
     }
-  open = open && !out;
+  const double cx = fabs(nearest<PER>(cl.x - pos_x, w)), cy = fabs(nearest<PER>(cl.y - pos_y, w)),
+               cz = fabs(nearest<PER>(cl.z - pos_z, w));
+  if(PER)
+    {
+      const double eff_dist = w.rcut + 0.5 * len;
+      out                   = beyond & ((cx > eff_dist) | (cy > eff_dist) | (cz > eff_dist));
+    }
+  const double in = 0.60 * len;
+  open            = (open | (!w.bh & (cx < in) & (cy < in) & (cz < in))) & !out;
 }
 
-// One contribution of a walk entry (sm: centre of mass and mass, type_fl: softening type and node flag) to a
+// One contribution of a walk entry (at dx, dy, dz from the target; type_fl: softening type and node flag) to a
 // target, src/gravity/forcetree_walk.c:363-488, added with add(x, y, z, potential); type >= 0: the node's
 // mass of that softening type (MULTIPLE_NODE_SOFTENING, forcetree_walk.c:382-401).  False: beyond the table.
 template <bool EWALD, bool MNS, class Add>
-__device__ __forceinline__ bool interact(uint32_t e, int type, const double4 sm, int type_fl, double pos_x, double pos_y, double pos_z,
+__device__ __forceinline__ bool interact(uint32_t e, int type, double mass, int type_fl, double dx, double dy, double dz, double r2,
                                          double h_i, const WalkConst &w, Add add)
 {
-  const double dx = nearest(sm.x - pos_x, w), dy = nearest(sm.y - pos_y, w), dz = nearest(sm.z - pos_z, w);
-  const double r2     = dx * dx + dy * dy + dz * dz;
   double r            = sqrt(r2);
   double factor_force = 0, factor_pot = 0;
   if(w.pm)
@@ -110,8 +107,7 @@ __device__ __forceinline__ bool interact(uint32_t e, int type, const double4 sm,
       factor_force     = (1.0 - tabweight) * w.tab_force[tabindex] + tabweight * w.tab_force[tabindex + 1];
       factor_pot       = (1.0 - tabweight) * w.tab_pot[tabindex] + tabweight * w.tab_pot[tabindex + 1];
     }
-  double mass      = sm.w;
-  double h_j       = w.soft[type_fl & 0xff];
+  double h_j = w.soft[type_fl & 0xff];
   if(MNS && type >= 0)
     {
       mass = w.w_mpt[(int64_t)e * w.nsoft + type];
@@ -180,9 +176,10 @@ __device__ __forceinline__ bool interact(uint32_t e, int type, const double4 sm,
 // were 1.2 times faster in a zoom box but 1.5 times slower in an even set of 2^18, whose warps the queues'
 // shared memory kept off the SM.
 //
-// EWALD (pure periodic tree: two contributions per entry) and MNS (MULTIPLE_NODE_SOFTENING) are compiled in
-// only where used.
-template <bool EWALD, bool MNS, int BLOCKS>
+// EWALD (pure periodic tree: two contributions per entry), MNS (MULTIPLE_NODE_SOFTENING) and PER (nearest images)
+// are compiled in only where used: an isolated sphere of 2^20 particles took 23.6 ms with the selects of PER and
+// the separations formed in the test and again in the interaction, 17.2 without.
+template <bool EWALD, bool MNS, bool PER, int BLOCKS>
 __global__ void __launch_bounds__(32 * kWarps, BLOCKS) k_walk64(const double4 *__restrict__ w_sm, const double4 *__restrict__ w_cl,
                                                         const int2 *__restrict__ w_link, uint32_t n_entries,
                                                         const double4 *__restrict__ tpm, const uint8_t *__restrict__ tst,
@@ -235,9 +232,11 @@ __global__ void __launch_bounds__(32 * kWarps, BLOCKS) k_walk64(const double4 *_
           const int2 link  = w_link[i];
           const double4 sm = w_sm[i], cl = w_cl[i];
           const bool node  = (link.y & kNodeFlag) != 0;
+          const double dx = nearest<PER>(sm.x - pos_x, w), dy = nearest<PER>(sm.y - pos_y, w), dz = nearest<PER>(sm.z - pos_z, w);
+          const double r2 = dx * dx + dy * dy + dz * dz;
           bool open = false, out = false;
           if(node)
-            test_node<MNS>(sm, cl, link.y, pos_x, pos_y, pos_z, aold, h_i, w, open, out);
+            test_node<MNS, PER>(sm.w, cl, link.y, r2, pos_x, pos_y, pos_z, aold, h_i, w, open, out);
           const bool here = next == i, take = here && !open && !out && sm.w != 0;
           if(here)
             next = node && !open ? (uint32_t)link.x : i + 1;
@@ -248,9 +247,9 @@ __global__ void __launch_bounds__(32 * kWarps, BLOCKS) k_walk64(const double4 *_
               bool did = false;
               if(MNS && split)
                 for(int t = 0; t < w.nsoft; t++)
-                  did = interact<EWALD, MNS>(i, t, sm, link.y, pos_x, pos_y, pos_z, h_i, w, add_own);
+                  did = interact<EWALD, MNS>(i, t, sm.w, link.y, dx, dy, dz, r2, h_i, w, add_own);
               else
-                did = interact<EWALD, false>(i, -1, sm, link.y, pos_x, pos_y, pos_z, h_i, w, add_own);
+                did = interact<EWALD, false>(i, -1, sm.w, link.y, dx, dy, dz, r2, h_i, w, add_own);
               ninteractions += did ? 1 : 0;
             }
         }
@@ -292,11 +291,26 @@ cudaError_t walk64_stage(gpugrav_ctx *c, const WalkConst &wc)
   GG_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
   auto plan = [&](auto blocks) {
     constexpr int B = decltype(blocks)::value;
-    return wc.ewald ? (wc.mns ? k_walk64<true, true, B> : k_walk64<true, false, B>)
-                    : (wc.mns ? k_walk64<false, true, B> : k_walk64<false, false, B>);
+    return wc.ewald      ? (wc.mns ? k_walk64<true, true, true, B> : k_walk64<true, false, true, B>)
+           : wc.periodic ? (wc.mns ? k_walk64<false, true, true, B> : k_walk64<false, false, true, B>)
+                         : (wc.mns ? k_walk64<false, true, false, B> : k_walk64<false, false, false, B>);
   };
-  const bool large = (t_end - t_begin) / 32 >= (int64_t)kLarge * kBlocks * kWarps * sms;
-  auto kern        = large ? plan(std::integral_constant<int, kBlocksLarge>()) : plan(std::integral_constant<int, kBlocks>());
+  // The warps of an even set all take as long: the fewest blocks that need the fewest rounds of warps, and
+  // kBlocksMore beyond two rounds.  A clustered set's differ (its tree is deeper; displaced grids and random sets
+  // of 10^5 to 10^6 are deeper than even by up to 5 levels, zoom boxes and spheres by 8 and more), and the long
+  // ones want the registers.
+  const int64_t warps = (t_end - t_begin + 31) / 32, per_block = (int64_t)kWarps * sms;
+  auto rounds         = [&](int b) { return (warps + b * per_block - 1) / (b * per_block); };
+  int blocks          = kBlocks;
+  if(deep_tree(c, 6))
+    blocks = warps >= kLarge * kBlocks * per_block ? kBlocksMore : kBlocks;
+  else if(rounds(kBlocks) > 2 || rounds(kBlocksMore) < rounds(kBlocks))
+    blocks = kBlocksMore;
+  else if(rounds(kBlocksMost) < rounds(kBlocks))
+    blocks = kBlocksMost;
+  auto kern = blocks == kBlocks       ? plan(std::integral_constant<int, kBlocks>())
+              : blocks == kBlocksMore ? plan(std::integral_constant<int, kBlocksMore>())
+                                      : plan(std::integral_constant<int, kBlocksMost>());
   GG_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarps, 0));
   // Targets per warp: as few as keep all warps running at once, 4 to 32.  The walk of a set that does not fill
   // the chip takes as long as its longest warp, and that steps on the union of its targets' entries (ms with
