@@ -251,11 +251,11 @@ __global__ void k_map_targets(const int64_t *__restrict__ tg, int64_t nt, const 
 //
 // Only the additions have to follow each other; the terms (a square root, divisions, the table) do not.
 // A warp takes T targets and 32 sources at a time: every lane computes the terms of its source for the T
-// targets into shared memory, then 4 T lanes add them, one sum component each, in source order.
-template <bool EWALD>
+// targets into shared memory, then 4 T lanes add them, one sum component each, in source order.  Sets that fill
+// the chip with one thread per target have no need of that (k_gravity_direct_wide).
+template <bool EWALD, int P>  // P: component pitch of `out`
 __device__ __forceinline__ void direct_terms(const double4 s, double h_j, double4 me, double h_i, const WalkConst &w, double *__restrict__ out)
 {
-  constexpr int P = 33;  // component pitch of `out`
 #pragma unroll
   for(int c = 0; c < (EWALD ? 8 : 4); c++)
     out[c * P] = 0.0;
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_gravity_direct(const double 
           const double h_j = w.soft[ty < w.nsoft ? ty : 0];
 #pragma unroll
           for(int t = 0; t < T; t++)
-            direct_terms<EWALD>(s, h_j, me[t], h_i[t], w, &term[warp][t][0][lane]);
+            direct_terms<EWALD, 33>(s, h_j, me[t], h_i[t], w, &term[warp][t][0][lane]);
         }
       __syncwarp();
       const int cnt = n - jb < 32 ? (int)(n - jb) : 32;
@@ -419,6 +419,63 @@ __global__ void __launch_bounds__(32 * kDirWarps) k_gravity_direct(const double 
     }
 }
 
+// The same sums, one thread per target over source tiles in shared memory: each thread adds its terms as it
+// computes them.
+constexpr int kWide = 128;
+constexpr int64_t kDirWide = 45000, kDirWideEwald = 110000;  // targets from which it is the faster one
+template <bool EWALD>
+__global__ void __launch_bounds__(kWide) k_gravity_direct_wide(const double *__restrict__ pos, const double *__restrict__ mass,
+                                                               const uint8_t *__restrict__ st, int64_t n,
+                                                               const WalkConst *__restrict__ wcp, double *__restrict__ acc,
+                                                               double *__restrict__ pot, int *__restrict__ flag)
+{
+  __shared__ WalkConst w;
+  __shared__ double4 src[kWide];
+  __shared__ double hsrc[kWide];
+  for(int t = threadIdx.x; t < (int)(sizeof(WalkConst) / 4); t += blockDim.x)
+    ((int *)&w)[t] = ((const int *)wcp)[t];
+  __syncthreads();
+  const int64_t i = (int64_t)blockIdx.x * kWide + threadIdx.x, k = i < n ? i : n - 1;  // past the end: the last target
+  const int ty    = st[k];
+  if(ty >= w.nsoft)
+    atomicOr(flag, 1);
+  const double4 me = make_double4(pos[3 * k + 0], pos[3 * k + 1], pos[3 * k + 2], 0.0);
+  const double h_i = w.soft[ty < w.nsoft ? ty : 0];
+  double sum[4]    = {0, 0, 0, 0};
+  for(int64_t jb = 0; jb < n; jb += kWide)
+    {
+      const int64_t j = jb + threadIdx.x;
+      __syncthreads();
+      if(j < n)
+        {
+          const int tj      = st[j];
+          src[threadIdx.x]  = make_double4(pos[3 * j + 0], pos[3 * j + 1], pos[3 * j + 2], mass[j]);
+          hsrc[threadIdx.x] = w.soft[tj < w.nsoft ? tj : 0];
+        }
+      __syncthreads();
+      const int cnt = n - jb < kWide ? (int)(n - jb) : kWide;
+      for(int q = 0; q < cnt; q++)
+        {
+          double term[EWALD ? 8 : 4];
+          direct_terms<EWALD, 1>(src[q], hsrc[q], me, h_i, w, term);
+#pragma unroll
+          for(int c = 0; c < 4; c++)
+            {
+              sum[c] += term[c];
+              if(EWALD)
+                sum[c] += term[4 + c];
+            }
+        }
+    }
+  if(i < n)
+    {
+      for(int c = 0; c < 3; c++)
+        acc[3 * i + c] = sum[c];
+      if(pot)
+        pot[i] = sum[3];
+    }
+}
+
 __global__ void k_fill_i32(int32_t *__restrict__ a, int64_t n, int32_t v)
 {
   for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -429,14 +486,27 @@ __global__ void k_fill_i32(int32_t *__restrict__ a, int64_t n, int32_t v)
 cudaError_t gravity_direct_stage(gpugrav_ctx *c, int64_t n, const double *d_pos, const double *d_mass, const uint8_t *d_st,
                                  double *d_acc, double *d_pot, int32_t *d_nint, int *d_flag)
 {
-  // one target per warp while the chip has room for more warps than targets, else 4
+  // One target per warp while the chip has room for more warps than targets, then 4, and one per thread once
+  // that fills it.  Kernel (ms) with 1 / 4 / one per thread: isolated 3000 0.13 / 0.15 / 0.59, 8000 0.67 / 0.44 /
+  // 1.56, 16384 2.6 / 1.8 / 3.2, 40000 15.2 / 8.5 / 8.8, 49152 22.9 / 13.0 / 10.9, 131072 158 / 83 / 54; TreePM 40000
+  // 17.4 / 12.9 / 15.9, 49152 26.2 / 19.6 / 19.6, 131072 184 / 128 / 84; Ewald, whose interpolation outweighs the
+  // additions, 32768 103 / 103 / 102, 65536 - / 412 / 441, 131072 - / 1642 / 1568.
   const bool ewald = c->prm.periodic && !(c->prm.asmth > 0);
-  const int T      = n <= kDirOneTarget ? 1 : 4;
-  auto kern        = T == 1 ? (ewald ? k_gravity_direct<1, true> : k_gravity_direct<1, false>)
-                            : (ewald ? k_gravity_direct<4, true> : k_gravity_direct<4, false>);
-  const int64_t per = (int64_t)kDirWarps * T;
-  kern<<<(unsigned)((n + per - 1) / per), 32 * kDirWarps, 0, c->stream>>>(d_pos, d_mass, d_st, n, c->wconst.as<WalkConst>(), d_acc, d_pot,
-                                                                        d_flag);
+  if(n > (ewald ? kDirWideEwald : kDirWide))
+    {
+      auto kern = ewald ? k_gravity_direct_wide<true> : k_gravity_direct_wide<false>;
+      kern<<<(unsigned)((n + kWide - 1) / kWide), kWide, 0, c->stream>>>(d_pos, d_mass, d_st, n, c->wconst.as<WalkConst>(), d_acc,
+                                                                        d_pot, d_flag);
+    }
+  else
+    {
+      const int T       = n <= kDirOneTarget ? 1 : 4;
+      auto kern         = T == 1 ? (ewald ? k_gravity_direct<1, true> : k_gravity_direct<1, false>)
+                                 : (ewald ? k_gravity_direct<4, true> : k_gravity_direct<4, false>);
+      const int64_t per = (int64_t)kDirWarps * T;
+      kern<<<(unsigned)((n + per - 1) / per), 32 * kDirWarps, 0, c->stream>>>(d_pos, d_mass, d_st, n, c->wconst.as<WalkConst>(), d_acc,
+                                                                            d_pot, d_flag);
+    }
   if(d_nint)
     k_fill_i32<<<(unsigned)((n + 255) / 256 < 2368 ? (n + 255) / 256 : 2368), 256, 0, c->stream>>>(d_nint, n, (int32_t)n);
   return cudaGetLastError();
