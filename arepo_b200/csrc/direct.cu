@@ -521,11 +521,16 @@ cudaError_t direct_stage(gpugrav_ctx *c, const WalkConst &wc, int64_t nt, const 
   const int64_t n     = c->n;
   const int64_t ntile = (n + kTileSrc - 1) / kTileSrc, nwarp = (nt + kTgt - 1) / kTgt;
   // enough warps for several waves whatever the number of targets (at least 8 chunks, at most one
-  // batch of tiles each: 32, or down to 4 while there is not a warp per SM: one target among 3271 sources took
-  // 154 us with batches of 32, four warps in all, and 89 with 4; more chunks than that cost the last sum
-  // more than they save: one among 100000 162 us with 98 chunks, 180 with 782)
-  int batch = 32;
-  while(batch > 4 && nwarp * ((ntile + batch - 1) / batch) < 148)
+  // batch of tiles each: 32, or down to 4 while there is not a warp per SM, or not eight and few chunks: one
+  // target among 3271 sources took 154 us with batches of 32, four warps in all, and 89 with 4; 500 among 2000
+  // took 155 with 32 and 93 with 4.  More chunks than that cost the last sum more than they save: one among
+  // 100000 162 us with 98 chunks, 180 with 782)
+  int batch       = 32;
+  auto more_warps = [&]() {
+    const int64_t nb = (ntile + batch - 1) / batch, warps = nwarp * nb;
+    return warps < 148 || (warps < 8 * 148 && nb < 64);
+  };
+  while(batch > 4 && more_warps())
     batch /= 2;
   int64_t chunks         = 148 * 128 / nwarp;
   const int64_t nbatch   = (ntile + batch - 1) / batch;
