@@ -57,8 +57,10 @@ __device__ __forceinline__ void cic_axis(double x, double f, int n, int &c0, int
 // of bricks of 16^3 cells (a sort of 15 bits at 512^3), so that those running together share the mesh's
 // lines; results are written in that order and read back by the caller's.  With 2^24 particles on 512^3 the
 // call went from 9.36 to 7.63 ms for a zoom box and from 11.3 to 7.6 ms for an even set.  The sort and the
-// two permutations cost 80 us per 2^20 particles: on meshes that fit in L2, or with few particles per brick
-// (256^3: 2^22 particles of a zoom box 1.63 -> 1.92 ms, 2^24 4.54 -> 3.92 ms), the caller's order stays.
+// two permutations cost 80 us per 2^20 particles: on meshes that fit in L2, or with few particles per brick, the
+// caller's order stays.  Caller's / brick order (ms), zoom box and even set: 256^3 with 2^22 particles 1.64 / 1.90 and
+// 1.66 / 1.28, 2^23 2.6 either way for the zoom box; 512^3 with 2^20 5.43 / 5.59 and 5.57 / 5.08, 2^21 5.69 / 5.47 and
+// 5.93 / 5.05, 2^22 6.20 / 5.68 and 6.70 / 5.34.  The line below is 256^3's; on larger meshes it could lie at 2^21.
 constexpr int kBrick             = 4;    // log2 of a brick's side in cells
 constexpr int kSortMesh          = 256;  // from 128 MB of potential, which is the L2's size
 constexpr int64_t kSortParticles = 1 << 23;
@@ -266,6 +268,12 @@ __global__ void k_pm_fd4(int n, double fac, const double *__restrict__ phi, doub
         }
     }
 }
+
+// Call (ms) with the records / component by component on 512^3: 1000 and 2^16 particles 5.20 / 5.07, 2^20 of a zoom
+// box 5.46 / 5.45, of an even set 5.59 / 5.71, 2^22 6.25 / 6.57 and 6.75 / 7.50; on 384^3 and smaller meshes the records
+// are never behind (1000 particles 3.00 / 3.01, on 256^3 0.69 / 0.77).
+constexpr int kFewMesh  = 384;
+constexpr int kFewShare = 128;  // few: less than one particle to so many mesh points
 
 // CIC readout of the records: accelerations and (pot not null) potentials scaled by `scale`
 __global__ void __launch_bounds__(256) k_pm_read4(int64_t np, const double *__restrict__ pos, int n, double f, const double4 *__restrict__ mesh,
@@ -528,10 +536,12 @@ cudaError_t pm_stage(gpugrav_ctx *c, int pmgrid, int64_t np, const double *pos, 
       k_pm_out<<<blocks_for(np), kOutTile, 0, st>>>(np, s_res, iperm, acc, pot);
       return cudaGetLastError();
     }
-  // the records take 32 bytes per mesh point; where they would take more than a quarter of the device's free
-  // memory, one component after the other in the complex buffer, which is free after the inverse transform
-  bool records = c->pm_force.cap >= N3 * sizeof(double4);
-  if(!records)
+  // The records take 32 bytes per mesh point, written once.  Few particles on a large mesh (kFewMesh, kFewShare) do
+  // not pay for that, and where the records would take more than a quarter of the device's free memory there is
+  // no room: then one component after the other in the complex buffer, which is free after the inverse transform.
+  const bool few = n > kFewMesh && np * kFewShare < N3;
+  bool records   = !few && c->pm_force.cap >= N3 * sizeof(double4);
+  if(!few && !records)
     {
       size_t free_b = 0, total_b = 0;
       records = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && N3 * sizeof(double4) <= free_b / 4 &&
