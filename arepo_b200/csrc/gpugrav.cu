@@ -31,6 +31,57 @@ void gpugrav_ctx::mark(const char *what)
   prof_t = t;
 }
 
+// ---- buffers that any allocation may take back ----
+// A PM call leaves gigabytes of working space for the next one.  Between calls those buffers stand here, and an
+// allocation of any context that finds no memory frees those of its device and tries again.  A buffer is listed
+// only while no work that uses it is in flight.
+namespace
+{
+struct Spare
+{
+  gg::DevBuf *buf;
+  int device;
+};
+std::mutex g_spare_lock;
+std::vector<Spare> g_spare;
+
+bool reclaim_spare()
+{
+  int device = -1;
+  if(cudaGetDevice(&device) != cudaSuccess)
+    return false;
+  std::lock_guard<std::mutex> lock(g_spare_lock);
+  bool any  = false;
+  size_t at = 0;
+  for(const Spare &s : g_spare)
+    if(s.device == device)
+      {
+        any = any || s.buf->p != nullptr;
+        s.buf->release();
+      }
+    else
+      g_spare[at++] = s;
+  g_spare.resize(at);
+  return any;
+}
+}  // namespace
+
+void gg::spare_offer(gg::DevBuf *b, int device)
+{
+  std::lock_guard<std::mutex> lock(g_spare_lock);
+  g_spare.push_back(Spare{b, device});
+}
+
+void gg::spare_take(gg::DevBuf *b)
+{
+  std::lock_guard<std::mutex> lock(g_spare_lock);
+  size_t at = 0;
+  for(const Spare &s : g_spare)
+    if(s.buf != b)
+      g_spare[at++] = s;
+  g_spare.resize(at);
+}
+
 cudaError_t gg::DevBuf::ensure(size_t bytes)
 {
   if(bytes <= cap && p)
@@ -47,6 +98,11 @@ cudaError_t gg::DevBuf::ensure(size_t bytes)
     want += want / 4;
   want        = (want + 255) & ~(size_t)255;
   cudaError_t e = cudaMalloc(&p, want);
+  if(e == cudaErrorMemoryAllocation && reclaim_spare())
+    {
+      cudaGetLastError();
+      e = cudaMalloc(&p, want);
+    }
   if(e != cudaSuccess)
     {
       p = nullptr;
@@ -580,6 +636,8 @@ int32_t gpugrav_pm_periodic(gpugrav_ctx *c, int32_t pmgrid, int64_t n, const dou
     }
   cudaEventRecord(c->ev[18], st);
   int fft_status = 0;
+  gg::spare_take(&c->pm_force);
+  gg::spare_take(&c->pm_sort);
   CK(gg::pm_stage(c, pmgrid, n, d_pos, d_mass, d_acc, d_pot, &fft_status), "pm");
   cudaEventRecord(c->ev[19], st);
   if(fft_status != 0)
@@ -596,6 +654,8 @@ int32_t gpugrav_pm_periodic(gpugrav_ctx *c, int32_t pmgrid, int64_t n, const dou
   int bad = 0;
   CK(cudaMemcpyAsync(&bad, c->counters.as<int>() + 15, 4, cudaMemcpyDeviceToHost, st), "pm flags");
   CK(cudaStreamSynchronize(st), "pm");
+  gg::spare_offer(&c->pm_force, c->device);
+  gg::spare_offer(&c->pm_sort, c->device);
   c->timings.pm_ms = elapsed(c->ev[18], c->ev[19]);
   if(bad)
     return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_pm_periodic: non-finite position or position far outside the box");

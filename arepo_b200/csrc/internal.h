@@ -301,6 +301,9 @@ __device__ __forceinline__ int common_depth(uint64_t ax, uint64_t ay, uint64_t a
 namespace gg
 {
 // launchers implemented in the .cu files; each returns cudaGetLastError() of its launches
+// buffers that any allocation may take back between calls (gpugrav.cu)
+void spare_offer(DevBuf *b, int device);
+void spare_take(DevBuf *b);
 cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent);
 cudaError_t sort_lead_stage(gpugrav_ctx *c, int64_t n, int *flags);
 cudaError_t sort_full_stage(gpugrav_ctx *c, int64_t n, int bits);

@@ -579,6 +579,8 @@ void pm_release(gpugrav_ctx *c)
   c->pm_rho.release();
   c->pm_rhok.release();
   c->pm_tab.release();
+  spare_take(&c->pm_force);
+  spare_take(&c->pm_sort);
   c->pm_force.release();
   c->pm_sort.release();
   c->pm_tab_n = 0;
