@@ -1932,23 +1932,19 @@ cudaError_t walk32_order(gpugrav_ctx *c, const WalkConst &wc)
   // neighbours' cache lines were lost there (2^24 particles of an early box, depth 8: 16.6 ms in key order,
   // 16.8 ms in this one).
   const int64_t targets = (c->w_ntargets > 0 ? c->w_ntargets : c->n) / c->nslices;
-  const size_t cap      = c->g_groups.cap / sizeof(int4);
   if(wc.bh || !deep_tree(c, 4) || targets / (32 * walk32_tpl(c)) <= (int64_t)c->w32_blocks * (c->w32_threads / 32))
     return cudaSuccess;
-  if(c->g_order.ensure(sizeof(GroupOrder) + cap * (sizeof(int) + 1)) != cudaSuccess)
-    cudaGetLastError();  // no room: key order
-  else
-    {
-      GroupOrder *o      = c->g_order.as<GroupOrder>();
-      int *order         = (int *)(o + 1);
-      uint8_t *key       = (uint8_t *)(order + cap);
-      const int64_t *rng = c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr;
-      GG_TRY(cudaMemsetAsync(o, 0, sizeof(GroupOrder), c->stream));
-      k_order_key<<<148 * 8, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), c->slice, c->nslices, rng, c->g_groups.as<int4>(), c->w_tlist,
-                                                          c->oldacc_s.as<float>(), key, o);
-      k_order_scatter<<<148, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), c->slice, c->nslices, rng, key, o, order);
-      c->w32_order = order;
-    }
+  GG_TRY(c->g_order.ensure(sizeof(GroupOrder)));
+  // the order and the keys take the place of two arrays that only the making of the table uses
+  GroupOrder *o      = c->g_order.as<GroupOrder>();
+  int *order         = c->g_gflag.as<int>();
+  uint8_t *key       = c->g_gpd.as<uint8_t>();
+  const int64_t *rng = c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr;
+  GG_TRY(cudaMemsetAsync(o, 0, sizeof(GroupOrder), c->stream));
+  k_order_key<<<148 * 8, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), c->slice, c->nslices, rng, c->g_groups.as<int4>(), c->w_tlist,
+                                                      c->oldacc_s.as<float>(), key, o);
+  k_order_scatter<<<148, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), c->slice, c->nslices, rng, key, o, order);
+  c->w32_order = order;
   return cudaGetLastError();
 }
 }  // namespace gg

@@ -37,3 +37,23 @@ def test_pm_space_is_given_back(same, cuda_lib):
         b, q = pm.pm_periodic(grid, pos, mass)
     assert np.isfinite(acc).all()
     assert np.max(np.abs(a - b)) <= 1e-11 * np.max(np.abs(a)) and np.max(np.abs(p - q)) <= 1e-11 * np.max(np.abs(p))
+
+
+def test_group_order_takes_no_space_per_particle(cuda_lib):
+    """The relative walk of a clustered set orders its groups in arrays that are there already."""
+    import torch
+
+    ic = ics.zoom_box(log2_half=21, seed=3, pmgrid=256)
+    n = len(ic["mass"])
+    old = np.full(n, 50.0, np.float32)
+    prm = ics.params_for(ic, precision=L.PREC_FP32, err_tol_force_acc=0.01)
+    with GravityTree(prm) as t:
+        t.domain_decomposition(ic["pos"], ic["mass"], ic["softtype"])
+        t.construct_forcetree()
+        t.gravity_tree(old)  # by the geometric criterion: no order
+        before, _ = torch.cuda.mem_get_info()
+        prm.err_tol_theta = 0.0
+        t.set_params(prm)
+        t.gravity_tree(old)
+        after, _ = torch.cuda.mem_get_info()
+    assert before - after <= 4 << 20  # 5 bytes a particle would be 21 MB
