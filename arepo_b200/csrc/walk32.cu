@@ -1284,13 +1284,13 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
 }
 
 // ---- order of the groups ----
-// A walk of several groups per warp ends when its last group does.  The cost of a group under the relative
-// criterion spans three orders of magnitude (a background particle amid a dense core opens the core: 180 ms
-// against 6 ms for the median group), and in key order expensive ones began as late as half-way: the last
-// third of the 328 ms walk of a 2^24-particle zoom box ran on 80 of 3552 warps.  So the groups go by falling
-// cost, as far as it can be told before the walk: by the binary exponent of their smallest OldAcc, which
-// opens the most, and by key within one exponent.  That walk takes 250 ms (240 ms for all warps busy to the
-// end).  Every group's result is its own; the order changes none.
+// A walk of several groups per warp ends when its last group does, and the cost of a group under the relative
+// criterion varies.  So the groups go by falling cost, as far as it can be told before the walk: by the binary
+// exponent of their smallest OldAcc, which opens the most, and by key within one exponent.  Zoom boxes with OldAcc
+// of a previous pass, key order / this order: 2^19 particles 11.3 / 11.1 ms, 2^21 39.6 / 29.4, 2^24 303.9 / 295.1.  It
+// matters most where single groups are far off: with the background's OldAcc also for the few background particles
+// inside the core (180 ms for such a group against 6 for the median) the 2^24 walk takes 331 ms in key order, its
+// last third on 80 of 3552 warps, and 249 in this one.  Every group's result is its own; the order changes none.
 constexpr int kOrderBlock = 256;
 constexpr int kOrderRun   = 4;  // consecutive groups that stay together
 struct GroupOrder
