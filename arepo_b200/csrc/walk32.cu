@@ -1285,12 +1285,18 @@ __global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, 
 
 // ---- order of the groups ----
 // A walk of several groups per warp ends when its last group does, and the cost of a group under the relative
-// criterion varies.  So the groups go by falling cost, as far as it can be told before the walk: by the binary
-// exponent of their smallest OldAcc, which opens the most, and by key within one exponent.  Zoom boxes with OldAcc
-// of a previous pass, key order / this order: 2^19 particles 11.3 / 11.1 ms, 2^21 39.6 / 29.4, 2^24 303.9 / 295.1.  It
-// matters most where single groups are far off: with the background's OldAcc also for the few background particles
-// inside the core (180 ms for such a group against 6 for the median) the 2^24 walk takes 331 ms in key order, its
-// last third on 80 of 3552 warps, and 249 in this one.  Every group's result is its own; the order changes none.
+// criterion varies.  So clustered sets' groups go by falling cost, as far as it can be told before the walk, by the
+// binary exponents of the smallest and the largest OldAcc of a run of groups: lo, hi.
+//  * TreePM: by lo, which opens the most.  Zoom boxes with OldAcc of a previous pass, key order / this order:
+//    2^19 particles 11.3 / 11.1 ms, 2^21 39.6 / 29.4, 2^24 303.9 / 295.1.  It matters most where single groups are far
+//    off: with the background's OldAcc also for the few background particles inside the core (180 ms for such a
+//    group against 6 for the median) the 2^24 walk takes 331 ms in key order, its last third on 80 of 3552 warps, and
+//    249 in this one.
+//  * isolated sets, whose cost rises inwards: by hi + 2 (hi - lo), the dear half; the rest follow by key.  By lo the
+//    outskirts went first and the core last: Hernquist 2^20 2.34 ms against 1.83 in key order.  Key order / by lo /
+//    this order: Plummer 2^18 1.31 / 1.30 / 1.22, 2^20 3.28 / 2.84 / 2.70, 2^22 11.4 / 11.4 / 11.6; Hernquist 2^18 0.71 /
+//    0.85 / 0.78, 2^20 1.83 / 2.34 / 1.86 (with OldAcc of a previous pass 2.19 / 2.33 / 2.02), 2^22 12.3 / 11.8 / 10.5.
+// Every group's result is its own; the order changes none.
 constexpr int kOrderBlock = 256;
 constexpr int kOrderRun   = 4;  // consecutive groups that stay together
 struct GroupOrder
@@ -1303,7 +1309,7 @@ __device__ __forceinline__ void group_range(const int *ngroups_dev, int slice, i
   b                = slice_rng ? (int)slice_rng[0] : (int)(ng * slice / nslices);
   e                = slice_rng ? (int)slice_rng[1] : (int)(ng * (slice + 1) / nslices);
 }
-__global__ void __launch_bounds__(kOrderBlock) k_order_key(const int *__restrict__ ngroups_dev, int slice, int nslices,
+__global__ void __launch_bounds__(kOrderBlock) k_order_key(const int *__restrict__ ngroups_dev, int isolated, int slice, int nslices,
                                                            const int64_t *__restrict__ slice_rng, const int4 *__restrict__ groups,
                                                            const int32_t *__restrict__ tlist, const float *__restrict__ oldacc,
                                                            uint8_t *__restrict__ key, GroupOrder *__restrict__ o)
@@ -1320,15 +1326,21 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_key(const int *__restrict
       const int g0 = b + r * kOrderRun, g1 = g0 + kOrderRun < e ? g0 + kOrderRun : e;
       // consecutive groups hold consecutive targets
       const int4 last = groups[g1 - 1];
-      float a         = 3.0e38f;
+      float lo = 3.0e38f, hi = 0.0f;
 #pragma unroll 8
       for(int k = groups[g0].x + lane; k < last.x + last.y; k += 32)
-        a = fminf(a, oldacc[tlist ? tlist[k] : k]);
-      a = wminf(a);
+        {
+          const float a = oldacc[tlist ? tlist[k] : k];
+          lo            = fminf(lo, a);
+          hi            = fmaxf(hi, a);
+        }
+      lo = wminf(lo);
+      hi = wmaxf(hi);
       if(lane == 0)
         {
-          const int x = (__float_as_int(a) >> 23) & 255;
-          key[r]      = (uint8_t)x;
+          const int eh = (__float_as_int(hi) >> 23) & 255, el = (__float_as_int(lo) >> 23) & 255;
+          const int x  = isolated ? 255 - min(max(eh + 2 * min(max(eh - el, 0), 63) - 64, 0), 255) : el;
+          key[r]       = (uint8_t)x;
           atomicAdd(&h[x], g1 - g0);
         }
     }
@@ -1337,23 +1349,35 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_key(const int *__restrict
     if(h[t])
       atomicAdd(&o->hist[t], h[t]);
 }
-__global__ void __launch_bounds__(kOrderBlock) k_order_scatter(const int *__restrict__ ngroups_dev, int slice, int nslices,
+__global__ void __launch_bounds__(kOrderBlock) k_order_scatter(const int *__restrict__ ngroups_dev, int share, int slice, int nslices,
                                                                const int64_t *__restrict__ slice_rng, const uint8_t *__restrict__ key,
                                                                GroupOrder *__restrict__ o, int *__restrict__ order)
 {
   static_assert(kOrderBlock == 256, "one thread per exponent");
   typedef cub::BlockScan<int, kOrderBlock> Scan;
   __shared__ typename Scan::TempStorage tmp;
-  __shared__ int cnt[256], base[256];
+  __shared__ int cnt[256], base[256], heads, first;  // heads: classes of the dear half; first: groups in them
+  const int in_class = o->hist[threadIdx.x];
   int start, b, e;
-  Scan(tmp).ExclusiveSum(o->hist[threadIdx.x], start);
+  Scan(tmp).ExclusiveSum(in_class, start);
   group_range(ngroups_dev, slice, nslices, slice_rng, b, e);
+  if(threadIdx.x == 0)
+    heads = first = 0;
+  __syncthreads();
+  if(share * (int64_t)(start + in_class) <= e - b)
+    {
+      atomicMax(&heads, (int)threadIdx.x + 1);
+      atomicMax(&first, start + in_class);
+    }
+  __syncthreads();
+  if(threadIdx.x == 255 && heads < 256)
+    start = first;  // the rest share the last class
   const int runs = (e - b + kOrderRun - 1) / kOrderRun;
   for(int r0 = blockIdx.x * kOrderBlock; r0 < runs; r0 += gridDim.x * kOrderBlock)
     {
       cnt[threadIdx.x] = 0;
       __syncthreads();
-      const int r = r0 + threadIdx.x, x = r < runs ? key[r] : -1;
+      const int r = r0 + threadIdx.x, x = r < runs ? (key[r] < heads ? key[r] : 255) : -1;
       const int g0 = b + r * kOrderRun, g1 = g0 + kOrderRun < e ? g0 + kOrderRun : e;
       const int at = x >= 0 ? atomicAdd(&cnt[x], g1 - g0) : 0;
       __syncthreads();
@@ -1927,12 +1951,12 @@ cudaError_t slice_mask_stage(gpugrav_ctx *c, bool fp32)
 cudaError_t walk32_order(gpugrav_ctx *c, const WalkConst &wc)
 {
   // Where some warps take more than one group (a walk that all runs at once needs no order), by the relative
-  // criterion (the geometric one, bh, does not look at OldAcc), in a tree deeper by four levels than an even
-  // set's of that size: the groups of an even set cost the same, and the 25 us of the two kernels and the
-  // neighbours' cache lines were lost there (2^24 particles of an early box, depth 8: 16.6 ms in key order,
-  // 16.8 ms in this one).
+  // criterion (the geometric one, bh, does not look at OldAcc), in a tree deeper by nine levels than an even
+  // set's of that size, as zoom boxes and spheres are: displaced grids and random sets, deeper by up to eight,
+  // have groups of one cost and lost 0.3 to 5 % by the two kernels' 25 us and the neighbours' cache lines (2^18
+  // uniform particles 0.311 -> 0.329 ms, 160^3 of a grid 6.05 -> 6.18).
   const int64_t targets = (c->w_ntargets > 0 ? c->w_ntargets : c->n) / c->nslices;
-  if(wc.bh || !deep_tree(c, 4) || targets / (32 * walk32_tpl(c)) <= (int64_t)c->w32_blocks * (c->w32_threads / 32))
+  if(wc.bh || !deep_tree(c, 9) || targets / (32 * walk32_tpl(c)) <= (int64_t)c->w32_blocks * (c->w32_threads / 32))
     return cudaSuccess;
   GG_TRY(c->g_order.ensure(sizeof(GroupOrder)));
   // the order and the keys take the place of two arrays that only the making of the table uses
@@ -1941,9 +1965,9 @@ cudaError_t walk32_order(gpugrav_ctx *c, const WalkConst &wc)
   uint8_t *key       = c->g_gpd.as<uint8_t>();
   const int64_t *rng = c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr;
   GG_TRY(cudaMemsetAsync(o, 0, sizeof(GroupOrder), c->stream));
-  k_order_key<<<148 * 8, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), c->slice, c->nslices, rng, c->g_groups.as<int4>(), c->w_tlist,
+  k_order_key<<<148 * 8, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), !wc.pm, c->slice, c->nslices, rng, c->g_groups.as<int4>(), c->w_tlist,
                                                       c->oldacc_s.as<float>(), key, o);
-  k_order_scatter<<<148, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), c->slice, c->nslices, rng, key, o, order);
+  k_order_scatter<<<148, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), wc.pm ? 1 : 2, c->slice, c->nslices, rng, key, o, order);
   c->w32_order = order;
   return cudaGetLastError();
 }
