@@ -515,6 +515,7 @@ int32_t gpugrav_load(gpugrav_ctx *c, int64_t n, const double *pos, const double 
   cudaEventRecord(c->ev[1], st);
 
   // softening types must index ForceSoftening[0..nsofttypes-1]: validated on the host copy when given
+  gg::IoWait io_wait{c};
   gg::HostIo *io = c->io();
   if(!io)
     return fail(c, GPUGRAV_ERR_OOM, "gpugrav_load: pinned allocation");
@@ -543,6 +544,7 @@ int32_t gpugrav_load(gpugrav_ctx *c, int64_t n, const double *pos, const double 
   CK(cudaMemcpyAsync(&bc, c->bconst.p, sizeof(bc), cudaMemcpyDeviceToHost, st), "download domain");
   CK(cudaMemcpyAsync(io->counters, c->counters.p, sizeof(int), cudaMemcpyDeviceToHost, st), "download flags");
   CK(cudaStreamSynchronize(st), "domain stage");
+  io_wait.waited  = true;
   const int flags = io->counters[0];
   if(flags & 2)
     return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_load: non-finite particle position");
@@ -572,6 +574,7 @@ int32_t gpugrav_build(gpugrav_ctx *c, const gpugrav_topnode *top, int32_t ntop)
   if(!c->loaded)
     return fail(c, GPUGRAV_ERR_STATE, "gpugrav_build before gpugrav_load");
   DeviceGuard g(c->device);
+  gg::IoWait io_wait{c};
   cudaStream_t st = c->stream;
   c->built        = false;
   c->layout32_valid = false;
@@ -597,6 +600,7 @@ int32_t gpugrav_build(gpugrav_ctx *c, const gpugrav_topnode *top, int32_t ntop)
   cudaEventRecord(c->ev[5], st);
   int s = 0;
   CK(gg::build_stage(c, &s), "tree build");
+  io_wait.waited = true;
   if(s == GPUGRAV_ERR_TOPNODES && c->top_dev && c->ntop < 0)
     return fail(c, s, "gpugrav_build: top-level tree could not be refined (PEANOGRID too coarse)");
   if(s != GPUGRAV_OK)
@@ -763,6 +767,7 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
      c->nint_s.ensure(n * sizeof(int32_t)) != cudaSuccess || c->oldacc_s.ensure(n * sizeof(float)) != cudaSuccess ||
      c->oldacc_in.ensure(n * sizeof(float)) != cudaSuccess || (active && c->t_in.ensure(nt * sizeof(int32_t) + 16) != cudaSuccess))
     return fail(c, GPUGRAV_ERR_OOM, "gpugrav_walk: device allocation");
+  gg::IoWait io_wait{c};
   gg::HostIo *io = c->io();
   if(!io)
     return fail(c, GPUGRAV_ERR_OOM, "gpugrav_walk: pinned allocation");
@@ -894,6 +899,7 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
   CK(cudaMemcpyAsync(io->counters, c->counters.p, kCounters * sizeof(int), cudaMemcpyDeviceToHost, st), "walk flags");
   cudaEventRecord(c->ev[10], st);
   CK(cudaStreamSynchronize(st), "walk");
+  io_wait.waited = true;
   if(fp32 && io->counters[13])
     {
       c->layout32_valid = false;
@@ -921,6 +927,7 @@ int gravity_direct_impl(gpugrav_ctx *c, int64_t n, const double *pos, const doub
   DeviceGuard g(c->device);
   cudaStream_t st = c->stream;
   c->loaded = c->built = false;  // the particle buffers are reused
+  gg::IoWait io_wait{c};
   gg::HostIo *io = c->io();
   if(!io)
     return fail(c, GPUGRAV_ERR_OOM, "gpugrav_gravity_direct: pinned allocation");
@@ -956,6 +963,7 @@ int gravity_direct_impl(gpugrav_ctx *c, int64_t n, const double *pos, const doub
       cudaEventRecord(c->ev[9], st);
       CK(cudaMemcpyAsync(h + out, d + out, flag_at + 4 - out, cudaMemcpyDeviceToHost, st), "download");
       CK(cudaStreamSynchronize(st), "direct summation");
+      io_wait.waited = true;
       if(*(int *)(h + flag_at))
         return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_gravity_direct: softening type >= nsofttypes");
       memcpy(acc, h + out, n * 24);
@@ -1001,6 +1009,7 @@ int gravity_direct_impl(gpugrav_ctx *c, int64_t n, const double *pos, const doub
   int bad = 0;
   CK(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, st), "flags");
   CK(cudaStreamSynchronize(st), "direct summation");
+  io_wait.waited = true;
   if(bad)
     return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_gravity_direct: softening type >= nsofttypes");
   c->timings.walk_ms              = elapsed(c->ev[8], c->ev[9]);

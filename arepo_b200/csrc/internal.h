@@ -283,7 +283,8 @@ struct gpugrav_ctx
   gg::DevBuf dir_buf, dir_io;                 // direct summation: working space; targets and results
   gg::PinnedBuf pinned, stage;  // HostIo; arrays of small direct sums
   // Pinned block for the small transfers of a call: what several kernels leave for the host comes back
-  // together, with one wait, and constants go out without staging.  Every call that uses it ends with a wait.
+  // together, with one wait, and constants go out without staging.  Every call that uses it ends with a wait,
+  // its error returns too (IoWait).
   gg::HostIo *io() { return pinned.ensure(sizeof(gg::HostIo)) == cudaSuccess ? (gg::HostIo *)pinned.p : nullptr; }
 
   cudaEvent_t ev[20] = {};
@@ -363,4 +364,15 @@ inline bool deep_tree(const gpugrav_ctx *c, int more)
 // GPUGRAV_OK or GPUGRAV_ERR_INVALID: ABI version, softening table (finite, >= 0, zero end entry),
 // box size, TreePM split (asmth, rcut, rcut_cells > 0 unless asmth == 0), tolerances, flags
 int validate_params(const gpugrav_params *p);
+// Waits for the context's stream where a call that uses the pinned block returns without having done so.
+struct IoWait
+{
+  gpugrav_ctx *c;
+  bool waited = false;
+  ~IoWait()
+  {
+    if(!waited)
+      cudaStreamSynchronize(c->stream);
+  }
+};
 }  // namespace gg

@@ -761,6 +761,7 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
   if(nsys == 0)
     return GPUGRAV_OK;
 
+  gg::IoWait io_wait{c};
   // ---- system table ----
   std::vector<SysDev> sd(nsys);
   std::vector<int64_t> cst(nsys);
@@ -891,6 +892,7 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
   SCK(cudaMemcpyAsync(flags, c->counters.p, kCounters * sizeof(int), cudaMemcpyDeviceToHost, st), "walk flags");
   SCK(cudaMemsetAsync(c->counters.as<int>() + 32, 0, 8, st), "walk flags");
   SCK(cudaStreamSynchronize(st), "tick");
+  io_wait.waited = true;
   unsigned long long inter = 0;
   memcpy(&inter, flags + 32, sizeof(inter));
   c->mark("s3 walk graph");
