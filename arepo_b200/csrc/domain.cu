@@ -179,7 +179,9 @@ __global__ void k_keys(const double *__restrict__ pos, int64_t n, const BuildCon
 // Sorting 126-bit keys takes 16 radix passes over 20 bytes a particle; their leading 64 bits (21 levels
 // of the curve, a cell of 5e-7 of the domain) take 8 over 12 bytes and leave few particles in runs of
 // equal leading bits, which are ordered here by their full keys.  A run longer than kMaxRun (coincident
-// or nearly coincident points) sets flag 8: the caller then sorts the full keys.
+// or nearly coincident points, the centre of a deep zoom) sets flag 8: the caller then sorts the full keys, and
+// goes on with these for the next sets of the context until k_long_runs finds none (2^22 particles with such a
+// clump: 2.0 ms for both sorts and gathers, 1.2 for the full sort alone; 2^24 7.5 and 4.2).
 constexpr int kMaxRun = 32;
 __global__ void k_sort_ties(int64_t n, const uint64_t *__restrict__ lead, const u128 *__restrict__ key, uint32_t *__restrict__ perm,
                             int *__restrict__ flags)
@@ -208,6 +210,16 @@ __global__ void k_sort_ties(int64_t n, const uint64_t *__restrict__ lead, const 
           perm[b] = o;
         }
     }
+}
+
+// flag 8: the sorted keys hold a run of more than kMaxRun equal leading bits (k >> shift)
+__global__ void k_long_runs(int64_t n, const u128 *__restrict__ key, int shift, int *__restrict__ flags)
+{
+  bool found = false;
+  for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i + kMaxRun < n; i += (int64_t)gridDim.x * blockDim.x)
+    found |= (uint64_t)(key[i] >> shift) == (uint64_t)(key[i + kMaxRun] >> shift);
+  if(found)
+    atomicOr(flags, 8);
 }
 
 // ---- gather into sorted SoA ----
@@ -310,6 +322,13 @@ cudaError_t sort_full_stage(gpugrav_ctx *c, int64_t n, int bits)
   GG_TRY(c->sort_tmp.ensure(tb));
   return cub::DeviceRadixSort::SortPairs(c->sort_tmp.p, tb, c->key.as<u128>(), c->key_alt.as<u128>(), c->idx.as<uint32_t>(),
                                          c->perm.as<uint32_t>(), (int)n, 0, bits, c->stream);
+}
+
+// after sort_full_stage: whether sort_lead_stage, on leading bits k >> shift, would have needed it (flag 8 of *flags)
+cudaError_t sort_runs_stage(gpugrav_ctx *c, int64_t n, int shift, int *flags)
+{
+  k_long_runs<<<grid_for(n, 256), 256, 0, c->stream>>>(n, c->key_alt.as<u128>(), shift, flags);
+  return cudaGetLastError();
 }
 
 cudaError_t gather_stage(gpugrav_ctx *c)

@@ -538,7 +538,13 @@ int32_t gpugrav_load(gpugrav_ctx *c, int64_t n, const double *pos, const double 
 
   CK(gg::domain_stage(c, dom == nullptr), "domain stage");
   cudaEventRecord(c->ev[2], st);
-  CK(gg::sort_lead_stage(c, n, c->counters.as<int>()), "key sort");
+  if(c->sort_full)
+    {
+      CK(gg::sort_full_stage(c, n, 3 * kBits), "key sort");
+      CK(gg::sort_runs_stage(c, n, 3 * kBits - 64, c->counters.as<int>()), "key sort");
+    }
+  else
+    CK(gg::sort_lead_stage(c, n, c->counters.as<int>()), "key sort");
   cudaEventRecord(c->ev[3], st);
   CK(gg::gather_stage(c), "gather");
   CK(cudaMemcpyAsync(&bc, c->bconst.p, sizeof(bc), cudaMemcpyDeviceToHost, st), "download domain");
@@ -553,7 +559,9 @@ int32_t gpugrav_load(gpugrav_ctx *c, int64_t n, const double *pos, const double 
   c->dom = bc.dom;
   if(flags & 4)
     return fail(c, GPUGRAV_ERR_INVALID, "gpugrav_load: softening type >= nsofttypes");
-  if(flags & 8)
+  const bool sorted = c->sort_full;
+  c->sort_full      = (flags & 8) != 0;
+  if(c->sort_full && !sorted)
     {
       CK(gg::sort_full_stage(c, n, 3 * kBits), "key sort");
       cudaEventRecord(c->ev[3], st);

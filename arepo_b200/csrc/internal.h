@@ -52,6 +52,7 @@ struct BuildConst
 };
 
 constexpr int kSortFlag     = 24;  // gpugrav_ctx::counters: sort_lead_stage's flag in the serving loop
+constexpr int kSortRuns     = 25;  // ... and sort_runs_stage's
 constexpr int kTopCount     = 40;  // gpugrav_ctx::counters: nodes of the library's top tree (< 0: it could not be refined)
 constexpr int kNeedFullSort = 1;   // build_stage status: the particles are not in full key order yet
 
@@ -221,6 +222,7 @@ struct gpugrav_ctx
   gg::DevBuf pos_in, mass_in, st_in;          // caller order
   gg::DevBuf key, key_alt, idx, perm;         // full keys (caller order); leading key bits before and after the sort; order
   gg::DevBuf sort_tmp;
+  bool sort_full = false;                     // the last set needed the sort by full keys: the next is sorted so at once
   gg::DevBuf s_pm, s_ix, s_iy, s_iz, s_st;    // sorted SoA: (x,y,z,m) double4, 52-bit coordinates, softening type
   gg::DevBuf s_cd, s_tl, s_tlnode;            // pair depth, top-leaf depth / node
   gg::DevBuf cnt, base, hcnt, hack_list, hack_scratch, counters;
@@ -308,6 +310,7 @@ void spare_take(DevBuf *b);
 cudaError_t domain_stage(gpugrav_ctx *c, bool compute_extent);
 cudaError_t sort_lead_stage(gpugrav_ctx *c, int64_t n, int *flags);
 cudaError_t sort_full_stage(gpugrav_ctx *c, int64_t n, int bits);
+cudaError_t sort_runs_stage(gpugrav_ctx *c, int64_t n, int shift, int *flags);
 cudaError_t gather_stage(gpugrav_ctx *c);
 cudaError_t toptree_stage(gpugrav_ctx *c, int *status);
 cudaError_t skeleton_stage(gpugrav_ctx *c, int *status);

@@ -809,8 +809,15 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
                                                   c->m_doms.as<gpugrav_domain>(), c->key.as<u128>(), c->key_alt.as<uint64_t>(),
                                                   14 - slot_bits, c->idx.as<uint32_t>());
   int *sort_flag = c->counters.as<int>() + kSortFlag;
-  SCK(cudaMemsetAsync(sort_flag, 0, sizeof(int), st), "sort");
-  SCK(gg::sort_lead_stage(c, ntot, sort_flag), "sort");
+  static_assert(kSortRuns == kSortFlag + 1, "cleared together");
+  SCK(cudaMemsetAsync(sort_flag, 0, 2 * sizeof(int), st), "sort");
+  if(c->sort_full)
+    {
+      SCK(gg::sort_full_stage(c, ntot, 128), "sort");
+      SCK(gg::sort_runs_stage(c, ntot, 50 + slot_bits, c->counters.as<int>() + kSortRuns), "sort");
+    }
+  else
+    SCK(gg::sort_lead_stage(c, ntot, sort_flag), "sort");
   auto gather = [&]() {
     k_srv_gather<<<grid_for(ntot, 256), 256, 0, st>>>(ntot, c->perm.as<uint32_t>(), s->csys.as<int32_t>(), s->c2p.as<int64_t>(),
                                                       s->pos.as<double4>(), s->stype.as<uint8_t>(), s->oldacc.as<float>(),
@@ -835,6 +842,7 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
     {
       SCK(cudaMemsetAsync(sort_flag, 0, sizeof(int), st), "sort");
       SCK(gg::sort_full_stage(c, ntot, 128), "sort");
+      SCK(gg::sort_runs_stage(c, ntot, 50 + slot_bits, c->counters.as<int>() + kSortRuns), "sort");
       gather();
       SCK(gg::build_stage(c, &bstat), "build");
     }
@@ -895,6 +903,7 @@ int32_t gpugrav_serve_tick(gpugrav_serve *s, int32_t *n_active)
   io_wait.waited = true;
   unsigned long long inter = 0;
   memcpy(&inter, flags + 32, sizeof(inter));
+  c->sort_full = flags[kSortRuns] != 0;
   c->mark("s3 walk graph");
   if(flags[13])
     return sfail(s, GPUGRAV_ERR_CUDA, "layout self-check failed");
