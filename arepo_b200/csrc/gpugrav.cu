@@ -680,7 +680,7 @@ int32_t gpugrav_export_mass_per_type(gpugrav_ctx *c, double *out)
     return GPUGRAV_ERR_INVALID;
   if(!c->built)
     return fail(c, GPUGRAV_ERR_STATE, "gpugrav_export_mass_per_type before gpugrav_build");
-  if(!(c->prm.flags & GPUGRAV_FLAG_MULTIPLE_NODE_SOFTENING))
+  if(!(c->prm.flags & GPUGRAV_FLAG_MULTIPLE_NODE_SOFTENING) || !c->built_mns)
     return fail(c, GPUGRAV_ERR_STATE, "gpugrav_export_mass_per_type: built without MULTIPLE_NODE_SOFTENING");
   DeviceGuard g(c->device);
   CK(cudaMemcpyAsync(out, c->n_mpt.p, (size_t)c->num_nodes * c->prm.nsofttypes * sizeof(double), cudaMemcpyDeviceToHost,

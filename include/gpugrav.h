@@ -164,6 +164,11 @@ int32_t gpugrav_abi_version(void);
  * the context owns all device memory and grows it as needed. */
 int32_t gpugrav_create(gpugrav_ctx **ctx, int32_t device, const gpugrav_params *params);
 int32_t gpugrav_destroy(gpugrav_ctx *ctx);
+/* New parameters for the following calls.  Loaded particles and a built tree stay valid unless periodic,
+ * box_size, nsofttypes or force_softening change; everything else (criterion, tolerances, precision, the
+ * TreePM split, flags) may change between walks of one tree -- except that
+ * GPUGRAV_FLAG_MULTIPLE_NODE_SOFTENING needs the per-type node masses of a tree built with it: a walk with the flag
+ * of a tree built without returns GPUGRAV_ERR_STATE (switching it off on a built tree is fine). */
 int32_t gpugrav_set_params(gpugrav_ctx *ctx, const gpugrav_params *params);
 /* Run all library work on a caller-owned cudaStream_t (NULL: the context's own non-blocking stream,
  * which does not order against the caller's work; the legacy default stream is cudaStreamLegacy). */
@@ -189,7 +194,8 @@ int32_t gpugrav_load(gpugrav_ctx *ctx, int64_t n, const double *pos, const doubl
  * (force_update_node_recursive :1217-1429).
  * top: the caller's TopNodes (domain_determineTopTree output) or NULL, in which case the library
  * derives the top tree from the sorted keys with the same refinement rule (one rank, work load =
- * particle count). */
+ * particle count).  A caller's tree is checked: daughters and leaves in range, every leaf reached,
+ * morton_to_peano that of the curve (GPUGRAV_ERR_TOPNODES otherwise). */
 int32_t gpugrav_build(gpugrav_ctx *ctx, const gpugrav_topnode *top, int32_t ntop);
 
 /* ---- walk ----
@@ -197,7 +203,13 @@ int32_t gpugrav_build(gpugrav_ctx *ctx, const gpugrav_topnode *top, int32_t ntop
  * (src/gravity/forcetree_walk.c:115-514) for every loaded particle as a target.
  * The opening criterion follows err_tol_theta: > 0 Barnes-Hut, == 0 relative (uses oldacc).
  * oldacc: n floats in caller order or NULL (zeros); acc: n*3 doubles; pot, ninter: n each or NULL.
- * All arrays in caller order, in memory of kind `mem`. */
+ * All arrays in caller order, in memory of kind `mem`.
+ * Precision: GPUGRAV_PREC_FP32 and GPUGRAV_PREC_FP64_GROUP take periodic images relative to the centre of a group of
+ * 64 targets consecutive in key order (32 without a TreePM split).  That is each target's own nearest image
+ * while half a group's extent plus Rcut is within half the box, which sets of some thousand particles and more
+ * satisfy; for smaller periodic sets, or an Rcut near half the box, use GPUGRAV_PREC_FP64.  Without a split the
+ * correction is tabulated up to half the box, and groups that span a tenth of it (fewer than 10^4 particles) lose
+ * accuracy in the same way. */
 int32_t gpugrav_walk(gpugrav_ctx *ctx, const float *oldacc, double *acc, double *pot, int32_t *ninter, int32_t mem);
 /* The walk of an active subset: gravity_tree(timebin) builds TargetList from
  * TimeBinsGravity.ActiveParticleList (src/gravity/gravtree.c:494-520) and walks only those particles
@@ -219,7 +231,7 @@ int32_t gpugrav_walk_targets(gpugrav_ctx *ctx, int64_t ntargets, const int32_t *
 int32_t gpugrav_set_target_slice(gpugrav_ctx *ctx, int32_t slice, int32_t nslices);
 
 /* Read-back of ExtNodes[].mass_per_type under MULTIPLE_NODE_SOFTENING: num_nodes x nsofttypes
- * doubles in the reference's node order (parity checks). */
+ * doubles in the reference's node order (parity checks).  GPUGRAV_ERR_STATE where the tree was built without. */
 int32_t gpugrav_export_mass_per_type(gpugrav_ctx *ctx, double *out);
 
 /* The same with slices of equal COST instead of equal target counts: cost (n floats in caller order,
