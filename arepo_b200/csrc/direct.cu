@@ -254,7 +254,8 @@ __global__ void k_map_targets(const int64_t *__restrict__ tg, int64_t nt, const 
 // targets into shared memory, then 4 T lanes add them, one sum component each, in source order.  Sets that fill
 // the chip with one thread per target have no need of that (k_gravity_direct_wide).
 template <bool EWALD, int P>  // P: component pitch of `out`
-__device__ __forceinline__ void direct_terms(const double4 s, double h_j, double4 me, double h_i, const WalkConst &w, double *__restrict__ out)
+__device__ __forceinline__ void direct_terms(const double4 s, double h_j, double4 me, double h_i, const WalkConst &w,
+                                             double *__restrict__ out)
 {
 #pragma unroll
   for(int c = 0; c < (EWALD ? 8 : 4); c++)

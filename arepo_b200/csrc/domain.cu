@@ -340,7 +340,8 @@ cudaError_t gather_stage(gpugrav_ctx *c)
      (e = c->s_st.ensure(n + 16)) != cudaSuccess || (e = c->iperm.ensure(n * sizeof(uint32_t))) != cudaSuccess)
     return e;
   k_gather<<<grid_for(n, 256), 256, 0, c->stream>>>(c->pos_in.as<double>(), c->mass_in.as<double>(), c->st_in.as<uint8_t>(),
-                                                   c->perm.as<uint32_t>(), n, c->bconst.as<BuildConst>(), c->iperm.as<uint32_t>(), c->s_pm.as<double4>(),
+                                                   c->perm.as<uint32_t>(), n, c->bconst.as<BuildConst>(),
+                                                   c->iperm.as<uint32_t>(), c->s_pm.as<double4>(),
                                                    c->s_ix.as<uint64_t>(), c->s_iy.as<uint64_t>(), c->s_iz.as<uint64_t>(),
                                                    c->s_st.as<uint8_t>(), c->counters.as<int>());
   return cudaGetLastError();

@@ -248,6 +248,13 @@ float elapsed(cudaEvent_t a, cudaEvent_t b)
 }
 }  // namespace
 
+cudaError_t gg::results_out(cudaStream_t st, int64_t n, const double4 *res, const int32_t *nint, const uint32_t *iperm, double *acc,
+                            double *pot, int32_t *nint_out)
+{
+  k_gather_out<<<grid_for(n, kOutTile), kOutTile, 0, st>>>(res, nint, iperm, n, acc, pot, nint_out);
+  return cudaGetLastError();
+}
+
 // Parameter checks shared by every entry point that takes a gpugrav_params.
 int gg::validate_params(const gpugrav_params *p)
 {
@@ -422,9 +429,12 @@ int32_t gpugrav_destroy(gpugrav_ctx *c)
                         &c->sort_tmp, &c->s_pm, &c->s_ix, &c->s_iy, &c->s_iz, &c->s_st, &c->s_cd, &c->s_tl, &c->s_tlnode,
                         &c->cnt, &c->base, &c->hcnt, &c->hack_list, &c->hack_scratch, &c->counters, &c->top, &c->skel,
                         &c->n_suns, &c->n_depth, &c->n_cl, &c->n_sm, &c->n_maxsoft, &c->n_size, &c->n_father, &c->n_sibling,
-                        &c->n_next, &c->n_dfs, &c->n_count, &c->n_arrived, &c->n_off, &c->p_next, &c->p_father, &c->p_off, &c->w_sm, &c->w_cl, &c->w_link, &c->g_scan, &c->g_sm, &c->g_rel, &c->g_kids, &c->g_pm, &c->g_pst, &c->g_stack, &c->res_s,
+                        &c->n_next, &c->n_dfs, &c->n_count, &c->n_arrived, &c->n_off, &c->p_next, &c->p_father, &c->p_off,
+                        &c->w_sm, &c->w_cl, &c->w_link, &c->g_scan, &c->g_sm, &c->g_rel, &c->g_kids, &c->g_pm, &c->g_pst,
+                        &c->g_stack, &c->res_s,
                         &c->nint_s, &c->oldacc_s, &c->oldacc_in, &c->out_acc, &c->out_pot, &c->out_nint, &c->scratch,
-                        &c->g_groups, &c->g_ngroups, &c->g_order, &c->g_gpd, &c->g_gseg, &c->g_gflag, &c->g_gid, &c->t_cd, &c->t_pd, &c->m_sys, &c->m_doms,
+                        &c->g_groups, &c->g_ngroups, &c->g_order, &c->g_gpd, &c->g_gseg, &c->g_gflag, &c->g_gid, &c->t_cd,
+                        &c->t_pd, &c->m_sys, &c->m_doms,
                         &c->pm_pos, &c->pm_mass, &c->pm_acc, &c->pm_pot, &c->ewd, &c->ewd32, &c->n_mpt, &c->w_mpt,
                         &c->g_mpt, &c->iperm, &c->t_in, &c->t_pos, &c->t_pos_alt, &c->t_idx, &c->t_idx_alt,
                         &c->cost_in, &c->cost_u, &c->cost_p, &c->slice_rng, &c->dir_buf, &c->dir_io};
@@ -891,9 +901,8 @@ int walk_impl(gpugrav_ctx *c, int64_t nt, const int32_t *targets, const float *o
     CK(gg::targets_scatter(c, nt, fp32, d_acc, d_pot, d_nint), "scatter");
   else
     {
-      k_gather_out<<<grid_for(n, kOutTile), kOutTile, 0, st>>>(c->res_s.as<double4>(), c->nint_s.as<int32_t>(),
-                                                               c->iperm.as<uint32_t>(), n, d_acc, d_pot, d_nint);
-      CK(cudaGetLastError(), "scatter");
+      CK(gg::results_out(st, n, c->res_s.as<double4>(), c->nint_s.as<int32_t>(), c->iperm.as<uint32_t>(), d_acc, d_pot, d_nint),
+         "scatter");
     }
   if(mem == GPUGRAV_MEM_HOST)
     {

@@ -304,6 +304,9 @@ __device__ __forceinline__ int common_depth(uint64_t ax, uint64_t ay, uint64_t a
 namespace gg
 {
 // launchers implemented in the .cu files; each returns cudaGetLastError() of its launches
+// results in sorted order to the caller's (iperm: sorted position per particle); nint, pot may be null
+cudaError_t results_out(cudaStream_t st, int64_t n, const double4 *res, const int32_t *nint, const uint32_t *iperm, double *acc,
+                        double *pot, int32_t *nint_out);
 // buffers that any allocation may take back between calls (gpugrav.cu)
 void spare_offer(DevBuf *b, int device);
 void spare_take(DevBuf *b);

@@ -101,31 +101,6 @@ __global__ void k_pm_scatter(int64_t np, const uint32_t *__restrict__ iperm, con
                  "d"(mass[o])
                  : "memory");
 }
-constexpr int kOutTile = 256;
-__global__ void __launch_bounds__(kOutTile) k_pm_out(int64_t np, const double4 *__restrict__ res, const uint32_t *__restrict__ iperm,
-                                                     double *__restrict__ acc, double *__restrict__ pot)
-{
-  __shared__ double a[3 * kOutTile];
-  for(int64_t t0 = (int64_t)blockIdx.x * kOutTile; t0 < np; t0 += (int64_t)gridDim.x * kOutTile)
-    {
-      const int64_t o = t0 + threadIdx.x;
-      __syncthreads();
-      if(o < np)
-        {
-          const double4 r        = res[iperm[o]];
-          a[3 * threadIdx.x + 0] = r.x;
-          a[3 * threadIdx.x + 1] = r.y;
-          a[3 * threadIdx.x + 2] = r.z;
-          if(pot)
-            pot[o] = r.w;
-        }
-      __syncthreads();
-      const int cnt = (int)(3 * (np - t0 < kOutTile ? np - t0 : kOutTile));
-      for(int q = threadIdx.x; q < cnt; q += kOutTile)
-        acc[3 * t0 + q] = a[q];
-    }
-}
-
 // SORTED: positions and masses in brick order (pm), else the caller's arrays
 template <bool SORTED>
 __global__ void k_pm_deposit(int64_t np, const double *__restrict__ pos, const double *__restrict__ mass, const double4 *__restrict__ pm, int n,
@@ -533,8 +508,7 @@ cudaError_t pm_stage(gpugrav_ctx *c, int pmgrid, int64_t np, const double *pos, 
       GG_TRY(cudaFuncSetAttribute(k_pm_read_brick, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       k_pm_read_brick<<<(int)((np + kReadChunk - 1) / kReadChunk), 256, smem, st>>>(np, s_pm, start, n, nb, f, c->pm_rho.as<double>(),
                                                                                     fac_pot / (2.0 * d), fac_pot, s_res, bad);
-      k_pm_out<<<blocks_for(np), kOutTile, 0, st>>>(np, s_res, iperm, acc, pot);
-      return cudaGetLastError();
+      return results_out(st, np, s_res, nullptr, iperm, acc, pot, nullptr);
     }
   // The records take 32 bytes per mesh point, written once.  Few particles on a large mesh (kFewMesh, kFewShare) do
   // not pay for that, and where the records would take more than a quarter of the device's free memory there is

@@ -205,8 +205,9 @@ __device__ bool top_less(const TopTmp *T, int a, int b)
 }
 
 constexpr int kTopThreads = 256;
-__global__ void __launch_bounds__(kTopThreads) k_toptree(const u128 *__restrict__ keys, const uint32_t *__restrict__ perm, int64_t n, double tnf, int mdom, TopTmp *T, int *queue,
-                                                         int *list, int *sorted, gpugrav_topnode *out, int max_top, int *result)
+__global__ void __launch_bounds__(kTopThreads)
+    k_toptree(const u128 *__restrict__ keys, const uint32_t *__restrict__ perm, int64_t n, double tnf, int mdom, TopTmp *T, int *queue,
+              int *list, int *sorted, gpugrav_topnode *out, int max_top, int *result)
 {
   const int ntask = 1;
   int a = 1 + (ntask / 7 + 1) * 8, b = (int)(tnf * mdom * ntask);
@@ -381,10 +382,10 @@ __global__ void __launch_bounds__(kTopThreads) k_toptree(const u128 *__restrict_
 // 35 us from global memory); validation and output are everyone's.
 // ------------------------------------------------------------------------------
 constexpr int kSkelThreads = 128, kSkelShared = 256;
-__global__ void __launch_bounds__(kSkelThreads) k_skeleton(const gpugrav_topnode *__restrict__ top_g, int ntop, const int *__restrict__ ntop_dev, const BuildConst *__restrict__ bc,
-                                                           int32_t *__restrict__ suns, double4 *__restrict__ cl_g, uint8_t *__restrict__ depth,
-                                                           int32_t *__restrict__ father, int32_t *__restrict__ leafnode,
-                                                           int32_t *__restrict__ nodetop, SkelInfo *info)
+__global__ void __launch_bounds__(kSkelThreads)
+    k_skeleton(const gpugrav_topnode *__restrict__ top_g, int ntop, const int *__restrict__ ntop_dev, const BuildConst *__restrict__ bc,
+               int32_t *__restrict__ suns, double4 *__restrict__ cl_g, uint8_t *__restrict__ depth, int32_t *__restrict__ father,
+               int32_t *__restrict__ leafnode, int32_t *__restrict__ nodetop, SkelInfo *info)
 {
   __shared__ gpugrav_topnode top_sh[kSkelShared];
   __shared__ double4 cl_sh[kSkelShared];

@@ -247,7 +247,7 @@ __device__ __forceinline__ double wrapd(double d, const W32Const &w)
   return d;
 }
 
-// 32 bytes in one load (32-byte aligned)
+// 32 bytes in one load (32-byte aligned): a double4, and two float4 (load2)
 __device__ __forceinline__ double4 load32(const double4 *p)
 {
   double4 v;
@@ -343,7 +343,6 @@ struct Tgt
   int ni;
 };
 
-// 32 bytes in one load (32-byte aligned)
 __device__ __forceinline__ void load2(const float4 *p, float4 &a, float4 &b)
 {
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -875,17 +874,14 @@ struct BlockSh
 // gives both the same lists, and each evaluates one target per lane.  While there are fewer groups than
 // half the warps the walk takes as long as its slowest warp, and the evaluation is most of that.
 template <bool PERIODIC, bool POT, int TPL, bool EWALD = false, typename R = float, bool SPLIT = false>
-__global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, PERIODIC, TPL>::blocks) k_walk32(const double4 *__restrict__ g_sm, const float4 *__restrict__ g_rel,
-                                                        const int4 *__restrict__ g_kids, const double4 *__restrict__ g_pm,
-                                                        const uint8_t *__restrict__ g_pst, const double4 *__restrict__ tpm,
-                                                        const uint8_t *__restrict__ tst, const float *__restrict__ oldacc,
-                                                        const int *__restrict__ ngroups_dev, const int4 *__restrict__ groups,
-                                                        const int *__restrict__ order, const int32_t *__restrict__ tlist, int slice, int nslices,
-                                                        const int64_t *__restrict__ slice_rng,
-                                                        const W32Const *__restrict__ wcp,
-                                                        int *__restrict__ stack_base, int *__restrict__ work,
-                                                        double4 *__restrict__ res_out, int32_t *__restrict__ nint_out, unsigned long long *__restrict__ total,
-                                                        int *__restrict__ err, const int *__restrict__ layout_err)
+__global__ void __launch_bounds__(32 * Shape<R, PERIODIC, TPL>::warps, Shape<R, PERIODIC, TPL>::blocks)
+    k_walk32(const double4 *__restrict__ g_sm, const float4 *__restrict__ g_rel, const int4 *__restrict__ g_kids,
+             const double4 *__restrict__ g_pm, const uint8_t *__restrict__ g_pst, const double4 *__restrict__ tpm,
+             const uint8_t *__restrict__ tst, const float *__restrict__ oldacc, const int *__restrict__ ngroups_dev,
+             const int4 *__restrict__ groups, const int *__restrict__ order, const int32_t *__restrict__ tlist, int slice,
+             int nslices, const int64_t *__restrict__ slice_rng, const W32Const *__restrict__ wcp, int *__restrict__ stack_base,
+             int *__restrict__ work, double4 *__restrict__ res_out, int32_t *__restrict__ nint_out,
+             unsigned long long *__restrict__ total, int *__restrict__ err, const int *__restrict__ layout_err)
 {
   constexpr int kWarps = Shape<R, PERIODIC, TPL>::warps;
   constexpr bool WRAP  = PERIODIC || EWALD;  // nearest images in a periodic box
@@ -1821,14 +1817,12 @@ cudaError_t walk32_launch(gpugrav_ctx *c)
   int *err        = c->counters.as<int>() + 14;
   GG_TRY(cudaMemsetAsync(work, 0, sizeof(int), st));
   Walk32Kernel kern = (Walk32Kernel)c->w32_kernel;
-  kern<<<c->w32_blocks, c->w32_threads, c->w32_smem, st>>>(c->g_sm.as<double4>(), c->g_rel.as<float4>(), c->g_kids.as<int4>(),
-                                              c->g_pm.as<double4>(), c->g_pst.as<uint8_t>(), c->s_pm.as<double4>(),
-                                              c->s_st.as<uint8_t>(), c->oldacc_s.as<float>(), c->g_ngroups.as<int>(),
-                                              c->g_groups.as<int4>(), c->w32_order, c->w_tlist, c->slice, c->nslices,
-                                              c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr,
-                                              (const W32Const *)c->scratch.p,
-                                              c->g_stack.as<int>(), work, c->res_s.as<double4>(),
-                                              c->nint_s.as<int32_t>(), (unsigned long long *)(c->counters.as<int>() + 32), err, c->counters.as<int>() + 13);
+  kern<<<c->w32_blocks, c->w32_threads, c->w32_smem, st>>>(
+      c->g_sm.as<double4>(), c->g_rel.as<float4>(), c->g_kids.as<int4>(), c->g_pm.as<double4>(), c->g_pst.as<uint8_t>(),
+      c->s_pm.as<double4>(), c->s_st.as<uint8_t>(), c->oldacc_s.as<float>(), c->g_ngroups.as<int>(), c->g_groups.as<int4>(),
+      c->w32_order, c->w_tlist, c->slice, c->nslices, c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr,
+      (const W32Const *)c->scratch.p, c->g_stack.as<int>(), work, c->res_s.as<double4>(), c->nint_s.as<int32_t>(),
+      (unsigned long long *)(c->counters.as<int>() + 32), err, c->counters.as<int>() + 13);
   return cudaGetLastError();
 }
 
@@ -1965,9 +1959,11 @@ cudaError_t walk32_order(gpugrav_ctx *c, const WalkConst &wc)
   uint8_t *key       = c->g_gpd.as<uint8_t>();
   const int64_t *rng = c->slice_rng_on ? c->slice_rng.as<int64_t>() : nullptr;
   GG_TRY(cudaMemsetAsync(o, 0, sizeof(GroupOrder), c->stream));
-  k_order_key<<<148 * 8, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), !wc.pm, c->slice, c->nslices, rng, c->g_groups.as<int4>(), c->w_tlist,
-                                                      c->oldacc_s.as<float>(), key, o);
-  k_order_scatter<<<148, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), wc.pm ? 1 : 2, c->slice, c->nslices, rng, key, o, order);
+  k_order_key<<<148 * 8, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), !wc.pm, c->slice, c->nslices, rng,
+                                                      c->g_groups.as<int4>(), c->w_tlist, c->oldacc_s.as<float>(), key, o);
+  // TreePM: every class in its order; isolated: those of the dear half
+  k_order_scatter<<<148, kOrderBlock, 0, c->stream>>>(c->g_ngroups.as<int>(), wc.pm ? 1 : 2, c->slice, c->nslices, rng, key, o,
+                                                      order);
   c->w32_order = order;
   return cudaGetLastError();
 }
