@@ -885,6 +885,7 @@ __global__ void k_children(int64_t nn, int32_t n, const int32_t *__restrict__ su
     atomicMax(deepest, d);
 }
 
+constexpr int kChildren = 4;  // records that k_moments reads at a time
 // ancestors of a node: a replayed cell's chain has up to 4096 (replay_cell's bound), below the tree's levels
 constexpr int kMaxChain = 4096 + 64;
 
@@ -892,12 +893,18 @@ constexpr int kMaxChain = 4096 + 64;
 // Every thread starts at a node without node children and goes up as long as it is the last to arrive at
 // the parent, so that the whole tree takes one launch; what other threads wrote is read from L2.  One
 // launch per level (two dozen) left the narrow upper levels to pay a launch and a memory latency chain
-// each: 0.15 ms on 4099 particles and 0.9 ms on the 2^24 zoom box.
-__global__ void __launch_bounds__(128) k_moments(int64_t nn, int32_t n, const int32_t *__restrict__ suns, const uint8_t *__restrict__ count,
-                                                 int32_t *__restrict__ arrived, const int32_t *__restrict__ father,
-                                                 const double4 *__restrict__ pm, const uint8_t *__restrict__ st,
-                                                 const double4 *__restrict__ cl, double4 *sm, uint8_t *maxsoft, int32_t *size,
-                                                 const BuildConst *__restrict__ bc, double *mpt, int *err)
+// each: 0.15 ms on 4099 particles against 0.05.  Bound by latency -- a warp's lanes go up at different times, each
+// step a round trip to the children, one to the counter --, hence by the warps in flight: the children are read
+// four at a time, which leaves 64 registers and eight blocks per SM, and the counter's addition carries the ordering
+// (release of this node's record, acquire of the siblings') instead of two fences around it.  With all eight
+// children at once (104 registers) and fences the build of the 2^24 zoom box took 4.26 ms, of 256^3 targets 2.21, of
+// 2^20 0.38; now 2.96, 1.86 and 0.30 (level by level 1.3 of it were moments, in one launch 2.7, now 1.3).
+template <bool MNS>
+__global__ void __launch_bounds__(128, 8)
+    k_moments(int64_t nn, int32_t n, const int32_t *__restrict__ suns, const uint8_t *__restrict__ count, int32_t *__restrict__ arrived,
+              const int32_t *__restrict__ father, const double4 *__restrict__ pm, const uint8_t *__restrict__ st,
+              const double4 *__restrict__ cl, double4 *sm, uint8_t *maxsoft, int32_t *size, const BuildConst *__restrict__ bc,
+              double *mpt, int *err)
 {
   int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   // after a failed self-check some fathers and children are not set: the build ends without following any
@@ -907,7 +914,7 @@ __global__ void __launch_bounds__(128) k_moments(int64_t nn, int32_t n, const in
     {
       int32_t c[8];
       load_suns(suns, k, c);
-      if(mpt)
+      if(MNS)
         {
           // ExtNodes[].mass_per_type (MULTIPLE_NODE_SOFTENING, src/gravity/forcetree.c:1256-1308): per type,
           // the particle masses and the child sums of slots 0..7 in order
@@ -931,44 +938,49 @@ __global__ void __launch_bounds__(128) k_moments(int64_t nn, int32_t n, const in
           for(int q = 0; q < ns; q++)
             mpt[k * ns + q] = acc[q];
         }
-      // the children's records, fetched together
-      double4 m[8];
-      int ts[8], sz[8];
-#pragma unroll
-      for(int q = 0; q < 8; q++)
-        {
-          m[q]  = make_double4(0, 0, 0, 0);
-          ts[q] = sz[q] = 0;
-          if(c[q] >= n)
-            {
-              const double2 *r = (const double2 *)(sm + (c[q] - n));
-              const double2 u = __ldcg(r), v = __ldcg(r + 1);
-              m[q]  = make_double4(u.x, u.y, v.x, v.y);
-              ts[q] = __ldcg(maxsoft + (c[q] - n));
-              sz[q] = __ldcg(size + (c[q] - n));
-            }
-          else if(c[q] >= 0)
-            {
-              m[q]  = pm[c[q]];
-              ts[q] = st[c[q]];
-              sz[q] = 1;
-            }
-        }
       double mass = 0, sx = 0, sy = 0, sz_ = 0;
       int ms    = bc->nsoft;  // NSOFTTYPES + NSOFTTYPES_HYDRO: the entry whose softening is 0
       int total = 1;
 #pragma unroll
-      for(int q = 0; q < 8; q++)
-        if(c[q] >= 0)
-          {
-            mass = __dadd_rn(mass, m[q].w);
-            sx   = __dadd_rn(sx, __dmul_rn(m[q].w, m[q].x));
-            sy   = __dadd_rn(sy, __dmul_rn(m[q].w, m[q].y));
-            sz_  = __dadd_rn(sz_, __dmul_rn(m[q].w, m[q].z));
-            if(bc->soft[ms] < bc->soft[ts[q]])
-              ms = ts[q];
-            total += sz[q];
-          }
+      for(int h = 0; h < 8; h += kChildren)
+        {
+          // some children's records, fetched together
+          double4 m[kChildren];
+          int ts[kChildren], sz[kChildren];
+#pragma unroll
+          for(int q = 0; q < kChildren; q++)
+            {
+              const int32_t v = c[h + q];
+              m[q]            = make_double4(0, 0, 0, 0);
+              ts[q] = sz[q] = 0;
+              if(v >= n)
+                {
+                  const double2 *r = (const double2 *)(sm + (v - n));
+                  const double2 a = __ldcg(r), b = __ldcg(r + 1);
+                  m[q]  = make_double4(a.x, a.y, b.x, b.y);
+                  ts[q] = __ldcg(maxsoft + (v - n));
+                  sz[q] = __ldcg(size + (v - n));
+                }
+              else if(v >= 0)
+                {
+                  m[q]  = pm[v];
+                  ts[q] = st[v];
+                  sz[q] = 1;
+                }
+            }
+#pragma unroll
+          for(int q = 0; q < kChildren; q++)
+            if(c[h + q] >= 0)
+              {
+                mass = __dadd_rn(mass, m[q].w);
+                sx   = __dadd_rn(sx, __dmul_rn(m[q].w, m[q].x));
+                sy   = __dadd_rn(sy, __dmul_rn(m[q].w, m[q].y));
+                sz_  = __dadd_rn(sz_, __dmul_rn(m[q].w, m[q].z));
+                if(bc->soft[ms] < bc->soft[ts[q]])
+                  ms = ts[q];
+                total += sz[q];
+              }
+        }
       if(mass != 0)
         {
           sx  = __ddiv_rn(sx, mass);
@@ -989,10 +1001,10 @@ __global__ void __launch_bounds__(128) k_moments(int64_t nn, int32_t n, const in
       if(p < n)
         return;  // a root
       k = p - n;
-      __threadfence();
-      if(atomicAdd(&arrived[k], 1) + 1 < (count[k] & 15))
+      int before;
+      asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(before) : "l"(arrived + k) : "memory");
+      if(before + 1 < (count[k] & 15))
         return;
-      __threadfence();
     }
   atomicOr(err, 16);  // no root above: the build's self-check
 }
@@ -1462,11 +1474,12 @@ cudaError_t build_stage(gpugrav_ctx *c, int *status)
     GG_TRY(c->n_mpt.ensure((size_t)(nn + 16) * c->prm.nsofttypes * sizeof(double)));
   k_children<<<grid_for(nn, 256), 256, 0, st>>>(nn, (int32_t)n, c->n_suns.as<int32_t>(), c->n_depth.as<uint8_t>(),
                                                  c->n_count.as<uint8_t>(), c->n_arrived.as<int32_t>(), counters + 4);
-  k_moments<<<(unsigned)((nn + 127) / 128), 128, 0, st>>>(nn, (int32_t)n, c->n_suns.as<int32_t>(), c->n_count.as<uint8_t>(),
-                                                          c->n_arrived.as<int32_t>(), c->n_father.as<int32_t>(), c->s_pm.as<double4>(),
-                                                          c->s_st.as<uint8_t>(), c->n_cl.as<double4>(), c->n_sm.as<double4>(),
-                                                          c->n_maxsoft.as<uint8_t>(), c->n_size.as<int32_t>(),
-                                                          c->bconst.as<BuildConst>(), mns ? c->n_mpt.as<double>() : nullptr, a.err);
+  auto moments = mns ? k_moments<true> : k_moments<false>;
+  moments<<<(unsigned)((nn + 127) / 128), 128, 0, st>>>(nn, (int32_t)n, c->n_suns.as<int32_t>(), c->n_count.as<uint8_t>(),
+                                                        c->n_arrived.as<int32_t>(), c->n_father.as<int32_t>(), c->s_pm.as<double4>(),
+                                                        c->s_st.as<uint8_t>(), c->n_cl.as<double4>(), c->n_sm.as<double4>(),
+                                                        c->n_maxsoft.as<uint8_t>(), c->n_size.as<int32_t>(),
+                                                        c->bconst.as<BuildConst>(), mns ? c->n_mpt.as<double>() : nullptr, a.err);
   launches += 2;
   c->mark("b5 moments");
   // 6. threading and the layout of the FP64 walk; the group walk needs neither (several systems are
