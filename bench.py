@@ -60,8 +60,8 @@ UNIT = "particles/s"
 FLOPS_PER_INTERACTION = 23.0  # convention of the path's roofline
 # DRAM bytes (read + write) of one FP32 walk launch per particle: ncu capture of the zoom box at
 # N=2^21 (dram__bytes_read.sum + dram__bytes_write.sum = 591.5 MB + 110.8 MB), scaled by the
-# particle count (the walk reads the tree and the particles once from DRAM; everything else hits
-# in L2)
+# particle count (groups in order of cost read the tree and the particles about twice from DRAM;
+# everything else hits in L2)
 WALK32_DRAM_BYTES_PER_PARTICLE = 702.3e6 / (1 << 21)
 # ErrTolForceAcc of the per-target FP64 walk in the precision ablation: the value at which its RMS
 # error on the zoom box is at most the FP32 walk's at 6e-5 (8.2e-4 against 9.4e-4)
